@@ -123,6 +123,10 @@ static CollInfo fused_gemm_decode(Comm& comm, DType t, const GemmArPtrs* ptrs, i
   // split K until the tiles x splits fill the GPU (every split keeps at least two stages of work)
   int64_t splits = std::max<int64_t>(1, cap / tiles);
   splits = std::min<int64_t>(splits, std::min<int64_t>(kDecodeMaxSplits, std::max<int64_t>(1, kb_total / (2 * kDecKSub))));
+  // A split takes a whole number of stages, so fewer splits than asked for may already cover K (18 column blocks over
+  // 4 splits: 6 + 6 + 6).  A split without work would add an accumulator that nothing has written.
+  const int64_t kb_per = ceil_div64(ceil_div64(kb_total, splits), kDecKSub) * kDecKSub;
+  splits = ceil_div64(kb_total, kb_per);
   const int64_t units = tiles * splits;
   int ctas = ctas_req > 0 ? ctas_req : int(std::min<int64_t>(cap, std::max<int64_t>(units, M)));
   B200_REQUIRE(ctas <= cap, "requested " << ctas << " CTAs, only " << cap << " can run at once");

@@ -60,6 +60,19 @@ def test_local_linear_on_the_weight_streaming_kernel(world):
             torch.testing.assert_close(o.float(), x.float() @ w.float().t(), atol=3e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("M,K,N", [(16, 1152, 3072), (32, 1088, 1024), (1, 1344, 2560), (7, 3200, 2432)])
+def test_every_split_of_k_has_work(M, K, N):
+    """Column blocks that do not divide over the K splits of the decode-sized kernel: the splits then cover K with
+    fewer of them.  The tolerance is that of one rounding of the product to fp16 on top of the fp32 sum."""
+    with Communicator.virtual(1, 0, staging_bytes=64 << 20) as comm:
+        for rep in range(2):
+            xs, ws, _, _ = _mk(1, M, K, N, torch.float16, seed=rep)
+            outs = comm.linear_allreduce(xs, ws)
+            torch.cuda.synchronize()
+            comm.check()
+            torch.testing.assert_close(outs[0].float(), xs[0].float() @ ws[0].float().t(), atol=4e-3, rtol=2e-3)
+
+
 @pytest.mark.parametrize("world", [1, 8])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_gemm_allreduce_residual_rmsnorm(world, dtype):

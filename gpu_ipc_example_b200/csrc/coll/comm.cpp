@@ -502,11 +502,34 @@ CollInfo Comm::launch_ll(LLOpId op, AlgoSpec algo, DType t, const void* const* i
 // ----------------------------------------------------------------------------
 // Large messages
 // ----------------------------------------------------------------------------
+// Whether the barrier-based kernel can work on the callers' own buffers: all ranks live in this process (their buffers
+// are in one launch's arguments and one address space), everything is 16-byte aligned, and no output overlaps an
+// input except as the collective's in-place form (the staged form has read all inputs before it writes).
+bool Comm::bulk_direct_ok(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems) const {
+  if (!is_virtual()) return false;
+  const size_t N = size_t(world_);
+  const size_t in_bytes = nelems * 2;
+  const size_t out_bytes = mode == BulkModeId::AllReduce ? in_bytes : (mode == BulkModeId::AllGather ? in_bytes * N : in_bytes / N);
+  for (size_t i = 0; i < N; ++i) {
+    const uintptr_t o = reinterpret_cast<uintptr_t>(outs[i]);
+    if (((reinterpret_cast<uintptr_t>(ins[i]) | o) & 15) != 0) return false;
+    for (size_t j = 0; j < N; ++j) {
+      const uintptr_t p = reinterpret_cast<uintptr_t>(ins[j]);
+      if (p + in_bytes <= o || o + out_bytes <= p) continue;  // disjoint
+      const bool in_place = mode == BulkModeId::AllReduce ? (i == j && p == o)
+                                                          : (mode == BulkModeId::AllGather && i == j && p == o + i * in_bytes);
+      if (!in_place) return false;
+    }
+  }
+  return true;
+}
+
 CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* const* ins, void* const* outs,
                            size_t nelems, LaunchGeom geom, cudaStream_t stream, uint32_t flags) {
   const int N = world_;
   if (nvls) B200_REQUIRE(has_nvls(), "NVLS was not set up for this communicator: " << heaps_[0]->nvls_note());
-  KernelFn fn = bulk_kernel_lookup(mode, t, N, nvls);
+  const bool direct = !nvls && bulk_direct_ok(mode, ins, outs, nelems);
+  KernelFn fn = direct ? bulk_direct_kernel_lookup(mode, t, N) : bulk_kernel_lookup(mode, t, N, nvls);
   B200_REQUIRE(fn != nullptr, "no kernel for world size " << N << " (supported: 2, 4, 8)");
   const HeapLayout& lay = heaps_[0]->layout();
   if (mode == BulkModeId::ReduceScatter) B200_REQUIRE(nelems % size_t(N) == 0, "reduce-scatter input must divide by the world size");
@@ -526,14 +549,16 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
   const size_t sym_bytes = size_t(shard_vec) * 16 * size_t(N);
   const bool exact = (mode == BulkModeId::AllReduce) ? (nelems % (8 * size_t(N)) == 0) : (shard_elems % 8 == 0);
 
-  // Zero-copy when the caller's buffers already live in the symmetric heap at the
-  // same offset on every rank and the shards are vector-exact.
+  // An emulated world works on the callers' buffers as they are (`direct`).  Else: zero-copy when the caller's
+  // buffers already live in the symmetric heap at the same offset on every rank and the shards are vector-exact.
   //   all-reduce: in place on a symmetric buffer
   //   reduce-scatter: symmetric input
   //   all-gather: symmetric output
   size_t sym_off = SIZE_MAX;
   uint64_t copy_flags = 0;
-  {
+  if (direct) {
+    sym_off = 0;
+  } else {
     const void* probe = (mode == BulkModeId::AllGather) ? static_cast<const void*>(outs[0]) : ins[0];
     size_t off = exact ? sym_offset_of(probe, 0) : SIZE_MAX;
     bool ok = off != SIZE_MAX && off % 16 == 0;
@@ -543,7 +568,9 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
     }
     if (ok) sym_off = off;
   }
-  if (sym_off != SIZE_MAX) {
+  if (direct) {
+    // nothing to stage
+  } else if (sym_off != SIZE_MAX) {
     if (mode == BulkModeId::AllReduce) {
       bool in_place = true;
       for (int i = 0; i < nlocal(); ++i) in_place &= (ins[i] == outs[i]);
@@ -608,7 +635,7 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
 // ----------------------------------------------------------------------------
 // Public collectives
 // ----------------------------------------------------------------------------
-AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric) const {
+AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric, bool direct) const {
   AlgoSpec a;
   if (const char* e = std::getenv("B200IPC_PROTO")) {
     bool ag = false;
@@ -627,6 +654,11 @@ AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric) const {
       a.sched = (has_nvls() && world_ >= 8) ? SchedKind::Nvls : SchedKind::Bulk;
       a.proto = ProtoKind::LL512;
     }
+    return a;
+  }
+  if (direct && bytes > emulated_flag_max_bytes(EmuOp::AllReduce, world_)) {
+    a.sched = SchedKind::Bulk;
+    a.proto = ProtoKind::LL512;
     return a;
   }
   int rows = 0;
@@ -657,7 +689,7 @@ CollInfo Comm::all_reduce(AlgoSpec algo, DType t, const void* const* ins, void* 
   if (algo.automatic) {
     bool symmetric = true;
     for (int i = 0; i < nlocal(); ++i) symmetric &= (ins[i] == outs[i]) && sym_offset_of(ins[i], i) != SIZE_MAX;
-    algo = choose_all_reduce(nelems * 2, symmetric);
+    algo = choose_all_reduce(nelems * 2, symmetric, bulk_direct_ok(BulkModeId::AllReduce, ins, outs, nelems));
   }
   for (int i = 0; i < nlocal(); ++i) {
     B200_REQUIRE((reinterpret_cast<uintptr_t>(ins[i]) & 3) == 0 && (reinterpret_cast<uintptr_t>(outs[i]) & 3) == 0,
@@ -688,11 +720,15 @@ CollInfo Comm::all_gather(AlgoSpec algo, DType t, const void* const* ins, void* 
   if (algo.automatic) {
     algo = AlgoSpec{};
     const size_t bytes = nelems * 2;
+    const bool direct = nelems % 2 == 0 && bytes > emulated_flag_max_bytes(EmuOp::AllGather, world_) &&
+                        bulk_direct_ok(BulkModeId::AllGather, ins, outs, nelems);
     // two ranks: the direct flag-in-data push moves the same bytes as any other form and needs no
     // barrier; measured ahead of the barrier-based kernels and of NCCL up to 64 MiB per rank
     // measured on 8 GPUs (bytes per rank): the direct push wins up to 1 MiB (23 us against NCCL's 47), the
     // barrier kernel with peer loads from 2 to 8 MiB, the flag-in-data ring above (level with NCCL)
-    if (world_ == 2 || bytes <= (size_t(1) << 20) || nelems % 8 != 0) {
+    if (direct) {
+      algo.sched = SchedKind::Bulk;
+    } else if (world_ == 2 || bytes <= (size_t(1) << 20) || nelems % 8 != 0) {
       algo.sched = SchedKind::Ring;
       algo.proto = safe_protos_ ? ProtoKind::LL16 : ProtoKind::LL512;
       algo.direct_allgather = true;
@@ -724,8 +760,12 @@ CollInfo Comm::reduce_scatter(AlgoSpec algo, DType t, const void* const* ins, vo
   const bool was_auto = algo.automatic;
   if (algo.automatic) {
     algo = AlgoSpec{};
+    const bool direct = nelems % size_t(world_) == 0 && nelems * 2 > emulated_flag_max_bytes(EmuOp::ReduceScatter, world_) &&
+                        bulk_direct_ok(BulkModeId::ReduceScatter, ins, outs, nelems);
     // small inputs: one flag-in-data push to each slice's owner, no barrier
-    if (nelems % (2 * size_t(world_)) == 0 && nelems * 2 <= (safe_protos_ ? kReduceScatterLLMaxBytes / 2 : kReduceScatterLLMaxBytes)) {
+    if (direct) {
+      algo.sched = SchedKind::Bulk;
+    } else if (nelems % (2 * size_t(world_)) == 0 && nelems * 2 <= (safe_protos_ ? kReduceScatterLLMaxBytes / 2 : kReduceScatterLLMaxBytes)) {
       algo.sched = SchedKind::Parallel;
       algo.proto = safe_protos_ ? ProtoKind::LL16 : ProtoKind::LL512;
     } else {

@@ -105,7 +105,8 @@ class Comm {
 
   // Size -> algorithm choice used for AlgoSpec::automatic: the measured table of tuner.h unless
   // set_thresholds() installed explicit cut-offs (0, 0 restores the table).
-  AlgoSpec choose_all_reduce(size_t bytes, bool symmetric) const;
+  // `direct`: an emulated world whose buffers the barrier-based kernel can use as they are.
+  AlgoSpec choose_all_reduce(size_t bytes, bool symmetric, bool direct = false) const;
   void set_thresholds(size_t oneshot_max_bytes, size_t ll_max_bytes) {
     oneshot_max_bytes_ = oneshot_max_bytes;
     ll_max_bytes_ = ll_max_bytes;
@@ -186,6 +187,7 @@ class Comm {
   void common_init(const CommOptions& opt);
   CollInfo launch_ll(LLOpId op, AlgoSpec algo, DType t, const void* const* ins, void* const* outs, size_t nelems,
                      LaunchGeom geom, cudaStream_t stream, uint32_t flags);
+  bool bulk_direct_ok(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems) const;
   CollInfo launch_bulk(BulkModeId mode, bool nvls, DType t, const void* const* ins, void* const* outs, size_t nelems,
                        LaunchGeom geom, cudaStream_t stream, uint32_t flags);
 

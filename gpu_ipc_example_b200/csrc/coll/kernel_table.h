@@ -23,6 +23,8 @@ using KernelFn = void (*)(const KArgs);
 // nullptr when the combination is not compiled (world not in {2,4,8}).
 KernelFn ll_kernel_lookup(LLOpId op, DType t, ProtoKind k, int world);
 KernelFn bulk_kernel_lookup(BulkModeId m, DType t, int world, bool nvls);
+// The form that works on the callers' own buffers (emulated worlds: every rank can address all of them).
+KernelFn bulk_direct_kernel_lookup(BulkModeId m, DType t, int world);
 
 constexpr int kBulkThreadsPerCta = 512;
 // 16-byte vectors each thread keeps in flight per tile (host geometry and kernel agree on it).

@@ -50,4 +50,8 @@ KernelFn bulk_kernel_lookup(BulkModeId m, DType t, int world, bool nvls) {
   return bulk_lookup(t, world, nvls, static_cast<BulkMode>(int(m)));
 }
 
+KernelFn bulk_direct_kernel_lookup(BulkModeId m, DType t, int world) {
+  return bulk_direct_lookup(t, world, static_cast<BulkMode>(int(m)));
+}
+
 }  // namespace b200ipc

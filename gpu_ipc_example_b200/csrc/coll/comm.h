@@ -133,6 +133,7 @@ class Comm {
   bool device_seq() const { return device_seq_; }
   void set_seq(uint32_t s) { seq_ = s; }
   uint64_t launches() const { return launches_; }
+  void note_launch() { ++launches_; }  // a kernel that was not launched through launch_raw
   // After a failed self-test of the 64-byte-segment wire formats (LL128 / LL512 rely on a warp's aligned
   // 64-byte store arriving whole): `auto` then only uses formats whose atomic unit is an 8-byte granule.
   void set_safe_protos(bool on) { safe_protos_ = on; }

@@ -63,4 +63,10 @@ struct AgGemmPtrs {
 CollInfo fused_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64_t M, int64_t N, int64_t K, int ctas,
                               cudaStream_t stream);
 
+// The same two layers when this process drives every rank (a world of one, an emulated world): one GEMM over the callers'
+// operands, no exchange and no workspace (gemm_local.cuh).  `workspace` and `packed_kblocks` are not looked at.
+CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64_t M, int64_t N, int64_t K, float eps,
+                              bool with_norm, cudaStream_t stream);
+CollInfo local_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+
 }  // namespace b200ipc

@@ -1,18 +1,15 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <deque>
-#include <map>
 #include <mutex>
 #include <set>
-#include <tuple>
 
 #include "../common/check.h"
-#include "../common/cu_driver.h"
 #include "fused_ops.h"
 #include "ag_gemm.cuh"
 #include "gemm_ar.cuh"
 #include "gemm_decode.cuh"
+#include "tensor_map.h"
 
 namespace b200ipc {
 namespace {
@@ -29,45 +26,8 @@ const void* kernel_ptr() {
   return reinterpret_cast<const void*>(&gemm_ar_kernel<T, BN, STAGES, A_ROWS, KSUB>);
 }
 
-// Tensor maps depend only on (pointer, extents, box, type): weights and activation buffers are
-// reused call after call, so encoding is done once per distinct operand.  The cache is bounded: when
-// it is full the oldest entry makes room (never a wholesale clear in the middle of serving).
-using MapKey = std::tuple<const void*, uint64_t, uint64_t, uint32_t, int>;
-constexpr size_t kMaxCachedMaps = 4096;
 std::mutex g_map_mu;
-std::map<MapKey, CUtensorMap> g_maps;
-std::deque<MapKey> g_map_order;
 std::set<const void*> g_attr_done;
-
-void encode_2d(CUtensorMap* map, DType t, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  const MapKey key(base, rows, cols, box_rows, int(t));
-  {
-    std::lock_guard<std::mutex> lk(g_map_mu);
-    auto it = g_maps.find(key);
-    if (it != g_maps.end()) {
-      *map = it->second;
-      return;
-    }
-  }
-  B200_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "GEMM operands must be 16-byte aligned");
-  B200_REQUIRE((cols * 2) % 16 == 0, "the K extent must be a multiple of 8 elements");
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {uint32_t(kGemmBK), box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  B200_CU_CHECK(cu().TensorMapEncodeTiled(map, t == DType::F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                          2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-  std::lock_guard<std::mutex> lk(g_map_mu);
-  if (g_maps.emplace(key, *map).second) {
-    g_map_order.push_back(key);
-    if (g_map_order.size() > kMaxCachedMaps) {
-      g_maps.erase(g_map_order.front());
-      g_map_order.pop_front();
-    }
-  }
-}
 
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -154,7 +114,7 @@ static CollInfo fused_gemm_decode(Comm& comm, DType t, const GemmArPtrs* ptrs, i
     B200_REQUIRE(lo == landing_off && oo == out_off && ro == res_off, "symmetric tensors must sit at the same offset on every rank");
     B200_REQUIRE(lo % 256 == 0 && oo % 16 == 0 && ro % 16 == 0, "symmetric tensors must be 16-byte aligned");
     if (with_norm) B200_REQUIRE(p.gamma != nullptr && (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0, "RMSNorm needs gamma and an aligned residual");
-    encode_2d(&args.tma_a[i], t, p.x, uint64_t(M), uint64_t(K), uint32_t(kDecXRows));
+    encode_tile_map(&args.tma_a[i], t, p.x, uint64_t(M), uint64_t(K), uint32_t(kDecXRows));
     if (p.packed_kblocks > 0) {
       B200_REQUIRE(p.packed_kblocks == ptrs[0].packed_kblocks && int64_t(p.packed_kblocks) * 64 >= K,
                    "packed weight does not match K (pack it with Communicator.pack_weight)");
@@ -162,7 +122,7 @@ static CollInfo fused_gemm_decode(Comm& comm, DType t, const GemmArPtrs* ptrs, i
       args.packed_kblocks = p.packed_kblocks;
     } else {
       B200_REQUIRE(ptrs[0].packed_kblocks == 0, "either every rank's weight is packed or none");
-      encode_2d(&args.tma_b[i], t, p.w, uint64_t(N), uint64_t(K), uint32_t(kDecTileRows));
+      encode_tile_map(&args.tma_b[i], t, p.w, uint64_t(N), uint64_t(K), uint32_t(kDecTileRows));
     }
     args.residual[i] = p.residual;
     args.gamma[i] = p.gamma;
@@ -307,7 +267,7 @@ CollInfo fused_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64
     B200_REQUIRE(lo == landing_off && oo == out_off && ro == res_off, "symmetric tensors must sit at the same offset on every rank");
     B200_REQUIRE(lo % 256 == 0 && oo % 16 == 0 && ro % 16 == 0, "symmetric tensors must be 16-byte aligned");
     if (with_norm) B200_REQUIRE(p.gamma != nullptr, "RMSNorm needs gamma");
-    encode_2d(&args.tma_a[i], t, p.x, uint64_t(M), uint64_t(K), uint32_t(a_box));
+    encode_tile_map(&args.tma_a[i], t, p.x, uint64_t(M), uint64_t(K), uint32_t(a_box));
     if (p.packed_kblocks > 0) {
       B200_REQUIRE(p.packed_kblocks == ptrs[0].packed_kblocks && p.packed_kblocks % 4 == 0 && int64_t(p.packed_kblocks) * 64 >= K,
                    "packed weight does not match K (pack it with Communicator.pack_weight)");
@@ -316,7 +276,7 @@ CollInfo fused_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64
       args.packed_kblocks = p.packed_kblocks;
     } else {
       B200_REQUIRE(ptrs[0].packed_kblocks == 0, "either every rank's weight is packed or none");
-      encode_2d(&args.tma_b[i], t, p.w, uint64_t(N), uint64_t(K), uint32_t(BN));
+      encode_tile_map(&args.tma_b[i], t, p.w, uint64_t(N), uint64_t(K), uint32_t(BN));
     }
     args.residual[i] = p.residual;
     args.gamma[i] = p.gamma;
@@ -430,8 +390,8 @@ CollInfo fused_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64
     B200_REQUIRE((reinterpret_cast<uintptr_t>(p.x_shard) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0,
                  "x and out must be 16-byte aligned");
     const size_t xfull_off = ws_off + size_t(parity) * buf_bytes;
-    encode_2d(&args.tma_a[i], t, comm.sym_ptr(xfull_off, i), uint64_t(M), uint64_t(K), kGemmBM);
-    encode_2d(&args.tma_b[i], t, p.w, uint64_t(N), uint64_t(K), uint32_t(BN));
+    encode_tile_map(&args.tma_a[i], t, comm.sym_ptr(xfull_off, i), uint64_t(M), uint64_t(K), kGemmBM);
+    encode_tile_map(&args.tma_b[i], t, p.w, uint64_t(N), uint64_t(K), uint32_t(BN));
     args.x_shard[i] = p.x_shard;
     args.out[i] = p.out;
     args.xfull_off = xfull_off;

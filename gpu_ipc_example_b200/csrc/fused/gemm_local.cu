@@ -1,0 +1,243 @@
+#include <algorithm>
+#include <cstring>
+#include <map>
+#include <mutex>
+#include <utility>
+
+#include "../common/check.h"
+#include "fused_ops.h"
+#include "gemm_local.cuh"
+#include "tensor_map.h"
+
+namespace b200ipc {
+namespace {
+
+struct LocalPlan {
+  int bn = 32, m_tiles = 1, splits = 1;
+};
+
+// k blocks per stage: two where a block holds too little work for what its barriers and its commit cost
+int local_ksub(int bn) { return bn <= 128 ? 2 : 1; }
+
+int local_stages(int bn) {
+  const int stage = (128 + bn / 2) * kGemmBK * 2 * local_ksub(bn);
+  return std::min(kLocMaxStages, (kLocSmemBudget - 1024) / stage);
+}
+
+const void* local_kernel(DType t, int bn) {
+  const bool two = local_ksub(bn) == 2;
+  if (t == DType::F16)
+    return two ? reinterpret_cast<const void*>(&gemm_local_kernel<__half, 2>) : reinterpret_cast<const void*>(&gemm_local_kernel<__half, 1>);
+  return two ? reinterpret_cast<const void*>(&gemm_local_kernel<__nv_bfloat16, 2>)
+             : reinterpret_cast<const void*>(&gemm_local_kernel<__nv_bfloat16, 1>);
+}
+
+// Pairs (clusters of 2, 4, 8 CTAs) that can run at once on a device.
+int resident_clusters(const void* fn, int device, int splits) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, std::pair<int, int>>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(fn, std::make_pair(device, splits));
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  B200_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kLocSmemBudget));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(2 * splits));
+  cfg.blockDim = dim3(kLocThreads);
+  cfg.dynamicSmemBytes = kLocSmemBudget;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(2 * splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  B200_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, fn, &cfg));
+  known[key] = n;
+  return n;
+}
+
+// Microseconds that a plan takes apart from what all plans share (launch, first loads).  Fitted to one B200: a k block of a
+// pair 0.08 + 0.0012 BN (K = 8192, M = 2048, N = 7168: BN = 160 166 us, 224 170, 256 197, 128 197); the epilogue of a
+// tile 0.5 + 0.0133 BN, hidden behind the next tile's MMAs where there is one; handing partial sums between the pairs of a
+// cluster 1.6 + 0.006 BN (K = 1024, M = 1, N = 8192: one split 14.4 us, two 16.4; K = 3584, M = 16: 16.0 and 14.5).
+double plan_cost(int64_t tiles, int64_t room, int64_t kb_total, int bn, int splits) {
+  const double waves = double(ceil_div64(tiles, room));
+  const double main = double(ceil_div64(kb_total, splits)) * (0.08 + 0.0012 * bn);
+  const double epi = 0.5 + 0.0133 * bn / splits;
+  return waves * std::max(main, epi) + epi + (splits > 1 ? 1.6 + 0.006 * bn : 0);
+}
+
+// The tile height and the K split of a problem.  bn_only: the tile's height is given (merged shards).
+LocalPlan plan_local(DType t, int device, int64_t rows, int64_t shards, int64_t groups, int64_t N, int64_t kb_total, int bn_only) {
+  LocalPlan best;
+  double best_cost = 0;
+  const int64_t n_tiles = ceil_div64(N, kLocWRows);
+  for (int bn = bn_only ? bn_only : 32; bn <= (bn_only ? bn_only : kLocMaxBN); bn += 32) {
+    const int64_t m_tiles = bn_only ? 1 : ceil_div64(rows, bn);
+    if (!bn_only && bn > 32 && ceil_div64(rows, bn - 32) == m_tiles) continue;  // the lower tile covers the rows in as many
+    const int64_t tiles = m_tiles * shards * groups * n_tiles;
+    for (int splits = 1; splits <= 4; splits *= 2) {
+      const int64_t room = resident_clusters(local_kernel(t, bn), device, splits);
+      if (room < 1) continue;
+      if (splits > 1 && (tiles > room || kb_total < 4 * splits)) break;  // one tile per cluster, every split with work
+      const double cost = plan_cost(tiles, room, kb_total, bn, splits);
+      if (best_cost == 0 || cost < best_cost) {
+        best_cost = cost;
+        best.bn = bn;
+        best.m_tiles = int(m_tiles);
+        best.splits = splits;
+      }
+    }
+  }
+  return best;
+}
+
+void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, const void* const* xs,
+                  const void* const* ws, cudaStream_t stream, CollInfo* info) {
+  const int W = comm.world();
+  const void* fn = local_kernel(t, p.bn);
+  args.bn = p.bn;
+  args.m_tiles = p.m_tiles;
+  args.n_tiles = int(ceil_div64(args.N, kLocWRows));
+  args.splits = p.splits;
+  args.stages = local_stages(p.bn);
+  args.early_w = p.bn == 32 ? 1 : 0;
+  const int64_t mt_all = int64_t(args.shards) * p.m_tiles;
+  // as many m-tiles side by side as keep their X rows in a quarter of L2 while the W tiles pass by
+  const int64_t x_bytes = int64_t(p.bn) * args.K * 2 * args.segs;
+  args.band = int(std::min<int64_t>(mt_all, std::max<int64_t>(1, (int64_t(32) << 20) / x_bytes)));
+  for (int r = 0; r < W; ++r) {
+    encode_tile_map(&args.tma_x[r], t, xs[r], uint64_t(args.rows), uint64_t(args.K), uint32_t(args.merged ? args.merged_rows : p.bn / 2));
+    encode_tile_map(&args.tma_w[r], t, ws[r], uint64_t(args.N), uint64_t(args.K), 128);
+  }
+  KArgs views;
+  comm.fill_views(&views, nullptr, nullptr, 0, 0);
+  args.status = views.v[0].status;
+  args.abort_word = reinterpret_cast<uint32_t*>(views.v[0].heap + views.lay.ctrl_off + kCtrlAbortOff);
+  args.timeout_ns = views.v[0].timeout_ns;
+  args.rank = views.v[0].rank;
+
+  const int64_t total = mt_all * args.n_tiles * args.groups;
+  const int64_t clusters = std::min<int64_t>(total, resident_clusters(fn, comm.device(), p.splits));
+  B200_REQUIRE(clusters >= 1 && (p.splits == 1 || clusters == total), "GEMM kernel does not fit on the device");
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(clusters * 2 * p.splits));
+  cfg.blockDim = dim3(kLocThreads);
+  cfg.dynamicSmemBytes = kLocSmemBudget;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(2 * p.splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2u : 1u;
+  void* params[] = {&args};
+  B200_CUDA_CHECK(cudaLaunchKernelExC(&cfg, fn, params));
+  comm.note_launch();
+  info->sched = SchedKind::Bulk;
+  info->proto = ProtoKind::LL512;
+  info->ctas = int(cfg.gridDim.x);
+  info->warps = kLocThreads / 32;
+  info->nwires = info->ctas * info->warps;
+  info->steps = ceil_div64(total, clusters);
+  info->launches = 1;
+}
+
+void check_local(Comm& comm, int64_t M, int64_t N, int64_t K) {
+  B200_REQUIRE(comm.nlocal() == comm.world() && comm.world() <= kMaxRanks, "every rank must be driven by this process");
+  B200_REQUIRE(M > 0 && N > 0 && K > 0, "empty GEMM");
+  B200_REQUIRE(N % 64 == 0, "N must be a multiple of 64");
+  B200_REQUIRE(K % 8 == 0, "K must be a multiple of 8");
+  B200_CUDA_CHECK(cudaSetDevice(comm.device()));
+}
+
+}  // namespace
+
+CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64_t M, int64_t N, int64_t K, float eps,
+                              bool with_norm, cudaStream_t stream) {
+  check_local(comm, M, N, K);
+  const int W = comm.world();
+  LocalGemmArgs args;
+  std::memset(&args, 0, sizeof(args));
+  args.rows = int(M);
+  args.N = int(N);
+  args.K = int(K);
+  args.segs = W;
+  args.shards = args.groups = 1;
+  RowNormArgs norm;
+  std::memset(&norm, 0, sizeof(norm));
+  norm.N = int(N);
+  norm.eps = eps;
+  const void* xs[kMaxRanks];
+  const void* ws[kMaxRanks];
+  for (int i = 0; i < W; ++i) {
+    const GemmArPtrs& p = ptrs[i];
+    for (const void* q : {p.residual, p.gamma, static_cast<const void*>(p.out), static_cast<const void*>(p.res_out)})
+      B200_REQUIRE((reinterpret_cast<uintptr_t>(q) & 15) == 0, "linear + all-reduce needs 16-byte aligned tensors");
+    if (with_norm) B200_REQUIRE(p.gamma != nullptr, "RMSNorm needs gamma");
+    xs[i] = p.x;
+    ws[i] = p.w;
+    args.residual[i] = p.residual;
+    args.sum[i] = p.res_out ? p.res_out : p.out;
+    args.copy[i] = (p.res_out && !with_norm) ? p.out : nullptr;
+    norm.sum[i] = args.sum[i];
+    norm.gamma[i] = p.gamma;
+    norm.out[i] = p.out;
+  }
+  const int64_t kb = ceil_div64(K, kGemmBK) * W;
+  CollInfo info;
+  launch_local(comm, args, t, plan_local(t, comm.device(), M, 1, 1, N, kb, 0), xs, ws, stream, &info);
+  if (with_norm) {
+    // two vectors a thread where there are too few rows to fill the GPU otherwise
+    const int threads = M * W <= 2 * comm.sm_count() ? 512 : 256;
+    const void* nf = t == DType::F16 ? reinterpret_cast<const void*>(&row_norm_kernel<__half>)
+                                     : reinterpret_cast<const void*>(&row_norm_kernel<__nv_bfloat16>);
+    void* params[] = {&norm};
+    B200_CUDA_CHECK(launch_maybe_pdl(nf, dim3(unsigned(M), unsigned(W)), dim3(unsigned(threads)), params, 0, stream, true));
+    comm.note_launch();
+    info.launches = 2;
+  }
+  return info;
+}
+
+CollInfo local_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
+  check_local(comm, M, N, K);
+  const int W = comm.world();
+  B200_REQUIRE(M % W == 0, "the rows of X must divide evenly over the ranks");
+  LocalGemmArgs args;
+  std::memset(&args, 0, sizeof(args));
+  args.rows = int(M / W);
+  args.N = int(N);
+  args.K = int(K);
+  args.segs = 1;
+  args.shards = args.groups = W;
+  // Few rows: one tile takes the rows of all shards, so that W is read once and not once per shard (4 ranks, 16 rows each,
+  // K = 8192, N = 7168: 133 us, one shard per tile 180).
+  int bn_only = 0;
+  if (W > 1) {
+    const int64_t unit = W == 2 ? 16 : 8;  // whole swizzle blocks, and a tile of a multiple of 32 rows
+    const int64_t per_shard = ceil_div64(M / W, unit) * unit;
+    if (per_shard * W <= kLocMaxBN) {
+      args.merged = W;
+      args.merged_rows = int(per_shard);
+      args.shards = 1;
+      bn_only = int(per_shard * W);
+    }
+  }
+  const void* xs[kMaxRanks];
+  const void* ws[kMaxRanks];
+  for (int i = 0; i < W; ++i) {
+    B200_REQUIRE((reinterpret_cast<uintptr_t>(ptrs[i].out) & 15) == 0, "x and out must be 16-byte aligned");
+    xs[i] = ptrs[i].x_shard;
+    ws[i] = ptrs[i].w;
+    args.sum[i] = ptrs[i].out;
+  }
+  CollInfo info;
+  launch_local(comm, args, t, plan_local(t, comm.device(), M / W, args.shards, W, N, ceil_div64(K, kGemmBK), bn_only), xs, ws, stream, &info);
+  return info;
+}
+
+}  // namespace b200ipc

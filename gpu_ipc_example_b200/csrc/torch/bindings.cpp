@@ -339,6 +339,56 @@ std::vector<int64_t> fused_ag_gemm(std::vector<at::Tensor> xs, std::vector<at::T
   return info_vec(info);
 }
 
+// The same two layers with every rank in this process (a world of one or an emulated one): no workspace, outputs anywhere.
+std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::Tensor> ws, std::vector<at::Tensor> residuals,
+                                   std::vector<at::Tensor> gammas, std::vector<at::Tensor> outs, std::vector<at::Tensor> res_outs,
+                                   double eps, bool with_norm, int64_t comm_id) {
+  Comm& c = get(comm_id);
+  check_tensors(c, xs, "x");
+  check_tensors(c, ws, "weight");
+  check_tensors(c, outs, "output");
+  if (!residuals.empty()) check_tensors(c, residuals, "residual");
+  if (!gammas.empty()) check_tensors(c, gammas, "gamma");
+  if (!res_outs.empty()) check_tensors(c, res_outs, "residual output");
+  TORCH_CHECK(xs[0].dim() == 2 && ws[0].dim() == 2, "b200ipc: x must be [M, K] and weight [N, K] (or packed)");
+  const int64_t M = xs[0].size(0), K = xs[0].size(1), N = ws[0].size(0);
+  TORCH_CHECK(ws[0].size(1) == K, "b200ipc: weight must be [N, K] with the same K as x");
+  std::vector<GemmArPtrs> p(size_t(c.nlocal()));
+  for (int i = 0; i < c.nlocal(); ++i) {
+    TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes() && outs[i].numel() == M * N,
+                "b200ipc: shape mismatch between ranks");
+    TORCH_CHECK(xs[i].scalar_type() == ws[i].scalar_type() && xs[i].scalar_type() == outs[i].scalar_type(), "b200ipc: dtype mismatch");
+    p[size_t(i)].x = xs[i].data_ptr();
+    p[size_t(i)].w = ws[i].data_ptr();
+    p[size_t(i)].residual = residuals.empty() ? nullptr : residuals[i].data_ptr();
+    p[size_t(i)].gamma = gammas.empty() ? nullptr : gammas[i].data_ptr();
+    p[size_t(i)].out = outs[i].data_ptr();
+    p[size_t(i)].res_out = res_outs.empty() ? nullptr : res_outs[i].data_ptr();
+  }
+  c10::cuda::CUDAGuard guard(c.device());
+  return info_vec(local_gemm_allreduce(c, dtype_of(xs[0]), p.data(), M, N, K, float(eps), with_norm,
+                                       at::cuda::getCurrentCUDAStream(c.device())));
+}
+
+std::vector<int64_t> local_ag_gemm(std::vector<at::Tensor> xs, std::vector<at::Tensor> ws, std::vector<at::Tensor> outs, int64_t comm_id) {
+  Comm& c = get(comm_id);
+  check_tensors(c, xs, "x");
+  check_tensors(c, ws, "weight");
+  check_tensors(c, outs, "output");
+  TORCH_CHECK(xs[0].dim() == 2 && ws[0].dim() == 2, "b200ipc: x must be [M / world, K] and weight [N, K]");
+  const int64_t M = xs[0].size(0) * c.world(), K = xs[0].size(1), N = ws[0].size(0);
+  TORCH_CHECK(ws[0].size(1) == K, "b200ipc: weight must be [N, K] with the same K as x");
+  std::vector<AgGemmPtrs> p(size_t(c.nlocal()));
+  for (int i = 0; i < c.nlocal(); ++i) {
+    TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes() && outs[i].numel() == M * N,
+                "b200ipc: shape mismatch between ranks");
+    TORCH_CHECK(xs[i].scalar_type() == ws[i].scalar_type() && xs[i].scalar_type() == outs[i].scalar_type(), "b200ipc: dtype mismatch");
+    p[size_t(i)] = {xs[i].data_ptr(), ws[i].data_ptr(), outs[i].data_ptr(), nullptr};
+  }
+  c10::cuda::CUDAGuard guard(c.device());
+  return info_vec(local_allgather_gemm(c, dtype_of(xs[0]), p.data(), M, N, K, at::cuda::getCurrentCUDAStream(c.device())));
+}
+
 // ---- decode-step kernels (model/decode_ops.cu) --------------------------------------------------------
 int sm_count_of(int device) {
   int n = 0;
@@ -415,6 +465,11 @@ TORCH_LIBRARY(b200ipc, m) {
       "fused_gemm_ar(Tensor[] xs, Tensor[] ws, Tensor[] residuals, Tensor[] gammas, Tensor[] outs, Tensor[] res_outs, "
       "Tensor[] workspaces, float eps, bool with_norm, int comm, int ctas, bool local_only) -> int[]",
       &fused_gemm_ar);
+  m.def(
+      "local_gemm_ar(Tensor[] xs, Tensor[] ws, Tensor[] residuals, Tensor[] gammas, Tensor[] outs, Tensor[] res_outs, "
+      "float eps, bool with_norm, int comm) -> int[]",
+      &local_gemm_ar);
+  m.def("local_ag_gemm(Tensor[] xs, Tensor[] ws, Tensor[] outs, int comm) -> int[]", &local_ag_gemm);
   m.def("all_reduce(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_reduce);
   m.def("all_gather(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_gather);
   m.def("reduce_scatter(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int flags) -> int[]", &reduce_scatter);

@@ -255,9 +255,12 @@ class Communicator:
                          fused: Optional[bool] = None):
         """Row-parallel linear layer fused with its all-reduce in one tcgen05/TMA kernel.
 
-        fused=None picks by size: between 33 and 256 rows on four or more GPUs the framework's matmul followed by
-        `allreduce_residual_rmsnorm` measured ahead of the single kernel (8 GPUs, 128 rows: 40 us against 53 us),
-        so that pair runs there (plain weights with residual and gamma only); everything else takes the kernel.
+        fused=None picks: where this communicator drives every rank (a world of one, an emulated world) nothing has
+        to be exchanged, so plain weights take ONE GEMM over the ranks' concatenated K (fp32 sum, one rounding) and a
+        row norm behind it.  On several GPUs, between 33 and 256 rows on four or more of them, the framework's matmul
+        followed by `allreduce_residual_rmsnorm` measured ahead of the single kernel (8 GPUs, 128 rows: 40 us against
+        53 us), so that pair runs there (plain weights with residual and gamma only).  Everything else, and fused=True
+        or an explicit `ctas`, takes the kernel with the exchange.
 
         x: [M, K_local], weight: [N, K_local] (nn.Linear layout) of this rank, or that weight packed once by
         `pack_weight` (faster, most of all at decode sizes).  Returns
@@ -268,6 +271,7 @@ class Communicator:
         xs = [t.contiguous() for t in self._lists(x)]
         ws = [t.contiguous() for t in self._lists(weight)]
         M, N = xs[0].shape[0], ws[0].shape[0] * (64 if ws[0].dim() == 4 else 1)  # 4-D: packed by pack_weight
+        local = fused is None and ctas == 0 and self.nlocal == self.world and ws[0].dim() == 2
         if fused is None:
             fused = not (32 < M <= 256 and self.world >= 4 and not self._virtual and ws[0].dim() == 2
                          and residual is not None and gamma is not None)
@@ -277,20 +281,26 @@ class Communicator:
         key = (M, N, xs[0].dtype)
         cache = self.__dict__.setdefault("_gemm_buffers", {})
         if key not in cache:
+            # two sets of outputs, used in turn: the `res_out` of one call can be the `residual` of the next
+            cache[key] = [None, [(self.empty([M, N], xs[0].dtype), self.empty([M, N], xs[0].dtype)) for _ in range(2)], 0]
+        entry = cache[key]
+        if entry[0] is None and not local:
             nbytes = self._C.gemm_ar_workspace_bytes(self.world, M, N)
-            wsp = self.empty([nbytes // 2], torch.float16)
-            for t in (wsp if self._virtual else [wsp]):
+            entry[0] = self.empty([nbytes // 2], torch.float16)
+            for t in (entry[0] if self._virtual else [entry[0]]):
                 t.zero_()
             torch.cuda.synchronize()
             self.barrier()  # nobody may push into a workspace that its owner is still clearing
-            # two sets of outputs, used in turn: the `res_out` of one call can be the `residual` of the next
-            cache[key] = [wsp, [(self.empty([M, N], xs[0].dtype), self.empty([M, N], xs[0].dtype)) for _ in range(2)], 0]
-        entry = cache[key]
         wsp, (out, res_out) = entry[0], entry[1][entry[2]]
         entry[2] ^= 1
         L = (lambda t: t) if self._virtual else (lambda t: [t])
         with_norm = gamma is not None
         want_res = residual is not None
+        if local:
+            v = torch.ops.b200ipc.local_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
+                                                L(out), L(res_out) if want_res else [], eps, with_norm, self._h)
+            self.last_info = CollInfo.from_vec(v)
+            return (out, res_out) if with_norm or want_res else out
         v = torch.ops.b200ipc.fused_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
                                             L(out), L(res_out) if want_res else [], L(wsp), eps, with_norm, self._h, ctas, False)
         self.last_info = CollInfo.from_vec(v)
@@ -329,8 +339,9 @@ class Communicator:
     def allgather_linear(self, x_shard: TensorOrList, weight: TensorOrList, *, ctas: int = 0, fused: Optional[bool] = None):
         """Column-parallel linear layer on row-sharded activations, all-gather fused into the GEMM kernel.
 
-        fused=None picks by size: the fused kernel from 4096 gathered rows up (level with cuBLAS + NCCL at 8192
-        rows on 8 GPUs); below that this library's all-gather followed by the framework's matmul, which measured
+        fused=None picks: where this communicator drives every rank (a world of one, an emulated world) the GEMM reads the
+        shards where they are.  On several GPUs the fused kernel from 4096 gathered rows up (level with cuBLAS + NCCL at
+        8192 rows on 8 GPUs); below that this library's all-gather followed by the framework's matmul, which measured
         ahead of both the fused kernel and NCCL + cuBLAS (128 rows: 49 us against 60 and 55).
 
         x_shard: [M / world, K] (this rank's rows), weight: [N_local, K].  Returns `concat(x_shards) @ weight.T`,
@@ -341,6 +352,15 @@ class Communicator:
         M, K, N = xs[0].shape[0] * self.world, xs[0].shape[1], ws[0].shape[0]
         if fused is None:
             fused = M >= 4096 or self.world == 1
+            # below 4096 rows the pair of calls also takes what the kernel does not: any N and K, unaligned rows, a
+            # weight that wants a gradient
+            fits = fused or (N % 64 == 0 and K % 8 == 0 and not any(t.data_ptr() % 16 for t in xs + ws)
+                             and not (torch.is_grad_enabled() and any(t.requires_grad for t in ws)))
+            if fits and ctas == 0 and self.nlocal == self.world:
+                outs = [torch.empty(M, N, dtype=t.dtype, device=t.device) for t in xs]
+                v = torch.ops.b200ipc.local_ag_gemm(xs, ws, outs, self._h)
+                self.last_info = CollInfo.from_vec(v)
+                return self._ret(x_shard, outs)
         if not fused:
             gathered = self.all_gather(xs if self._virtual else xs[0], None, "allgather_auto")
             gs = gathered if self._virtual else [gathered]
@@ -407,6 +427,8 @@ class Communicator:
         no flag left by an interrupted launch can be taken for a later one."""
         self._C.reset(self._h)
         for entry in self.__dict__.get("_gemm_buffers", {}).values():
+            if entry[0] is None:
+                continue
             for t in (entry[0] if self._virtual else [entry[0]]):
                 t.zero_()
         torch.cuda.synchronize()

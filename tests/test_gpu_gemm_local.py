@@ -1,0 +1,105 @@
+"""The GEMM of a process that drives every rank (linear + all-reduce, all-gather + linear), at the edges of its tiles, splits
+and shards, against fp64 products.  fp32 sums of K products of N(0, 1) x N(0, 0.02) are off by less than K * 2^-24 * 0.02 * 4
+(at most 2e-5 here), the one rounding to 16 bit by half a unit in the last place."""
+import pytest
+import torch
+
+from gpu_ipc_example_b200 import Communicator
+
+pytestmark = pytest.mark.gpu
+HALF_ULP = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+def _rand(g, dtype, *shape, scale=1.0):
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).to(dtype)
+
+
+def _close(got, want, dtype):
+    torch.testing.assert_close(got.double(), want, atol=1e-4, rtol=1.01 * HALF_ULP[dtype])
+
+
+# one row, the edges of the 32-row tile steps, several tiles of rows, K that does not fill a 64-column block, N that does
+# not fill a 256-row tile of W, few blocks per K split, ranks that meet inside a stage
+@pytest.mark.parametrize("world,M,K,N", [(1, 1, 64, 64), (1, 31, 72, 192), (1, 33, 3584, 1024), (1, 257, 1000, 320), (1, 2048, 448, 1152),
+                                         (2, 16, 4096, 512), (2, 300, 200, 704), (4, 97, 8, 1024), (8, 5, 1032, 8192)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_linear(world, M, K, N, dtype):
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    xs = [_rand(g, dtype, M, K) for _ in range(world)]
+    ws = [_rand(g, dtype, N, K, scale=0.02) for _ in range(world)]
+    res = [_rand(g, dtype, M, N) for _ in range(world)]
+    gam = [1 + _rand(g, dtype, N, scale=0.1) for _ in range(world)]
+    y = sum(x.double() @ w.double().t() for x, w in zip(xs, ws))
+    with Communicator.virtual(world, 0, staging_bytes=96 << 20) as comm:
+        for o in comm.linear_allreduce(xs, ws):
+            _close(o, y, dtype)
+        for o, s, r in zip(*comm.linear_allreduce(xs, ws, res), res):
+            _close(s, y + r.double(), dtype)
+            assert torch.equal(o, s)
+        outs, sums = comm.linear_allreduce(xs, ws, res, gam, 1e-5)
+        for o, s, r, ga in zip(outs, sums, res, gam):
+            _close(s, y + r.double(), dtype)
+            want = s.double() * torch.rsqrt(s.double().pow(2).mean(-1, keepdim=True) + 1e-5) * ga.double()
+            _close(o, want, dtype)
+        norm_only, _ = comm.linear_allreduce(xs, ws, None, gam, 1e-5)  # the sum is normalised where it lies
+        for o, ga in zip(norm_only, gam):
+            want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * ga.double()
+            # two roundings: the sum's and the result's, and the statistic is taken from the rounded sums
+            torch.testing.assert_close(o.double(), want, atol=2e-3, rtol=3 * HALF_ULP[dtype])
+        torch.cuda.synchronize()
+        comm.check()
+
+
+# all shards in one tile (with padding rows between them and without), the largest such tile, one tile per shard, several
+@pytest.mark.parametrize("world,rows,K,N", [(1, 3, 512, 64), (2, 1, 520, 320), (2, 128, 64, 256), (2, 129, 256, 448), (4, 8, 1000, 1024),
+                                            (4, 13, 192, 7168), (4, 65, 128, 64), (2, 600, 328, 512), (1, 4100, 136, 256), (8, 9, 96, 128)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gather_linear(world, rows, K, N, dtype):
+    g = torch.Generator(device="cuda").manual_seed(rows + K)
+    xs = [_rand(g, dtype, rows, K) for _ in range(world)]
+    ws = [_rand(g, dtype, N, K, scale=0.02) for _ in range(world)]
+    full = torch.cat(xs).double()
+    with Communicator.virtual(world, 0, staging_bytes=32 << 20) as comm:
+        for o, w in zip(comm.allgather_linear(xs, ws), ws):
+            _close(o, full @ w.double().t(), dtype)
+        torch.cuda.synchronize()
+        comm.check()
+
+
+def test_what_the_kernel_does_not_take_still_runs():
+    """Below 4096 rows an all-gather followed by the framework's matmul took any N and K, unaligned rows and a weight that
+    wants a gradient; it still does."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    with Communicator.virtual(2, 0, staging_bytes=32 << 20) as comm:
+        for K, N, off in ((128, 40, 0), (36, 64, 0), (128, 64, 1)):
+            flat = [_rand(g, torch.float16, 8 * K + 8) for _ in range(2)]
+            xs = [f[off:off + 8 * K].view(8, K) for f in flat]
+            ws = [_rand(g, torch.float16, N, K, scale=0.02) for _ in range(2)]
+            for o, w in zip(comm.allgather_linear(xs, ws), ws):
+                torch.testing.assert_close(o.double(), torch.cat(xs).double() @ w.double().t(), atol=2e-3, rtol=2e-3)
+        ws = [w.detach().requires_grad_() for w in (_rand(g, torch.float16, 64, 128), _rand(g, torch.float16, 64, 128))]
+        outs = comm.allgather_linear([_rand(g, torch.float16, 8, 128) for _ in range(2)], ws)
+        outs[1].float().sum().backward()
+        assert ws[1].grad is not None
+
+
+@pytest.mark.parametrize("world", [1, 2, 8])
+@pytest.mark.parametrize("M", [1, 32, 40, 300])
+def test_the_kernels_with_the_exchange(world, M):
+    """fused=True: what runs with one process per GPU, on an emulated world.  Every rank's partial product is rounded to the
+    element type before the sum."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    xs = [_rand(g, torch.float16, M, 320) for _ in range(world)]
+    ws = [_rand(g, torch.float16, 1024, 320, scale=0.02) for _ in range(world)]
+    res, gam = _rand(g, torch.float16, M, 1024), 1 + _rand(g, torch.float16, 1024, scale=0.1)
+    with Communicator.virtual(world, 0, staging_bytes=96 << 20) as comm:
+        for _ in range(2):
+            comm.linear_allreduce(xs, ws, [res] * world, [gam] * world)  # the two forms take turns on one set of outputs
+            outs, sums = comm.linear_allreduce(xs, ws, [res] * world, [gam] * world, fused=True)
+            torch.cuda.synchronize()
+            comm.check()
+            y = sum((x.double() @ w.double().t()).half().double() for x, w in zip(xs, ws)) + res.double()
+            for o, s in zip(outs, sums):
+                torch.testing.assert_close(s.double(), y, atol=2e-3, rtol=2e-3)
+                want = s.double() * torch.rsqrt(s.double().pow(2).mean(-1, keepdim=True) + 1e-5) * gam.double()
+                torch.testing.assert_close(o.double(), want, atol=2e-3, rtol=2e-3)

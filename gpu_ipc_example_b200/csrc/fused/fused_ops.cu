@@ -4,6 +4,7 @@
 #include <cstring>
 
 #include "../common/check.h"
+#include "norm_direct.cuh"
 #include "oneshot_fused.cuh"
 
 namespace b200ipc {
@@ -21,10 +22,88 @@ KernelFn pick_world(int world) {
   }
 }
 
+// Vectors of a row that one CTA of the direct kernel can hold.
+int64_t direct_norm_cta_vecs(int world) { return (world == 8 ? 1 : 2) * kDirectNormThreads; }
+template <typename T, int N>
+const void* direct_norm_fn(int u) {
+  if constexpr (N < 8) {
+    if (u == 2) return reinterpret_cast<const void*>(&direct_norm_kernel<T, N, 2>);
+  }
+  return reinterpret_cast<const void*>(&direct_norm_kernel<T, N, 1>);
+}
+template <typename T>
+const void* direct_norm_lookup(int world, int u) {
+  switch (world) {
+    case 1: return direct_norm_fn<T, 1>(u);
+    case 2: return direct_norm_fn<T, 2>(u);
+    case 4: return direct_norm_fn<T, 4>(u);
+    case 8: return direct_norm_fn<T, 8>(u);
+    default: return nullptr;
+  }
+}
+
 uint32_t float_bits(float f) {
   uint32_t u;
   std::memcpy(&u, &f, 4);
   return u;
+}
+
+// One launch, clusters of `parts` CTAs per row.
+CollInfo direct_norm(Comm& comm, DType t, const FusedNormPtrs* ptrs, int64_t rows, int64_t hidden, float eps, cudaStream_t stream) {
+  const int N = comm.world();
+  const int64_t vecs = hidden / 8;
+  // as many CTAs per row as it takes to have a CTA on every SM, each with a warp's worth of vectors at least
+  const int64_t most = direct_norm_cta_vecs(N);
+  int64_t parts = 1;
+  while (parts < kDirectNormMaxParts &&
+         (ceil_div64(vecs, parts) > most || (rows * parts * 2 <= comm.sm_count() && ceil_div64(vecs, parts * 2) >= 32)))
+    parts *= 2;
+  const int64_t part_vecs = ceil_div64(vecs, parts);
+  const int u = part_vecs > kDirectNormThreads ? 2 : 1;
+  const int threads = int(round_up64(ceil_div64(part_vecs, u), 32));
+  B200_REQUIRE(part_vecs <= int64_t(u) * threads && threads <= kDirectNormThreads && rows * parts <= INT32_MAX, "row too long or too many rows");
+  DirectNormArgs args;
+  std::memset(&args, 0, sizeof(args));
+  for (int i = 0; i < N; ++i) {
+    args.x[i] = ptrs[i].x;
+    args.residual[i] = ptrs[i].residual;
+    args.gamma[i] = ptrs[i].gamma;
+    args.out[i] = ptrs[i].out;
+    args.res_out[i] = ptrs[i].residual_out;
+  }
+  args.row_vecs = int(vecs);
+  args.part_vecs = int(part_vecs);
+  args.hidden = float(hidden);
+  args.eps = eps;
+  const void* fn = t == DType::F16 ? direct_norm_lookup<__half>(N, u) : direct_norm_lookup<__nv_bfloat16>(N, u);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(rows * parts));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(parts);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2u : 1u;
+  void* params[] = {&args};
+  B200_CUDA_CHECK(cudaLaunchKernelExC(&cfg, fn, params));
+  comm.note_launch();
+  CollInfo info;
+  info.sched = SchedKind::Bulk;
+  info.proto = ProtoKind::LL512;
+  info.ctas = int(cfg.gridDim.x);
+  info.warps = threads / 32;
+  info.nwires = info.ctas * info.warps;
+  info.steps = u;
+  info.launches = 1;
+  return info;
+}
+bool direct_norm_ok(const Comm& comm, int64_t hidden) {
+  return comm.nlocal() == comm.world() && direct_norm_lookup<__half>(comm.world(), 1) != nullptr &&
+         hidden / 8 <= kDirectNormMaxParts * direct_norm_cta_vecs(comm.world());
 }
 
 }  // namespace
@@ -33,6 +112,13 @@ CollInfo fused_allreduce_residual_rmsnorm(Comm& comm, DType t, const FusedNormPt
                                           float eps, int ctas_req, cudaStream_t stream) {
   B200_REQUIRE(rows > 0 && hidden > 0 && hidden % 8 == 0, "hidden must be a positive multiple of 8");
   const int N = comm.world();
+  for (int i = 0; i < comm.nlocal(); ++i)
+    for (const void* p : {ptrs[i].x, ptrs[i].residual, ptrs[i].gamma, static_cast<const void*>(ptrs[i].out),
+                          static_cast<const void*>(ptrs[i].residual_out)})
+      B200_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, "fused all-reduce + RMSNorm needs 16-byte aligned tensors");
+  // Every rank is driven by this process: no exchange (an explicit CTA count asks for the kernel with it).  8 ranks, 16 rows
+  // of 8192: 8.x us against 97.
+  if (ctas_req == 0 && direct_norm_ok(comm, hidden)) return direct_norm(comm, t, ptrs, rows, hidden, eps, stream);
   KernelFn fn = t == DType::F16 ? pick_world<__half, __half, kEpiNorm>(N) : pick_world<__nv_bfloat16, __nv_bfloat16, kEpiNorm>(N);
   B200_REQUIRE(fn != nullptr, "no fused kernel for world size " << N);
   B200_CUDA_CHECK(cudaSetDevice(comm.device()));
@@ -57,9 +143,6 @@ CollInfo fused_allreduce_residual_rmsnorm(Comm& comm, DType t, const FusedNormPt
   for (int i = 0; i < comm.nlocal(); ++i) {
     ins[size_t(i)] = ptrs[i].x;
     outs[size_t(i)] = ptrs[i].out;
-    for (const void* p : {ptrs[i].x, ptrs[i].residual, ptrs[i].gamma, static_cast<const void*>(ptrs[i].out),
-                          static_cast<const void*>(ptrs[i].residual_out)})
-      B200_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, "fused all-reduce + RMSNorm needs 16-byte aligned tensors");
   }
   KArgs args;
   comm.fill_views(&args, ins.data(), outs.data(), size_t(rows * hidden), 0);

@@ -198,7 +198,8 @@ class Communicator:
         """Returns (RMSNorm(all_reduce(x) + residual) * gamma, all_reduce(x) + residual).
 
         Decode-sized inputs (up to 256 KiB per rank) take ONE kernel: the one-shot flag-in-data exchange with the
-        add and the norm in its epilogue.  Larger ones (prefill) would push world - 1 copies of everything over the
+        add and the norm in its epilogue (where this communicator drives every rank - a world of one, an emulated world -
+        one kernel without an exchange at any size, unless `ctas` is given).  Larger ones (prefill) would push world - 1 copies of everything over the
         links that way, so they take the bandwidth-optimal all-reduce of `auto` followed by one fused add + RMSNorm
         kernel over the local result."""
         xs = self._lists(x)
@@ -208,12 +209,19 @@ class Communicator:
         rs2 = [t.reshape(-1, t.shape[-1]) for t in rs]
         if xs2[0].numel() * xs2[0].element_size() > self.fused_oneshot_max_bytes and self.world > 1:
             ins = [t.contiguous() for t in xs2]
+            if self._virtual and ctas == 0 and ins[0].shape[-1] % 8 == 0 and ins[0].shape[-1] <= 32768:
+                rs2, gs = [t.contiguous() for t in rs2], [t.contiguous() for t in gs]
+                if not any(t.data_ptr() % 16 for t in ins + rs2 + gs):
+                    return self._fused_norm(x, xs, ins, rs2, gs, eps, 0)
             summed = [torch.empty_like(t) for t in ins]  # x itself is left alone
             self.all_reduce(ins if self._virtual else ins[0], summed if self._virtual else summed[0], "auto")
             pairs = [torch.ops.b200ipc.add_rmsnorm(s, r.contiguous(), g.contiguous(), eps) for s, r, g in zip(summed, rs2, gs)]
             outs = [p[0].view(t.shape) for p, t in zip(pairs, xs)]
             res_outs = [p[1].view(t.shape) for p, t in zip(pairs, xs)]
             return self._ret(x, outs), self._ret(x, res_outs)
+        return self._fused_norm(x, xs, xs2, rs2, gs, eps, ctas)
+
+    def _fused_norm(self, x, xs, xs2, rs2, gs, eps, ctas):
         outs = [torch.empty_like(t) for t in xs2]
         res_outs = [torch.empty_like(t) for t in xs2]
         v = torch.ops.b200ipc.fused_ar_rmsnorm(xs2, rs2, gs, outs, res_outs, eps, self._h, ctas)

@@ -23,6 +23,7 @@ enum class BulkMode : int { AllReduce = 0, ReduceScatter = 1, AllGather = 2 };
 // aux[1] bits
 constexpr uint64_t kBulkCopyIn = 1;   // stage `in` into the symmetric buffer first
 constexpr uint64_t kBulkCopyOut = 2;  // copy the result from the symmetric buffer to `out`
+constexpr uint64_t kBulkNoMeet = 4;   // Direct: the ranks do not meet (the launch need not be cooperative)
 
 // Where the ranks' data lives.  Heap: at one offset of every rank's symmetric heap.  Direct: in the callers' own
 // buffers, which every rank of an emulated world can address (the launch arguments hold all of them), so that
@@ -375,7 +376,9 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
   }
   // Every rank has arrived (so it has left the previous collective and, for the
   // reducing modes, its input is in place) before any remote access.
-  if (!cta_rank_barrier(me, lay, bar + 1, 10, /*publish=*/copy_in)) return;
+  // (Direct: all ranks are block rows of this one launch, which starts when every input is in place, and a rank only
+  // reads and writes its own shard of the buffers.  The barrier is for ranks that were told to send nothing.)
+  if ((P == BulkPlace::Heap || (me.aux[1] & kBulkNoMeet) == 0) && !cta_rank_barrier(me, lay, bar + 1, 10, /*publish=*/copy_in)) return;
 
   // ---- phase 1: the collective ---------------------------------------------------
   if constexpr (P == BulkPlace::Direct) {

@@ -310,15 +310,15 @@ int Comm::resident_ctas(KernelFn fn, int threads, size_t smem) {
   return total;
 }
 
-void Comm::launch(KernelFn fn, int ctas, int threads, KArgs* args, size_t smem, cudaStream_t stream, bool pdl) {
+void Comm::launch(KernelFn fn, int ctas, int threads, KArgs* args, size_t smem, cudaStream_t stream, bool pdl, bool meet) {
   void* params[] = {args};
-  launch_raw(reinterpret_cast<const void*>(fn), ctas, threads, params, smem, stream, pdl);
+  launch_raw(reinterpret_cast<const void*>(fn), ctas, threads, params, smem, stream, pdl, meet);
 }
 
-void Comm::launch_raw(const void* fn, int ctas, int threads, void** params, size_t smem, cudaStream_t stream, bool pdl) {
+void Comm::launch_raw(const void* fn, int ctas, int threads, void** params, size_t smem, cudaStream_t stream, bool pdl, bool meet) {
   dim3 grid(unsigned(ctas), unsigned(nlocal()), 1);
   dim3 block(unsigned(threads), 1, 1);
-  if (nlocal() > 1) {
+  if (nlocal() > 1 && meet) {
     // ranks wait on each other inside the kernel: all block rows must be resident
     B200_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, grid, block, params, smem, stream));
   } else {
@@ -611,13 +611,14 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
 
   KArgs args;
   fill_views(&args, ins, outs, nelems, flags);
-  const uint32_t bar = take_barrier();
+  const bool meet = !direct || (flags & kMuteSends) != 0;
+  const uint32_t bar = meet ? take_barrier() : 0;
   for (int i = 0; i < nlocal(); ++i) {
     args.v[i].bar_seq = bar;
     args.v[i].aux[0] = sym_off;
-    args.v[i].aux[1] = copy_flags;
+    args.v[i].aux[1] = copy_flags | (meet ? 0 : kBulkNoMeetBit);
   }
-  launch(fn, ctas, threads, &args, 0, stream);
+  launch(fn, ctas, threads, &args, 0, stream, false, meet);
 
   CollInfo info;
   info.sched = nvls ? SchedKind::Nvls : SchedKind::Bulk;
@@ -635,7 +636,14 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
 // ----------------------------------------------------------------------------
 // Public collectives
 // ----------------------------------------------------------------------------
-AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric, bool direct) const {
+// Emulated worlds: up to this many bytes `auto` takes the flag-in-data kernels.  The direct kernel is ahead at every size when
+// its ranks need not meet; a call with flags (rounding after each add, muted ranks) and a communicator that was moved to the
+// 8-byte-granule formats keep what is measured for the form with the barrier.
+size_t Comm::flag_max_bytes(EmuOp op, uint32_t flags) const {
+  return flags == 0 && !safe_protos_ ? 0 : emulated_flag_max_bytes(op, world_);
+}
+
+AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric, bool direct, uint32_t flags) const {
   AlgoSpec a;
   if (const char* e = std::getenv("B200IPC_PROTO")) {
     bool ag = false;
@@ -656,7 +664,7 @@ AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric, bool direct) cons
     }
     return a;
   }
-  if (direct && bytes > emulated_flag_max_bytes(EmuOp::AllReduce, world_)) {
+  if (direct && bytes > flag_max_bytes(EmuOp::AllReduce, flags)) {
     a.sched = SchedKind::Bulk;
     a.proto = ProtoKind::LL512;
     return a;
@@ -689,7 +697,7 @@ CollInfo Comm::all_reduce(AlgoSpec algo, DType t, const void* const* ins, void* 
   if (algo.automatic) {
     bool symmetric = true;
     for (int i = 0; i < nlocal(); ++i) symmetric &= (ins[i] == outs[i]) && sym_offset_of(ins[i], i) != SIZE_MAX;
-    algo = choose_all_reduce(nelems * 2, symmetric, bulk_direct_ok(BulkModeId::AllReduce, ins, outs, nelems));
+    algo = choose_all_reduce(nelems * 2, symmetric, bulk_direct_ok(BulkModeId::AllReduce, ins, outs, nelems), extra_flags);
   }
   for (int i = 0; i < nlocal(); ++i) {
     B200_REQUIRE((reinterpret_cast<uintptr_t>(ins[i]) & 3) == 0 && (reinterpret_cast<uintptr_t>(outs[i]) & 3) == 0,
@@ -720,7 +728,7 @@ CollInfo Comm::all_gather(AlgoSpec algo, DType t, const void* const* ins, void* 
   if (algo.automatic) {
     algo = AlgoSpec{};
     const size_t bytes = nelems * 2;
-    const bool direct = nelems % 2 == 0 && bytes > emulated_flag_max_bytes(EmuOp::AllGather, world_) &&
+    const bool direct = nelems % 2 == 0 && bytes > flag_max_bytes(EmuOp::AllGather, extra_flags) &&
                         bulk_direct_ok(BulkModeId::AllGather, ins, outs, nelems);
     // two ranks: the direct flag-in-data push moves the same bytes as any other form and needs no
     // barrier; measured ahead of the barrier-based kernels and of NCCL up to 64 MiB per rank
@@ -760,7 +768,7 @@ CollInfo Comm::reduce_scatter(AlgoSpec algo, DType t, const void* const* ins, vo
   const bool was_auto = algo.automatic;
   if (algo.automatic) {
     algo = AlgoSpec{};
-    const bool direct = nelems % size_t(world_) == 0 && nelems * 2 > emulated_flag_max_bytes(EmuOp::ReduceScatter, world_) &&
+    const bool direct = nelems % size_t(world_) == 0 && nelems * 2 > flag_max_bytes(EmuOp::ReduceScatter, extra_flags) &&
                         bulk_direct_ok(BulkModeId::ReduceScatter, ins, outs, nelems);
     // small inputs: one flag-in-data push to each slice's owner, no barrier
     if (direct) {

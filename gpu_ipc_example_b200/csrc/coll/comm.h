@@ -24,6 +24,7 @@
 
 #include "../mem/symm_heap.h"
 #include "kernel_table.h"
+#include "tuner.h"
 
 namespace b200ipc {
 
@@ -106,7 +107,8 @@ class Comm {
   // Size -> algorithm choice used for AlgoSpec::automatic: the measured table of tuner.h unless
   // set_thresholds() installed explicit cut-offs (0, 0 restores the table).
   // `direct`: an emulated world whose buffers the barrier-based kernel can use as they are.
-  AlgoSpec choose_all_reduce(size_t bytes, bool symmetric, bool direct = false) const;
+  AlgoSpec choose_all_reduce(size_t bytes, bool symmetric, bool direct = false, uint32_t flags = 0) const;
+  size_t flag_max_bytes(EmuOp op, uint32_t flags) const;
   void set_thresholds(size_t oneshot_max_bytes, size_t ll_max_bytes) {
     oneshot_max_bytes_ = oneshot_max_bytes;
     ll_max_bytes_ = ll_max_bytes;
@@ -149,14 +151,16 @@ class Comm {
 
   // Launch plumbing shared with the fused ops.
   void fill_views(KArgs* args, const void* const* ins, void* const* outs, size_t nelems, uint32_t flags) const;
-  void launch(KernelFn fn, int ctas, int threads, KArgs* args, size_t smem, cudaStream_t stream, bool pdl = false);
+  void launch(KernelFn fn, int ctas, int threads, KArgs* args, size_t smem, cudaStream_t stream, bool pdl = false, bool meet = true);
   int resident_ctas(KernelFn fn, int threads, size_t smem);
   uint32_t take_seq(uint32_t advance);
   uint32_t take_barrier();
   // Launch with caller-built parameters (cooperative when this communicator drives several ranks).
   // pdl: the kernel executes griddepcontrol.wait before it touches anything an earlier kernel wrote, so it may be
   // launched with programmatic stream serialisation (single-rank launches only; see common/pdl.h)
-  void launch_raw(const void* fn, int ctas, int threads, void** params, size_t smem, cudaStream_t stream, bool pdl = false);
+  // meet: block rows (emulated ranks) wait on one another inside the kernel, so that all have to be resident.
+  void launch_raw(const void* fn, int ctas, int threads, void** params, size_t smem, cudaStream_t stream, bool pdl = false,
+                  bool meet = true);
   // Running total of the delivery counter of the fused GEMM kernels: returns the value the
   // counter reaches after `inc` more deliveries.
   uint32_t take_done(uint32_t inc) {

@@ -101,12 +101,13 @@ CollInfo direct_norm(Comm& comm, DType t, const FusedNormPtrs* ptrs, int64_t row
   info.launches = 1;
   return info;
 }
-bool direct_norm_ok(const Comm& comm, int64_t hidden) {
-  return comm.nlocal() == comm.world() && direct_norm_lookup<__half>(comm.world(), 1) != nullptr &&
-         hidden / 8 <= kDirectNormMaxParts * direct_norm_cta_vecs(comm.world());
-}
 
 }  // namespace
+
+bool direct_norm_takes(const Comm& comm, int64_t hidden) {
+  return comm.nlocal() == comm.world() && hidden > 0 && hidden % 8 == 0 && direct_norm_lookup<__half>(comm.world(), 1) != nullptr &&
+         hidden / 8 <= kDirectNormMaxParts * direct_norm_cta_vecs(comm.world());
+}
 
 CollInfo fused_allreduce_residual_rmsnorm(Comm& comm, DType t, const FusedNormPtrs* ptrs, int64_t rows, int64_t hidden,
                                           float eps, int ctas_req, cudaStream_t stream) {
@@ -118,7 +119,7 @@ CollInfo fused_allreduce_residual_rmsnorm(Comm& comm, DType t, const FusedNormPt
       B200_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, "fused all-reduce + RMSNorm needs 16-byte aligned tensors");
   // Every rank is driven by this process: no exchange (an explicit CTA count asks for the kernel with it).  8 ranks, 16 rows
   // of 8192: 8.x us against 97.
-  if (ctas_req == 0 && direct_norm_ok(comm, hidden)) return direct_norm(comm, t, ptrs, rows, hidden, eps, stream);
+  if (ctas_req == 0 && direct_norm_takes(comm, hidden)) return direct_norm(comm, t, ptrs, rows, hidden, eps, stream);
   KernelFn fn = t == DType::F16 ? pick_world<__half, __half, kEpiNorm>(N) : pick_world<__nv_bfloat16, __nv_bfloat16, kEpiNorm>(N);
   B200_REQUIRE(fn != nullptr, "no fused kernel for world size " << N);
   B200_CUDA_CHECK(cudaSetDevice(comm.device()));

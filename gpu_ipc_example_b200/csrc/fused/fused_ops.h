@@ -21,6 +21,10 @@ struct FusedNormPtrs {
 CollInfo fused_allreduce_residual_rmsnorm(Comm& comm, DType t, const FusedNormPtrs* ptrs, int64_t rows, int64_t hidden,
                                           float eps, int ctas, cudaStream_t stream);
 
+// Whether that runs as one kernel without an exchange, for any number of rows (unless `ctas` is given): this process drives
+// every rank, and a row fits the registers of a cluster.
+bool direct_norm_takes(const Comm& comm, int64_t hidden);
+
 // out = cast<tout>(all_reduce(in) * scale).
 CollInfo fused_allreduce_scale_cast(Comm& comm, DType tin, DType tout, const void* const* ins, void* const* outs,
                                     size_t nelems, float scale, int ctas, cudaStream_t stream);

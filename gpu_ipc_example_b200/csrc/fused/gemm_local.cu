@@ -2,6 +2,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 #include "../common/check.h"
@@ -70,6 +71,14 @@ double plan_cost(int64_t tiles, int64_t room, int64_t kb_total, int bn, int spli
 
 // The tile height and the K split of a problem.  bn_only: the tile's height is given (merged shards).
 LocalPlan plan_local(DType t, int device, int64_t rows, int64_t shards, int64_t groups, int64_t N, int64_t kb_total, int bn_only) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int64_t, int64_t, int64_t, int64_t, int64_t, int>, LocalPlan> plans;
+  const auto key = std::make_tuple(int(t), device, rows, shards, groups, N, kb_total, bn_only);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = plans.find(key);
+    if (it != plans.end()) return it->second;
+  }
   LocalPlan best;
   double best_cost = 0;
   const int64_t n_tiles = ceil_div64(N, kLocWRows);
@@ -90,6 +99,9 @@ LocalPlan plan_local(DType t, int device, int64_t rows, int64_t shards, int64_t 
       }
     }
   }
+  std::lock_guard<std::mutex> lk(mu);
+  if (plans.size() >= 1024) plans.clear();  // a plan depends on nothing but its key and costs microseconds
+  plans[key] = best;
   return best;
 }
 

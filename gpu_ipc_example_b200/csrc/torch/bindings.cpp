@@ -139,7 +139,7 @@ std::vector<int64_t> info_vec(const CollInfo& i) {
           int64_t(i.staged)};
 }
 
-std::vector<int64_t> all_reduce(std::vector<at::Tensor> ins, std::vector<at::Tensor> outs, int64_t comm_id,
+std::vector<int64_t> all_reduce(const std::vector<at::Tensor>& ins, const std::vector<at::Tensor>& outs, int64_t comm_id,
                                 const std::string& algo, int64_t ctas, int64_t warps, int64_t flags) {
   Comm& c = get(comm_id);
   check_tensors(c, ins, "input");
@@ -159,7 +159,7 @@ std::vector<int64_t> all_reduce(std::vector<at::Tensor> ins, std::vector<at::Ten
   return info_vec(info);
 }
 
-std::vector<int64_t> all_gather(std::vector<at::Tensor> ins, std::vector<at::Tensor> outs, int64_t comm_id,
+std::vector<int64_t> all_gather(const std::vector<at::Tensor>& ins, const std::vector<at::Tensor>& outs, int64_t comm_id,
                                 const std::string& algo, int64_t ctas, int64_t warps, int64_t flags) {
   Comm& c = get(comm_id);
   check_tensors(c, ins, "input");
@@ -178,7 +178,7 @@ std::vector<int64_t> all_gather(std::vector<at::Tensor> ins, std::vector<at::Ten
   return info_vec(info);
 }
 
-std::vector<int64_t> reduce_scatter(std::vector<at::Tensor> ins, std::vector<at::Tensor> outs, int64_t comm_id,
+std::vector<int64_t> reduce_scatter(const std::vector<at::Tensor>& ins, const std::vector<at::Tensor>& outs, int64_t comm_id,
                                     const std::string& algo, int64_t ctas, int64_t flags) {
   Comm& c = get(comm_id);
   check_tensors(c, ins, "input");
@@ -196,6 +196,53 @@ std::vector<int64_t> reduce_scatter(std::vector<at::Tensor> ins, std::vector<at:
   CollInfo info = c.reduce_scatter(a, dtype_of(ins[0]), ip.data(), op.data(), size_t(ins[0].numel()), g,
                                    at::cuda::getCurrentCUDAStream(c.device()), uint32_t(flags));
   return info_vec(info);
+}
+
+// ---- the list forms that Communicator calls: what the kernels ask of their buffers (contiguous, 16-byte aligned) is seen to
+// here, and outputs that the caller did not bring are allocated here.
+bool fits_kernels(const at::Tensor& t) { return t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+at::Tensor aligned(const at::Tensor& t) {
+  at::Tensor c = t.contiguous();
+  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) == 0 ? c : c.clone();
+}
+
+// outs empty: in place.
+std::vector<int64_t> all_reduce_lists(const std::vector<at::Tensor>& ins, const std::vector<at::Tensor>& outs, int64_t comm_id,
+                                      const std::string& algo, int64_t ctas, int64_t warps, int64_t flags) {
+  const bool in_place = outs.empty();
+  const std::vector<at::Tensor>& dst = in_place ? ins : outs;
+  bool plain = true;
+  for (const at::Tensor& t : ins) plain = plain && fits_kernels(t);
+  if (!in_place)
+    for (const at::Tensor& t : outs) plain = plain && fits_kernels(t);
+  if (plain) return all_reduce(ins, dst, comm_id, algo, ctas, warps, flags);
+  std::vector<at::Tensor> fi, fo;
+  for (const at::Tensor& t : ins) fi.push_back(aligned(t));
+  if (in_place)
+    fo = fi;
+  else
+    for (const at::Tensor& t : outs) fo.push_back(fits_kernels(t) ? t : at::empty_like(t, at::MemoryFormat::Contiguous));
+  std::vector<int64_t> v = all_reduce(fi, fo, comm_id, algo, ctas, warps, flags);
+  for (size_t i = 0; i < fo.size(); ++i)
+    if (!dst[i].is_same(fo[i])) dst[i].copy_(fo[i]);
+  return v;
+}
+
+std::vector<at::Tensor> aligned_list(const std::vector<at::Tensor>& ts) {
+  std::vector<at::Tensor> r;
+  r.reserve(ts.size());
+  for (const at::Tensor& t : ts) r.push_back(aligned(t));
+  return r;
+}
+
+std::vector<int64_t> all_gather_lists(const std::vector<at::Tensor>& ins, const std::vector<at::Tensor>& outs, int64_t comm_id,
+                                      const std::string& algo, int64_t ctas, int64_t warps, int64_t flags) {
+  return all_gather(aligned_list(ins), outs, comm_id, algo, ctas, warps, flags);
+}
+
+std::vector<int64_t> reduce_scatter_lists(const std::vector<at::Tensor>& ins, const std::vector<at::Tensor>& outs, int64_t comm_id,
+                                          const std::string& algo, int64_t ctas, int64_t flags) {
+  return reduce_scatter(aligned_list(ins), outs, comm_id, algo, ctas, flags);
 }
 
 // In-place single-tensor form, the shape `dist.all_reduce(t)` has.
@@ -245,6 +292,35 @@ std::vector<int64_t> fused_ar_rmsnorm(std::vector<at::Tensor> ins, std::vector<a
   CollInfo info = fused_allreduce_residual_rmsnorm(c, dtype_of(ins[0]), p.data(), rows, hidden, float(eps), int(ctas),
                                                    at::cuda::getCurrentCUDAStream(c.device()));
   return info_vec(info);
+}
+
+// The same for a process that drives every rank (one kernel without an exchange), outputs included: [outs..., residual
+// outs...], or nothing where that kernel does not take the call and the general route has to.
+std::tuple<std::vector<at::Tensor>, std::vector<int64_t>> ar_rmsnorm_lists(const std::vector<at::Tensor>& xs, const std::vector<at::Tensor>& residuals,
+                                         const std::vector<at::Tensor>& gammas, double eps, int64_t comm_id) {
+  Comm& c = get(comm_id);
+  const size_t n = size_t(c.nlocal());
+  if (xs.size() != n || residuals.size() != n || gammas.size() != n || xs[0].dim() < 1 || xs[0].numel() == 0) return {std::vector<at::Tensor>{}, std::vector<int64_t>{}};
+  const at::Tensor& x0 = xs[0];
+  const int64_t hidden = x0.size(-1);
+  if ((x0.scalar_type() != at::kHalf && x0.scalar_type() != at::kBFloat16) || !direct_norm_takes(c, hidden)) return {std::vector<at::Tensor>{}, std::vector<int64_t>{}};
+  auto takes = [&](const at::Tensor& t, int64_t numel) {
+    return t.is_cuda() && t.get_device() == c.device() && t.scalar_type() == x0.scalar_type() && t.numel() == numel && fits_kernels(t);
+  };
+  for (size_t i = 0; i < n; ++i)
+    if (!takes(xs[i], x0.numel()) || xs[i].dim() < 1 || xs[i].size(-1) != hidden || !takes(residuals[i], x0.numel()) ||
+        residuals[i].dim() < 1 || residuals[i].size(-1) != hidden || !takes(gammas[i], hidden))
+      return {std::vector<at::Tensor>{}, std::vector<int64_t>{}};
+  c10::cuda::CUDAGuard guard(c.device());
+  std::vector<at::Tensor> outs;
+  outs.reserve(2 * n);
+  for (size_t i = 0; i < 2 * n; ++i) outs.push_back(at::empty(xs[i % n].sizes(), xs[i % n].options()));
+  std::vector<FusedNormPtrs> p(n);
+  for (size_t i = 0; i < n; ++i)
+    p[i] = {xs[i].data_ptr(), residuals[i].data_ptr(), gammas[i].data_ptr(), outs[i].data_ptr(), outs[n + i].data_ptr()};
+  CollInfo info = fused_allreduce_residual_rmsnorm(c, dtype_of(x0), p.data(), x0.numel() / hidden, hidden, float(eps), 0,
+                                                   at::cuda::getCurrentCUDAStream(c.device()));
+  return {std::move(outs), info_vec(info)};
 }
 
 std::vector<int64_t> fused_ar_scale_cast(std::vector<at::Tensor> ins, std::vector<at::Tensor> outs, double scale,
@@ -470,6 +546,10 @@ TORCH_LIBRARY(b200ipc, m) {
       "float eps, bool with_norm, int comm) -> int[]",
       &local_gemm_ar);
   m.def("local_ag_gemm(Tensor[] xs, Tensor[] ws, Tensor[] outs, int comm) -> int[]", &local_ag_gemm);
+  m.def("all_reduce_lists(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_reduce_lists);
+  m.def("all_gather_lists(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_gather_lists);
+  m.def("reduce_scatter_lists(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int flags) -> int[]", &reduce_scatter_lists);
+  m.def("ar_rmsnorm_lists(Tensor[] xs, Tensor[] residuals, Tensor[] gammas, float eps, int comm) -> (Tensor[], int[])", &ar_rmsnorm_lists);
   m.def("all_reduce(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_reduce);
   m.def("all_gather(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_gather);
   m.def("reduce_scatter(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int flags) -> int[]", &reduce_scatter);

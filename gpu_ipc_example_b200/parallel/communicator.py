@@ -68,7 +68,11 @@ class Communicator:
         self.world = self._C.world(handle)
         self.nlocal = self._C.nlocal(handle)
         self.rank = self._C.rank(handle, 0)
-        self.last_info: Optional[CollInfo] = None
+        self._info = None  # the launch report of the last call, as the native code gives it
+        ops = torch.ops.b200ipc
+        self._all_reduce_lists, self._all_gather_lists = ops.all_reduce_lists.default, ops.all_gather_lists.default
+        self._reduce_scatter_lists, self._ar_rmsnorm_lists = ops.reduce_scatter_lists.default, ops.ar_rmsnorm_lists.default
+        self._local_gemm_ar, self._local_ag_gemm = ops.local_gemm_ar.default, ops.local_ag_gemm.default
         # largest input (bytes per rank) the one-shot all-reduce + residual + RMSNorm kernel is used for
         self.fused_oneshot_max_bytes = 256 << 10
 
@@ -126,6 +130,11 @@ class Communicator:
         self.close()
 
     # ------------------------------------------------------------------ helpers
+    @property
+    def last_info(self) -> Optional[CollInfo]:
+        """How the last call was launched."""
+        return None if self._info is None else CollInfo.from_vec(self._info)
+
     def _lists(self, x: TensorOrList) -> List[torch.Tensor]:
         if isinstance(x, torch.Tensor):
             if self.nlocal != 1:
@@ -157,40 +166,29 @@ class Communicator:
         """Sum over ranks.  In place unless `out` is given.  Stream-ordered on the current stream."""
         ins = self._lists(x)
         outs = ins if out is None else self._lists(out)
-        fixed_in = [self._aligned(t) for t in ins]
-        fixed_out = [o if (o.is_contiguous() and o.data_ptr() % 16 == 0) else torch.empty_like(o, memory_format=torch.contiguous_format)
-                     for o in outs]
-        if out is None:
-            fixed_out = [fi if fi is i else fi for fi, i in zip(fixed_in, ins)]
-        v = torch.ops.b200ipc.all_reduce(fixed_in, fixed_out, self._h, algo, ctas, warps, flags)
-        for o, f in zip(outs, fixed_out):
-            if o is not f:
-                o.copy_(f)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = self._all_reduce_lists(ins, [] if out is None else outs, self._h, algo, ctas, warps, flags)
         return self._ret(x, outs)
 
     def all_gather(self, x: TensorOrList, out: Optional[TensorOrList] = None, algo: str = "allgather_auto", *,
                    ctas: int = 0, warps: int = 0, flags: int = 0):
         """Rank-ordered concatenation along dim 0."""
-        ins = [self._aligned(t) for t in self._lists(x)]
+        ins = self._lists(x)
         if out is None:
             outs = [torch.empty((self.world * t.shape[0],) + tuple(t.shape[1:]), dtype=t.dtype, device=t.device) for t in ins]
         else:
             outs = self._lists(out)
-        v = torch.ops.b200ipc.all_gather(ins, outs, self._h, algo, ctas, warps, flags)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = self._all_gather_lists(ins, outs, self._h, algo, ctas, warps, flags)
         return self._ret(x, outs)
 
     def reduce_scatter(self, x: TensorOrList, out: Optional[TensorOrList] = None, algo: str = "auto", *, ctas: int = 0,
                        flags: int = 0):
         """Sum over ranks; rank r keeps the r-th of `world` equal slices along dim 0."""
-        ins = [self._aligned(t) for t in self._lists(x)]
+        ins = self._lists(x)
         if out is None:
             outs = [torch.empty((t.shape[0] // self.world,) + tuple(t.shape[1:]), dtype=t.dtype, device=t.device) for t in ins]
         else:
             outs = self._lists(out)
-        v = torch.ops.b200ipc.reduce_scatter(ins, outs, self._h, algo, ctas, flags)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = self._reduce_scatter_lists(ins, outs, self._h, algo, ctas, flags)
         return self._ret(x, outs)
 
     def allreduce_residual_rmsnorm(self, x: TensorOrList, residual: TensorOrList, gamma: TensorOrList, eps: float = 1e-5,
@@ -205,27 +203,27 @@ class Communicator:
         xs = self._lists(x)
         rs = self._lists(residual)
         gs = self._lists(gamma)
+        if ctas == 0 and self.nlocal == self.world:
+            both, info = self._ar_rmsnorm_lists(xs, rs, gs, eps, self._h)
+            if both:
+                self._info = info
+                if isinstance(x, torch.Tensor):
+                    return both[0], both[1]
+                return both[:self.nlocal], both[self.nlocal:]
         xs2 = [t.reshape(-1, t.shape[-1]) for t in xs]
         rs2 = [t.reshape(-1, t.shape[-1]) for t in rs]
         if xs2[0].numel() * xs2[0].element_size() > self.fused_oneshot_max_bytes and self.world > 1:
             ins = [t.contiguous() for t in xs2]
-            if self._virtual and ctas == 0 and ins[0].shape[-1] % 8 == 0 and ins[0].shape[-1] <= 32768:
-                rs2, gs = [t.contiguous() for t in rs2], [t.contiguous() for t in gs]
-                if not any(t.data_ptr() % 16 for t in ins + rs2 + gs):
-                    return self._fused_norm(x, xs, ins, rs2, gs, eps, 0)
             summed = [torch.empty_like(t) for t in ins]  # x itself is left alone
             self.all_reduce(ins if self._virtual else ins[0], summed if self._virtual else summed[0], "auto")
             pairs = [torch.ops.b200ipc.add_rmsnorm(s, r.contiguous(), g.contiguous(), eps) for s, r, g in zip(summed, rs2, gs)]
             outs = [p[0].view(t.shape) for p, t in zip(pairs, xs)]
             res_outs = [p[1].view(t.shape) for p, t in zip(pairs, xs)]
             return self._ret(x, outs), self._ret(x, res_outs)
-        return self._fused_norm(x, xs, xs2, rs2, gs, eps, ctas)
-
-    def _fused_norm(self, x, xs, xs2, rs2, gs, eps, ctas):
         outs = [torch.empty_like(t) for t in xs2]
         res_outs = [torch.empty_like(t) for t in xs2]
         v = torch.ops.b200ipc.fused_ar_rmsnorm(xs2, rs2, gs, outs, res_outs, eps, self._h, ctas)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = v
         outs = [o.view(t.shape) for o, t in zip(outs, xs)]
         res_outs = [o.view(t.shape) for o, t in zip(res_outs, xs)]
         return self._ret(x, outs), self._ret(x, res_outs)
@@ -236,7 +234,7 @@ class Communicator:
         xs = [self._aligned(t) for t in self._lists(x)]
         outs = [torch.empty_like(t, dtype=dtype or t.dtype) for t in xs]
         v = torch.ops.b200ipc.fused_ar_scale_cast(xs, outs, scale, self._h, ctas)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = v
         return self._ret(x, outs)
 
     @staticmethod
@@ -305,13 +303,13 @@ class Communicator:
         with_norm = gamma is not None
         want_res = residual is not None
         if local:
-            v = torch.ops.b200ipc.local_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
+            v = self._local_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
                                                 L(out), L(res_out) if want_res else [], eps, with_norm, self._h)
-            self.last_info = CollInfo.from_vec(v)
+            self._info = v
             return (out, res_out) if with_norm or want_res else out
         v = torch.ops.b200ipc.fused_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
                                             L(out), L(res_out) if want_res else [], L(wsp), eps, with_norm, self._h, ctas, False)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = v
         if with_norm or want_res:
             return out, res_out
         return out
@@ -341,7 +339,7 @@ class Communicator:
         wsp, out = cache[key]
         L = (lambda t: t) if self._virtual else (lambda t: [t])
         v = torch.ops.b200ipc.fused_gemm_ar(xs, ws, [], [], L(out), [], L(wsp), 0.0, False, self._h, ctas, True)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = v
         return out
 
     def allgather_linear(self, x_shard: TensorOrList, weight: TensorOrList, *, ctas: int = 0, fused: Optional[bool] = None):
@@ -366,8 +364,8 @@ class Communicator:
                              and not (torch.is_grad_enabled() and any(t.requires_grad for t in ws)))
             if fits and ctas == 0 and self.nlocal == self.world:
                 outs = [torch.empty(M, N, dtype=t.dtype, device=t.device) for t in xs]
-                v = torch.ops.b200ipc.local_ag_gemm(xs, ws, outs, self._h)
-                self.last_info = CollInfo.from_vec(v)
+                v = self._local_ag_gemm(xs, ws, outs, self._h)
+                self._info = v
                 return self._ret(x_shard, outs)
         if not fused:
             gathered = self.all_gather(xs if self._virtual else xs[0], None, "allgather_auto")
@@ -382,7 +380,7 @@ class Communicator:
         wsp = cache[key]
         outs = [torch.empty(M, N, dtype=t.dtype, device=t.device) for t in xs]
         v = torch.ops.b200ipc.fused_ag_gemm(xs, ws, outs, wsp if self._virtual else [wsp], self._h, ctas)
-        self.last_info = CollInfo.from_vec(v)
+        self._info = v
         return self._ret(x_shard, outs)
 
     # ------------------------------------------------------------------ symmetric memory

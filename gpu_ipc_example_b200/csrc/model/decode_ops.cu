@@ -50,6 +50,11 @@ void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t s
   B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 
+// Pair (x1, x2) turned by an angle.  Spelled out so that every kernel that rotates gives the same bits.
+__device__ __forceinline__ float2 rope_pair(float x1, float x2, float sn, float cs) {
+  return make_float2(fmaf(x1, cs, -__fmul_rn(x2, sn)), fmaf(x2, cs, __fmul_rn(x1, sn)));
+}
+
 // ---------------------------------------------------------------------------------------------
 // RoPE + cache append.  qkv: [B, (hq + 2 hkv) * D] as the QKV projection leaves it.  Rotates q in
 // place (pairs (i, i + D/2)), writes the rotated k and the v of the new position into the caches
@@ -71,7 +76,8 @@ __global__ void rope_kv_append_kernel(T* qkv, T* kcache, T* vcache, int hq, int 
       float sn, cs;
       sincosf(float(pos) * inv, &sn, &cs);
       const float x1 = float(row[i]), x2 = float(row[i + half]);
-      const T y1 = T(x1 * cs - x2 * sn), y2 = T(x2 * cs + x1 * sn);
+      const float2 y = rope_pair(x1, x2, sn, cs);
+      const T y1 = T(y.x), y2 = T(y.y);
       if (head < hq) {
         row[i] = y1;
         row[i + half] = y2;
@@ -148,11 +154,15 @@ __device__ __forceinline__ void load_row_quarter(uint32_t (&w)[16], const T* row
   }
 }
 
-template <typename T, int G>
-__global__ void __launch_bounds__(kAttnThreads, 2) decode_attention_kernel(const T* q, const T* kcache, const T* vcache, T* out,
+// ROPE: `q` is the whole row of the QKV projection [hq q heads, hkv k heads, hkv v heads], not yet rotated, and position
+// ctx - 1 of the caches is not written yet.  Every CTA rotates its G query heads into shared memory; the CTA whose share of
+// the context ends at ctx rotates the new k, and writes it and the new v into the caches before it reads them.  That takes
+// the place of a kernel in front of this one (3.4 us and a launch per layer).
+template <typename T, int G, bool ROPE>
+__global__ void __launch_bounds__(kAttnThreads, 2) decode_attention_kernel(const T* q, T* kcache, T* vcache, T* out,
                                                                            float* part, unsigned int* counters,
                                                                         int hq, int hkv, int max_ctx, int ctx, int q_row_stride,
-                                                                        float scale_log2) {
+                                                                        float scale_log2, float log2_theta) {
   using T2 = typename Num<T>::T2;
   pdl_launch_dependents();
   pdl_wait();
@@ -162,11 +172,42 @@ __global__ void __launch_bounds__(kAttnThreads, 2) decode_attention_kernel(const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = lane >> 2, c = lane & 3;
 
+  __shared__ __align__(16) T s_q[ROPE ? G * kAttnD : 8];
+  if constexpr (ROPE) {
+    constexpr int half = kAttnD / 2;
+    const T* row = q + size_t(b) * q_row_stride;
+    const int pos = ctx - 1, i = threadIdx.x & (half - 1), sub = threadIdx.x / half;  // pair i, two heads at a time
+    // angle = pos * theta^(-i / half), as in rope_kv_append_kernel
+    const float inv = exp2f(-log2_theta * float(i) / float(half));
+    float sn, cs;
+    sincosf(float(pos) * inv, &sn, &cs);
+    auto rotate = [&](const T* src, T* dst) {
+      const float2 y = rope_pair(float(src[i]), float(src[i + half]), sn, cs);
+      dst[i] = T(y.x);
+      dst[i + half] = T(y.y);
+    };
+#pragma unroll
+    for (int g = 0; g < G; g += kAttnThreads / half)
+      if (g + sub < G) rotate(row + (size_t(h) * G + g + sub) * kAttnD, s_q + (g + sub) * kAttnD);
+    const int own_per = ((ctx + nsplit - 1) / nsplit + kAttnTile - 1) / kAttnTile * kAttnTile;
+    if (pos / own_per == split) {
+      const size_t at = ((size_t(b) * hkv + h) * size_t(max_ctx) + size_t(pos)) * kAttnD;
+      if (sub == 0) {
+        rotate(row + (size_t(hq) + h) * kAttnD, kcache + at);
+      } else {
+        const T* v = row + (size_t(hq) + hkv + h) * kAttnD;
+        vcache[at + i] = v[i];
+        vcache[at + i + half] = v[i + half];
+      }
+    }
+    __syncthreads();  // also makes the new k and v visible to the loads of this CTA
+  }
+
   // Q operand: head r of this KV head's group (rows G..15 of the 16-row operand are zero)
   uint32_t qa[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) qa[i] = 0u;
-  if (r < G) load_row_quarter<T>(qa, q + size_t(b) * q_row_stride + (size_t(h) * G + r) * kAttnD, c);
+  if (r < G) load_row_quarter<T>(qa, ROPE ? s_q + r * kAttnD : q + size_t(b) * q_row_stride + (size_t(h) * G + r) * kAttnD, c);
 
   // running state of head r (every lane of the quad holds the same m; l is a per-lane partial sum)
   float m = -INFINITY, l = 0.f;
@@ -389,7 +430,56 @@ __global__ void silu_mul_kernel(const T* gu, T* act, int64_t rows, int F) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// res_out = x + residual ; out = RMSNorm(res_out) * gamma.  One CTA per row, one pass: the row's sum stays in
+// Greatest value and its index in every row (the first one of equal values; NaN is greater than everything), one CTA per
+// row: what `logits.float().max(-1)` gives, in one pass over 16-bit values instead of a copy and a reduction (batch 32,
+// 16032 columns: 16 us before).
+// ---------------------------------------------------------------------------------------------
+constexpr int kArgmaxThreads = 512;
+struct Best {
+  float v;
+  int i;
+};
+__device__ __forceinline__ Best better(Best a, Best b) {
+  const bool na = a.v != a.v, nb = b.v != b.v;
+  const bool take_b = nb ? (!na || b.i < a.i) : (!na && (b.v > a.v || (b.v == a.v && b.i < a.i)));
+  return take_b ? b : a;
+}
+template <typename T>
+__global__ void __launch_bounds__(kArgmaxThreads) row_argmax_kernel(const T* x, float* values, int64_t* indices, int cols) {
+  using T2 = typename Num<T>::T2;
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ Best s_best[kArgmaxThreads / 32];
+  const T* row = x + size_t(blockIdx.x) * size_t(cols);
+  Best best{-INFINITY, 0x7fffffff};
+  if ((size_t(cols) * sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    for (int v = threadIdx.x; v < cols / 8; v += kArgmaxThreads) {
+      const uint4 w = *reinterpret_cast<const uint4*>(row + v * 8);
+      const T2* p = reinterpret_cast<const T2*>(&w);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = Num<T>::up(p[e]);
+        best = better(best, Best{f.x, v * 8 + 2 * e});
+        best = better(best, Best{f.y, v * 8 + 2 * e + 1});
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < cols; i += kArgmaxThreads) best = better(best, Best{float(row[i]), i});
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    best = better(best, Best{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
+  if ((threadIdx.x & 31) == 0) s_best[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kArgmaxThreads / 32; ++w) best = better(best, s_best[w]);
+    values[blockIdx.x] = best.v;
+    indices[blockIdx.x] = best.i;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// res_out = x + residual ; out = RMSNorm(res_out) * gamma (residual nullptr: out = RMSNorm(x) * gamma).  One CTA per row, one pass: the row's sum stays in
 // registers between the statistic and the scaling (rows of up to 8 x 4 x 256 elements, else a second read).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
@@ -404,6 +494,7 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const T* x, const T* r
   const T* xr = x + row * hidden;
   const T* rr = residual + row * hidden;
   T* orow = out + row * hidden;
+  const T* sum = residual ? res_out + row * hidden : xr;
   T* srow = res_out + row * hidden;
   __shared__ float s_part[8];
   uint4 keep[U];
@@ -415,7 +506,7 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const T* x, const T* r
       const int v = v0 + u * blockDim.x;
       if (v >= nvec) continue;
       const uint4 a = *reinterpret_cast<const uint4*>(xr + size_t(v) * 8);
-      const uint4 b = *reinterpret_cast<const uint4*>(rr + size_t(v) * 8);
+      const uint4 b = residual ? *reinterpret_cast<const uint4*>(rr + size_t(v) * 8) : make_uint4(0, 0, 0, 0);
       const T2* pa = reinterpret_cast<const T2*>(&a);
       const T2* pb = reinterpret_cast<const T2*>(&b);
       uint4 o;
@@ -427,7 +518,7 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const T* x, const T* r
         const float2 r = Num<T>::up(po[e]);
         ss += r.x * r.x + r.y * r.y;
       }
-      *reinterpret_cast<uint4*>(srow + size_t(v) * 8) = o;
+      if (residual) *reinterpret_cast<uint4*>(srow + size_t(v) * 8) = o;
       if (in_regs) keep[u] = o;
     }
   }
@@ -443,7 +534,7 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const T* x, const T* r
     for (int u = 0; u < U; ++u) {
       const int v = v0 + u * blockDim.x;
       if (v >= nvec) continue;
-      const uint4 xv = in_regs ? keep[u] : *reinterpret_cast<const uint4*>(srow + size_t(v) * 8);
+      const uint4 xv = in_regs ? keep[u] : *reinterpret_cast<const uint4*>(sum + size_t(v) * 8);
       const uint4 g = *reinterpret_cast<const uint4*>(gamma + size_t(v) * 8);
       const T2* px = reinterpret_cast<const T2*>(&xv);
       const T2* pg = reinterpret_cast<const T2*>(&g);
@@ -459,14 +550,15 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const T* x, const T* r
   }
 }
 
-template <typename T>
-void launch_attention(int G, dim3 grid, cudaStream_t stream, const T* q, const T* k, const T* v, T* out, float* part,
-                      unsigned int* counters, int hq, int hkv, int max_ctx, int ctx, int q_row_stride, float scale_log2) {
+template <typename T, bool ROPE>
+void launch_attention(int G, dim3 grid, cudaStream_t stream, const T* q, T* k, T* v, T* out, float* part,
+                      unsigned int* counters, int hq, int hkv, int max_ctx, int ctx, int q_row_stride, float scale_log2,
+                      float log2_theta) {
   switch (G) {
-    case 1: launch_pdl(decode_attention_kernel<T, 1>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2); break;
-    case 2: launch_pdl(decode_attention_kernel<T, 2>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2); break;
-    case 4: launch_pdl(decode_attention_kernel<T, 4>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2); break;
-    case 8: launch_pdl(decode_attention_kernel<T, 8>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2); break;
+    case 1: launch_pdl(decode_attention_kernel<T, 1, ROPE>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2, log2_theta); break;
+    case 2: launch_pdl(decode_attention_kernel<T, 2, ROPE>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2, log2_theta); break;
+    case 4: launch_pdl(decode_attention_kernel<T, 4, ROPE>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2, log2_theta); break;
+    case 8: launch_pdl(decode_attention_kernel<T, 8, ROPE>, grid, dim3(kAttnThreads), stream, q, k, v, out, part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2, log2_theta); break;
     default: B200_REQUIRE(false, "decode attention supports 1, 2, 4 or 8 query heads per KV head, got " << G);
   }
 }
@@ -507,8 +599,11 @@ int decode_attention_splits(int batch, int hkv, int ctx, int sm_count) {
   return s;
 }
 
-void decode_attention(DType t, const void* q, int q_row_stride, const void* kcache, const void* vcache, void* out, void* workspace,
-                      int batch, int hq, int hkv, int head_dim, int max_ctx, int ctx, int splits, cudaStream_t stream) {
+namespace {
+// theta 0: q is rotated and the caches hold position ctx - 1 already
+template <typename T>
+void run_attention(const void* q, int q_row_stride, void* kcache, void* vcache, void* out, void* workspace, int batch, int hq, int hkv,
+                   int head_dim, int max_ctx, int ctx, int splits, float theta, cudaStream_t stream) {
   B200_REQUIRE(head_dim == kAttnD, "decode attention is written for head_dim 128, got " << head_dim);
   B200_REQUIRE(hq % hkv == 0 && ctx >= 1 && ctx <= max_ctx && splits >= 1, "decode attention: bad shapes");
   const int G = hq / hkv;
@@ -518,15 +613,28 @@ void decode_attention(DType t, const void* q, int q_row_stride, const void* kcac
       static_cast<char*>(workspace) + (size_t(batch) * hkv * splits * G * (4 + kAttnD) * sizeof(float) + 255) / 256 * 256);
   const dim3 grid(static_cast<unsigned>(splits), static_cast<unsigned>(hkv), static_cast<unsigned>(batch));
   const float scale_log2 = 1.4426950408889634f / sqrtf(float(head_dim));
-  if (t == DType::F16)
-    launch_attention<__half>(G, grid, stream, static_cast<const __half*>(q), static_cast<const __half*>(kcache),
-                             static_cast<const __half*>(vcache), static_cast<__half*>(out), part, counters, hq, hkv, max_ctx, ctx,
-                             q_row_stride, scale_log2);
+  if (theta == 0.f)
+    launch_attention<T, false>(G, grid, stream, static_cast<const T*>(q), static_cast<T*>(kcache), static_cast<T*>(vcache),
+                               static_cast<T*>(out), part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2, 0.f);
   else
-    launch_attention<__nv_bfloat16>(G, grid, stream, static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(kcache),
-                                    static_cast<const __nv_bfloat16*>(vcache), static_cast<__nv_bfloat16*>(out), part, counters, hq, hkv,
-                                    max_ctx, ctx, q_row_stride, scale_log2);
+    launch_attention<T, true>(G, grid, stream, static_cast<const T*>(q), static_cast<T*>(kcache), static_cast<T*>(vcache),
+                              static_cast<T*>(out), part, counters, hq, hkv, max_ctx, ctx, q_row_stride, scale_log2, log2f(theta));
   B200_CUDA_CHECK(cudaGetLastError());
+}
+}  // namespace
+
+void decode_attention(DType t, const void* q, int q_row_stride, const void* kcache, const void* vcache, void* out, void* workspace,
+                      int batch, int hq, int hkv, int head_dim, int max_ctx, int ctx, int splits, cudaStream_t stream) {
+  (t == DType::F16 ? run_attention<__half> : run_attention<__nv_bfloat16>)(
+      q, q_row_stride, const_cast<void*>(kcache), const_cast<void*>(vcache), out, workspace, batch, hq, hkv, head_dim, max_ctx, ctx,
+      splits, 0.f, stream);
+}
+
+void rope_decode_attention(DType t, const void* qkv, int row_stride, void* kcache, void* vcache, void* out, void* workspace, int batch,
+                           int hq, int hkv, int head_dim, int max_ctx, int pos, int splits, float theta, cudaStream_t stream) {
+  B200_REQUIRE(pos >= 0 && pos < max_ctx && theta > 0.f, "rope_decode_attention: bad position or theta");
+  (t == DType::F16 ? run_attention<__half> : run_attention<__nv_bfloat16>)(qkv, row_stride, kcache, vcache, out, workspace, batch, hq,
+                                                                          hkv, head_dim, max_ctx, pos + 1, splits, theta, stream);
 }
 
 void add_rmsnorm(DType t, const void* x, const void* residual, const void* gamma, void* out, void* res_out, int64_t rows, int hidden,
@@ -540,6 +648,16 @@ void add_rmsnorm(DType t, const void* x, const void* residual, const void* gamma
     launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(unsigned(rows)), dim3(256), stream, static_cast<const __nv_bfloat16*>(x),
                static_cast<const __nv_bfloat16*>(residual), static_cast<const __nv_bfloat16*>(gamma),
                static_cast<__nv_bfloat16*>(out), static_cast<__nv_bfloat16*>(res_out), hidden, eps);
+  B200_CUDA_CHECK(cudaGetLastError());
+}
+
+void row_argmax(DType t, const void* x, float* values, int64_t* indices, int64_t rows, int cols, cudaStream_t stream) {
+  B200_REQUIRE(rows > 0 && cols > 0, "row_argmax: empty rows");
+  if (t == DType::F16)
+    launch_pdl(row_argmax_kernel<__half>, dim3(unsigned(rows)), dim3(kArgmaxThreads), stream, static_cast<const __half*>(x), values, indices, cols);
+  else
+    launch_pdl(row_argmax_kernel<__nv_bfloat16>, dim3(unsigned(rows)), dim3(kArgmaxThreads), stream, static_cast<const __nv_bfloat16*>(x),
+               values, indices, cols);
   B200_CUDA_CHECK(cudaGetLastError());
 }
 

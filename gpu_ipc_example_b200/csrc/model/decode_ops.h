@@ -27,8 +27,17 @@ size_t decode_attention_workspace_bytes(int batch, int hq, int hkv, int splits);
 void decode_attention(DType t, const void* q, int q_row_stride, const void* kcache, const void* vcache, void* out, void* workspace,
                       int batch, int hq, int hkv, int head_dim, int max_ctx, int ctx, int splits, cudaStream_t stream);
 
+// The two above in one kernel: qkv [batch, (hq + 2 hkv) * head_dim] as the projection leaves it (it is not changed); the rotated
+// k and the v of position `pos` are written into the caches, and attention runs over positions [0, pos].
+void rope_decode_attention(DType t, const void* qkv, int row_stride, void* kcache, void* vcache, void* out, void* workspace, int batch,
+                           int hq, int hkv, int head_dim, int max_ctx, int pos, int splits, float theta, cudaStream_t stream);
+
+// values[r], indices[r] = greatest value of row r of x [rows, cols] and where it stands (the first of equal ones; NaN wins).
+void row_argmax(DType t, const void* x, float* values, int64_t* indices, int64_t rows, int cols, cudaStream_t stream);
+
 // res_out = x + residual ; out = RMSNorm(res_out) * gamma, row by row ([rows, hidden], 16-byte aligned).  The local
 // half of "all-reduce, then residual add and RMSNorm" when the all-reduce is too large for the one-shot fused kernel.
+// residual and res_out nullptr: out = RMSNorm(x) * gamma.
 void add_rmsnorm(DType t, const void* x, const void* residual, const void* gamma, void* out, void* res_out, int64_t rows, int hidden,
                  float eps, cudaStream_t stream);
 

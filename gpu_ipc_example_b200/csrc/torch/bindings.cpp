@@ -507,6 +507,49 @@ at::Tensor decode_attention_op(at::Tensor qkv, at::Tensor kcache, at::Tensor vca
   return out;
 }
 
+// rope_kv_append followed by decode_attention over positions [0, pos], in one kernel (qkv is left as it is).
+at::Tensor rope_decode_attention_op(at::Tensor qkv, at::Tensor kcache, at::Tensor vcache, at::Tensor workspace, int64_t hq, int64_t hkv,
+                                    int64_t pos, int64_t splits, double theta) {
+  TORCH_CHECK(qkv.is_cuda() && qkv.is_contiguous() && kcache.is_contiguous() && vcache.is_contiguous() && kcache.dim() == 4,
+              "b200ipc: rope_decode_attention takes contiguous CUDA tensors, caches [B, hkv, max_ctx, D]");
+  const int64_t B = qkv.size(0), D = kcache.size(3);
+  TORCH_CHECK(qkv.size(1) == (hq + 2 * hkv) * D && kcache.size(0) == B && kcache.size(1) == hkv && vcache.sizes() == kcache.sizes() &&
+                  kcache.scalar_type() == qkv.scalar_type() && vcache.scalar_type() == qkv.scalar_type(),
+              "b200ipc: rope_decode_attention shape mismatch");
+  TORCH_CHECK(int64_t(workspace.numel() * workspace.element_size()) >= attention_workspace_bytes(B, hq, hkv, splits),
+              "b200ipc: attention workspace too small");
+  for (const at::Tensor* t : {&kcache, &vcache})
+    TORCH_CHECK((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "b200ipc: caches must be 16-byte aligned");
+  at::Tensor out = at::empty({B, hq * D}, qkv.options());
+  c10::cuda::CUDAGuard guard(qkv.device());
+  rope_decode_attention(dtype_of(qkv), qkv.data_ptr(), int(qkv.size(1)), kcache.data_ptr(), vcache.data_ptr(), out.data_ptr(),
+                        workspace.data_ptr(), int(B), int(hq), int(hkv), int(D), int(kcache.size(2)), int(pos), int(splits), float(theta),
+                        at::cuda::getCurrentCUDAStream(qkv.get_device()));
+  return out;
+}
+
+// RMSNorm(x) * gamma for [rows, hidden]
+at::Tensor rmsnorm_op(at::Tensor x, at::Tensor gamma, double eps) {
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && gamma.is_contiguous() && x.dim() == 2 && gamma.numel() == x.size(1) && x.size(1) % 8 == 0 &&
+                  gamma.scalar_type() == x.scalar_type() && fits_kernels(x) && fits_kernels(gamma),
+              "b200ipc: rmsnorm takes contiguous, 16-byte aligned [rows, hidden] tensors, hidden a multiple of 8");
+  at::Tensor out = at::empty_like(x);
+  c10::cuda::CUDAGuard guard(x.device());
+  add_rmsnorm(dtype_of(x), x.data_ptr(), nullptr, gamma.data_ptr(), out.data_ptr(), nullptr, x.size(0), int(x.size(1)), float(eps),
+              at::cuda::getCurrentCUDAStream(x.get_device()));
+  return out;
+}
+
+// (values fp32, indices) of the greatest element of every row of a 16-bit [rows, cols] tensor
+std::tuple<at::Tensor, at::Tensor> row_argmax_op(at::Tensor x) {
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.dim() == 2 && x.numel() > 0, "b200ipc: row_argmax takes a contiguous [rows, cols] CUDA tensor");
+  at::Tensor v = at::empty({x.size(0)}, x.options().dtype(at::kFloat)), i = at::empty({x.size(0)}, x.options().dtype(at::kLong));
+  c10::cuda::CUDAGuard guard(x.device());
+  row_argmax(dtype_of(x), x.data_ptr(), v.data_ptr<float>(), i.data_ptr<int64_t>(), x.size(0), int(x.size(1)),
+             at::cuda::getCurrentCUDAStream(x.get_device()));
+  return {v, i};
+}
+
 // (RMSNorm(x + residual) * gamma, x + residual) for [rows, hidden] tensors
 std::vector<at::Tensor> add_rmsnorm_op(at::Tensor x, at::Tensor residual, at::Tensor gamma, double eps) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && residual.is_contiguous() && gamma.is_contiguous() && x.dim() == 2 &&
@@ -562,6 +605,10 @@ TORCH_LIBRARY(b200ipc, m) {
   m.def("rope_kv_append(Tensor(a!) qkv, Tensor(b!) kcache, Tensor(c!) vcache, int hq, int hkv, int pos, float theta) -> ()", &rope_kv_append_op);
   m.def("decode_attention(Tensor qkv, Tensor kcache, Tensor vcache, Tensor(a!) workspace, int hq, int hkv, int ctx, int splits) -> Tensor",
         &decode_attention_op);
+  m.def("rope_decode_attention(Tensor qkv, Tensor(a!) kcache, Tensor(b!) vcache, Tensor(c!) workspace, int hq, int hkv, int pos, "
+        "int splits, float theta) -> Tensor", &rope_decode_attention_op);
+  m.def("rmsnorm(Tensor x, Tensor gamma, float eps) -> Tensor", &rmsnorm_op);
+  m.def("row_argmax(Tensor x) -> (Tensor, Tensor)", &row_argmax_op);
   m.def("silu_mul(Tensor gate_up) -> Tensor", &silu_mul_op);
   m.def("add_rmsnorm(Tensor x, Tensor residual, Tensor gamma, float eps) -> Tensor[]", &add_rmsnorm_op);
 }

@@ -15,8 +15,9 @@ three ways (`fusion=`):
   "nccl"       the baseline: cuBLAS projection, `torch.distributed.all_reduce`, separate add and norm
 
 What lies between the GEMMs and the collectives runs in three hand-written kernels when the head
-dimension is 128 (`kernels=True`, the default there): rotary embedding fused with the KV-cache append,
-attention of the new token over the cache (grouped-query, split over the context), SiLU(gate) * up.
+dimension is 128 (`kernels=True`, the default there): rotary embedding fused with the KV-cache append and
+attention of the new token over the cache (grouped-query, split over the context), SiLU(gate) * up; the first norm
+and the arg-max over the logits are one kernel each.
 With `kernels=False` the same steps are plain PyTorch ops (the reference path of the tests).
 
 The reference has no model code; its smoke script all-reduces decode-sized fp16 activations the way a
@@ -198,9 +199,12 @@ class LlamaTP:
         cfg = self.cfg
         B, D = tokens.shape[0], cfg.head_dim
         pos = self.pos
-        posv = torch.full((B,), pos, device=self.dev, dtype=torch.int64)
         h = [self.embed[tokens] for _ in range(self.nlocal)]                       # residual stream, replicated
-        normed = [rms_norm(h[i], self.norm_attn[0], cfg.eps) for i in range(self.nlocal)]
+        if self.kernels and cfg.hidden % 8 == 0 and self.norm_attn[0].dtype == h[0].dtype:
+            normed = [torch.ops.b200ipc.rmsnorm(h[i], self.norm_attn[0], cfg.eps) for i in range(self.nlocal)]
+        else:
+            normed = [rms_norm(h[i], self.norm_attn[0], cfg.eps) for i in range(self.nlocal)]
+        posv = None if self.kernels else torch.full((B,), pos, device=self.dev, dtype=torch.int64)
         for l in range(cfg.layers):
             attn_out = []
             with self._stage("qkv_gemm"):
@@ -208,11 +212,9 @@ class LlamaTP:
             for i in range(self.nlocal):
                 qkv = qkv_all[i]
                 if self.kernels:
-                    with self._stage("rope_append"):
-                        torch.ops.b200ipc.rope_kv_append(qkv, self.kcache[i][l], self.vcache[i][l], self.hq, self.hkv, pos, cfg.rope_theta)
-                    with self._stage("attention"):
-                        attn_out.append(torch.ops.b200ipc.decode_attention(qkv, self.kcache[i][l], self.vcache[i][l], self.attn_ws[i],
-                                                                           self.hq, self.hkv, pos + 1, self.attn_splits))
+                    with self._stage("rope_attention"):
+                        attn_out.append(torch.ops.b200ipc.rope_decode_attention(qkv, self.kcache[i][l], self.vcache[i][l], self.attn_ws[i], self.hq,
+                                                                                self.hkv, pos, self.attn_splits, cfg.rope_theta))
                     continue
                 q, k, v = qkv.split([self.hq * D, self.hkv * D, self.hkv * D], dim=-1)
                 q = apply_rope(q.view(B, self.hq, D), posv, cfg.rope_theta)
@@ -243,10 +245,10 @@ class LlamaTP:
         # vocabulary-parallel head: local arg-max, then the global one over ranks
         best_val, best_idx = [], []
         for i in range(self.nlocal):
-            logits = (normed[i] @ self.lm_head[i].t()).float()
-            v, ix = logits.max(dim=-1)
+            logits = normed[i] @ self.lm_head[i].t()
+            v, ix = torch.ops.b200ipc.row_argmax(logits) if self.kernels else logits.float().max(dim=-1)
             best_val.append(v)
-            best_idx.append(ix + self.ranks[i] * (cfg.vocab // self.world))
+            best_idx.append(ix + self.ranks[i] * (cfg.vocab // self.world) if self.ranks[i] else ix)
         self.pos += 1
         if self.world == 1:
             return best_idx[0]

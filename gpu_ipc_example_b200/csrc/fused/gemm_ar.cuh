@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_ar_kernel(const __grid_c
   const HeapLayout& lay = args.k.lay;
   const int W = me.world;
   const int rank = me.rank;
-  const int warp = int(threadIdx.x >> 5);
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);  // the same register in every lane
   const int lane = int(threadIdx.x & 31);
   const int G = int(gridDim.x);
   const int M = args.M, N = args.N, K = args.K;
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_ar_kernel(const __grid_c
 
   // ---- GEMM + exchange: four roles run side by side ---------------------------------------------
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const CUtensorMap* ta = &args.tma_a[blockIdx.y];
       const CUtensorMap* tb = &args.tma_b[blockIdx.y];
       const char* wp = static_cast<const char*>(args.w_packed[blockIdx.y]);
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_ar_kernel(const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc<T>(kGemmBM, BN);
       uint32_t it = 0, tile_i = 0;
       for (int t = int(blockIdx.x); t < total_tiles && !*abort_flag; t += G, ++tile_i) {

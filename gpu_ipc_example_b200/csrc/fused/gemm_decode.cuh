@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
   const HeapLayout& lay = args.k.lay;
   const int W = args.local_only ? 1 : me.world;
   const int rank = me.rank;
-  const int warp = int(threadIdx.x >> 5);
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);  // the same register in every lane
   const int lane = int(threadIdx.x & 31);
   const int G = int(gridDim.x);
   const int M = args.M, N = args.N, K = args.K;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
   // The weights do not depend on the kernel before this one: the producer fills the ring with the W halves of
   // its first stages before it waits for that kernel; the X halves follow after the wait.
   uint32_t npre = 0;
-  if (warp == 0 && lane == 0 && int(blockIdx.x) < units) {
+  if (warp == 0 && int(blockIdx.x) < units && elect_one()) {
     const int u = int(blockIdx.x);
     const int tile = u / splits, ks = u % splits;
     const int kb0 = ks * kb_per;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
   if (me.seq_dev) epoch += ld_volatile_u32(me.seq_dev + kGemmEpochSlot);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int u = int(blockIdx.x); u < units && !*abort_flag; u += G) {
         const int tile = u / splits, ks = u % splits;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc<T>(kDecTileRows, kDecXRows);
       uint32_t it = 0, unit_i = 0;
       for (int u = int(blockIdx.x); u < units && !*abort_flag; u += G, ++unit_i) {

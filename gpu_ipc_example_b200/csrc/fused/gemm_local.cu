@@ -20,9 +20,10 @@ struct LocalPlan {
 // k blocks per stage: two where a block holds too little work for what its barriers and its commit cost
 int local_ksub(int bn) { return bn <= 128 ? 2 : 1; }
 
-int local_stages(int bn) {
+int local_stages(int bn, int splits) {
   const int stage = (128 + bn / 2) * kGemmBK * 2 * local_ksub(bn);
-  return std::min(kLocMaxStages, (kLocSmemBudget - 1024) / stage);
+  const int slab = (splits - 1) * (bn / splits) * 128 * 4;  // what the other pairs of a cluster hand over
+  return std::min(kLocMaxStages, (kLocSmemBudget - 1024 - slab) / stage);
 }
 
 const void* local_kernel(DType t, int bn) {
@@ -61,12 +62,12 @@ int resident_clusters(const void* fn, int device, int splits) {
 // Microseconds that a plan takes apart from what all plans share (launch, first loads).  Fitted to one B200: a k block of a
 // pair 0.08 + 0.0012 BN (K = 8192, M = 2048, N = 7168: BN = 160 166 us, 224 170, 256 197, 128 197); the epilogue of a
 // tile 0.5 + 0.0133 BN, hidden behind the next tile's MMAs where there is one; handing partial sums between the pairs of a
-// cluster 1.6 + 0.006 BN (K = 1024, M = 1, N = 8192: one split 14.4 us, two 16.4; K = 3584, M = 16: 16.0 and 14.5).
+// cluster 1.4 + 0.006 BN (K = 1024, M = 16, N = 8192: one split 15.4 us, two 17.4; K = 3584: 18.6 and 14.5 back to back).
 double plan_cost(int64_t tiles, int64_t room, int64_t kb_total, int bn, int splits) {
   const double waves = double(ceil_div64(tiles, room));
   const double main = double(ceil_div64(kb_total, splits)) * (0.08 + 0.0012 * bn);
   const double epi = 0.5 + 0.0133 * bn / splits;
-  return waves * std::max(main, epi) + epi + (splits > 1 ? 1.6 + 0.006 * bn : 0);
+  return waves * std::max(main, epi) + epi + (splits > 1 ? 1.4 + 0.006 * bn : 0);
 }
 
 // The tile height and the K split of a problem.  bn_only: the tile's height is given (merged shards).
@@ -113,7 +114,7 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   args.m_tiles = p.m_tiles;
   args.n_tiles = int(ceil_div64(args.N, kLocWRows));
   args.splits = p.splits;
-  args.stages = local_stages(p.bn);
+  args.stages = local_stages(p.bn, p.splits);
   args.early_w = p.bn == 32 ? 1 : 0;
   const int64_t mt_all = int64_t(args.shards) * p.m_tiles;
   // as many m-tiles side by side as keep their X rows in a quarter of L2 while the W tiles pass by

@@ -17,7 +17,7 @@
 //
 // Few tiles (decode, narrow layers): K is split over the pairs of a cluster of 2, 4 or 8 CTAs; after the last MMA every
 // pair hands its fp32 partial sums for a share of the rows to the pair that owns them through distributed shared
-// memory, and the owners add them in a fixed order (the result does not depend on timing) and run the epilogue.
+// memory (st.async, counted on the receiver's barrier), and the owners add them in a fixed order (the result does not depend on timing) and run the epilogue.
 #pragma once
 
 #include "gemm_ar.cuh"
@@ -69,6 +69,11 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
   return a;
+}
+// Store into another CTA's shared memory whose bytes are counted on a barrier of that CTA.
+__device__ __forceinline__ void st_async(uint32_t cluster_addr, uint32_t v, uint32_t bar_cluster) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr), "r"(v), "r"(bar_cluster)
+               : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -136,7 +141,7 @@ __device__ __forceinline__ LocTile loc_tile(const LocalGemmArgs& a, int t) {
 template <typename T, int KSUB>
 __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid_constant__ LocalGemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full[kLocMaxStages], empty[kLocMaxStages], acc_full[2], acc_empty[2];
+  __shared__ uint64_t full[kLocMaxStages], empty[kLocMaxStages], acc_full[2], acc_empty[2], slab_full;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -168,6 +173,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_empty[i], 16);  // eight epilogue warps of both CTAs
     }
+    mbar_init(&slab_full, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -411,36 +417,36 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
     const int c_own = split * own, valid = tile_rows(t);
     const T* res0 = static_cast<const T*>(args.residual[0]);
     T rv[kLocChunk];
+    // What the pairs hand over lies behind the ring: nobody has to wait until the others' MMAs have read theirs.  A piece is
+    // 16 rows (8 at the end of a share that is not a multiple of 16); pieces without rows of X are not sent.
+    float* slab = reinterpret_cast<float*>(ring + size_t(stages) * stage_bytes);  // [splits - 1][own][128] fp32, in split order
+    auto sent_rows = [&](int o) { return o * own >= valid ? 0 : min(own, (valid - o * own + 15) / 16 * 16); };
+    if (threadIdx.x == 64) mbar_expect_tx(&slab_full, uint32_t(splits - 1) * uint32_t(sent_rows(split)) * 512u);
     if (warp >= 2) {
       const int c0 = group * kLocChunk;
       if (res0) load_residual(res0, out_off(t, c_own + c0), rows_left(t, c_own + c0, min(own - c0, kLocChunk)), rv);
-      mbar_wait(&acc_full[0], 0, abort_flag, timeout_ns);
     }
-    const bool bad = __syncthreads_or(*abort_flag) != 0;
-    tc_fence_after_sync();
-    cluster_sync_all();  // every pair's MMAs are done: the rings may be overwritten
-    float* slab = reinterpret_cast<float*>(ring);  // [splits - 1][own][128] fp32, from the other pairs in split order
-    if (warp >= 2 && !bad) {
-      // the groups take turns with the 16-row pieces of what goes to the other pairs
+    const bool bad = warp < 2 || __any_sync(0xffffffffu, !mbar_wait(&acc_full[0], 0, abort_flag, timeout_ns));
+    if (!bad) {
+      tc_fence_after_sync();
       for (int d = 1; d < splits; ++d) {
         const int o = (split + d) % splits;
         const int slot = split < o ? split : split - 1;
         const uint32_t dst = map_to_cta(smem_u32(slab + size_t(slot) * own * 128 + my_n), uint32_t(2 * o + side));
-        for (int c = 16 * group; c < own && o * own + c < valid; c += 32) {
+        const uint32_t bar = map_to_cta(smem_u32(&slab_full), uint32_t(2 * o + side));
+        for (int c = 16 * group; c < sent_rows(o); c += 32) {
           uint32_t acc[16];
           tmem_ld_8cols(tmem_base + tmem_lane + uint32_t(o * own + c), acc);
           if (c + 8 < own) tmem_ld_8cols(tmem_base + tmem_lane + uint32_t(o * own + c + 8), acc + 8);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (j < 8 || c + 8 < own)
-              asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + uint32_t(c + j) * 512u), "r"(acc[j]) : "memory");
+            if (j < 8 || c + 8 < own) st_async(dst + uint32_t(c + j) * 512u, acc[j], bar);
         }
       }
     }
-    __syncwarp();
-    cluster_sync_all();
-    if (warp >= 2 && !bad) {
+    if (!bad && !__any_sync(0xffffffffu, !mbar_wait(&slab_full, 0, abort_flag, timeout_ns))) {
+      asm volatile("fence.acq_rel.cluster;" ::: "memory");
       for (int c = group * kLocChunk; c < own && c_own + c < valid; c += 2 * kLocChunk) {
         const int cw = min(own - c, kLocChunk);
         if (res0 && c >= 2 * kLocChunk) load_residual(res0, out_off(t, c_own + c), rows_left(t, c_own + c, cw), rv);

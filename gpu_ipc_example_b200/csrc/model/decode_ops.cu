@@ -172,43 +172,6 @@ __global__ void __launch_bounds__(kAttnThreads, 2) decode_attention_kernel(const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = lane >> 2, c = lane & 3;
 
-  __shared__ __align__(16) T s_q[ROPE ? G * kAttnD : 8];
-  if constexpr (ROPE) {
-    constexpr int half = kAttnD / 2;
-    const T* row = q + size_t(b) * q_row_stride;
-    const int pos = ctx - 1, i = threadIdx.x & (half - 1), sub = threadIdx.x / half;  // pair i, two heads at a time
-    // angle = pos * theta^(-i / half), as in rope_kv_append_kernel
-    const float inv = exp2f(-log2_theta * float(i) / float(half));
-    float sn, cs;
-    sincosf(float(pos) * inv, &sn, &cs);
-    auto rotate = [&](const T* src, T* dst) {
-      const float2 y = rope_pair(float(src[i]), float(src[i + half]), sn, cs);
-      dst[i] = T(y.x);
-      dst[i + half] = T(y.y);
-    };
-#pragma unroll
-    for (int g = 0; g < G; g += kAttnThreads / half)
-      if (g + sub < G) rotate(row + (size_t(h) * G + g + sub) * kAttnD, s_q + (g + sub) * kAttnD);
-    const int own_per = ((ctx + nsplit - 1) / nsplit + kAttnTile - 1) / kAttnTile * kAttnTile;
-    if (pos / own_per == split) {
-      const size_t at = ((size_t(b) * hkv + h) * size_t(max_ctx) + size_t(pos)) * kAttnD;
-      if (sub == 0) {
-        rotate(row + (size_t(hq) + h) * kAttnD, kcache + at);
-      } else {
-        const T* v = row + (size_t(hq) + hkv + h) * kAttnD;
-        vcache[at + i] = v[i];
-        vcache[at + i + half] = v[i + half];
-      }
-    }
-    __syncthreads();  // also makes the new k and v visible to the loads of this CTA
-  }
-
-  // Q operand: head r of this KV head's group (rows G..15 of the 16-row operand are zero)
-  uint32_t qa[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) qa[i] = 0u;
-  if (r < G) load_row_quarter<T>(qa, ROPE ? s_q + r * kAttnD : q + size_t(b) * q_row_stride + (size_t(h) * G + r) * kAttnD, c);
-
   // running state of head r (every lane of the quad holds the same m; l is a per-lane partial sum)
   float m = -INFINITY, l = 0.f;
   // O^T: acc[t][0..3] = (dim 16r+2t, head 2c), (dim 16r+2t, head 2c+1), (dim 16r+2t+1, head 2c), (dim 16r+2t+1, head 2c+1)
@@ -248,6 +211,48 @@ __global__ void __launch_bounds__(kAttnThreads, 2) decode_attention_kernel(const
       }
     }
   };
+  // The first step's loads go out before q is looked at; only the step that holds the position being written has to wait.
+  uint32_t kA[2][16], vA[4][8];
+  int base = p0 + warp * kAttnTile;
+  const bool late = ROPE && base <= ctx - 1 && ctx - 1 < base + kAttnTile;
+  if (base < p1 && !late) load_tile(base, kA, vA);
+
+  __shared__ __align__(16) T s_q[ROPE ? G * kAttnD : 8];
+  if constexpr (ROPE) {
+    constexpr int half = kAttnD / 2;
+    const T* row = q + size_t(b) * q_row_stride;
+    const int pos = ctx - 1, i = threadIdx.x & (half - 1), sub = threadIdx.x / half;  // pair i, two heads at a time
+    // angle = pos * theta^(-i / half), as in rope_kv_append_kernel
+    const float inv = exp2f(-log2_theta * float(i) / float(half));
+    float sn, cs;
+    sincosf(float(pos) * inv, &sn, &cs);
+    auto rotate = [&](const T* src, T* dst) {
+      const float2 y = rope_pair(float(src[i]), float(src[i + half]), sn, cs);
+      dst[i] = T(y.x);
+      dst[i + half] = T(y.y);
+    };
+#pragma unroll
+    for (int g = 0; g < G; g += kAttnThreads / half)
+      if (g + sub < G) rotate(row + (size_t(h) * G + g + sub) * kAttnD, s_q + (g + sub) * kAttnD);
+    if (pos >= p0 && pos < p1) {
+      const size_t at = ((size_t(b) * hkv + h) * size_t(max_ctx) + size_t(pos)) * kAttnD;
+      if (sub == 0) {
+        rotate(row + (size_t(hq) + h) * kAttnD, kcache + at);
+      } else {
+        const T* v = row + (size_t(hq) + hkv + h) * kAttnD;
+        vcache[at + i] = v[i];
+        vcache[at + i + half] = v[i + half];
+      }
+    }
+    __syncthreads();  // also makes the new k and v visible to the loads of this CTA
+  }
+
+  // Q operand: head r of this KV head's group (rows G..15 of the 16-row operand are zero)
+  uint32_t qa[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) qa[i] = 0u;
+  if (r < G) load_row_quarter<T>(qa, ROPE ? s_q + r * kAttnD : q + size_t(b) * q_row_stride + (size_t(h) * G + r) * kAttnD, c);
+
   auto compute_tile = [&](int base, const uint32_t (&kw)[2][16], const uint32_t (&vw)[4][8]) {
     // ---- scores: s[j][0..1] = head r, positions base + 8j + 2c, + 1 --------------------------------
     float s[2][4];
@@ -290,9 +295,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) decode_attention_kernel(const
   // two register sets: the loads of the next step are in flight while this one is computed
   {
     const int stride = kAttnWarps * kAttnTile;
-    uint32_t kA[2][16], vA[4][8], kB[2][16], vB[4][8];
-    int base = p0 + warp * kAttnTile;
-    if (base < p1) load_tile(base, kA, vA);
+    uint32_t kB[2][16], vB[4][8];
+    if (base < p1 && late) load_tile(base, kA, vA);
     while (base < p1) {
       const int nb = base + stride;
       if (nb < p1) load_tile(nb, kB, vB);

@@ -58,8 +58,9 @@ inline const TuneRow* tune_table(int world, bool symmetric, int* rows) {
   return symmetric ? w2_sym : w2_user;
 }
 
-// Emulated worlds (all ranks on one GPU): the input size in bytes up to which the flag-in-data kernels are used; above it
-// the barrier-based kernel that reads and writes the callers' own buffers (BulkPlace::Direct).  There is no link whose hops
+// Emulated worlds (all ranks on one GPU), calls whose ranks meet at a barrier (flags given, or a communicator that was moved to
+// the 8-byte-granule formats; others take the direct kernel at every size): the input size in bytes up to which the
+// flag-in-data kernels are used; above it the barrier-based kernel that reads and writes the callers' own buffers (BulkPlace::Direct).  There is no link whose hops
 // a flag-in-data message saves, and its rings are extra passes over the same L2 and HBM; what it saves is the barrier.
 // Device time on one B200, fp16, flag-in-data against direct:
 //   all-reduce      2 ranks  512 KiB 3.3 / 3.4 us,  1 MiB 4.7 / 3.4,  16 MiB 25.8 / 8.4

@@ -2,7 +2,8 @@
 // world): nothing is exchanged.  A cluster of `parts` CTAs owns a row for ALL ranks: it reads the row of every rank's x
 // once, adds in rank order in fp32, adds each rank's residual, rounds, and normalises; the rows stay in registers between
 // the statistic and the scaling, and the CTAs of a row hand each other their sums of squares through distributed shared
-// memory.  Bound by launch and memory latency at decode sizes and by memory above.
+// memory.  Bound by launch and memory latency at decode sizes (8 ranks, 16 rows of 8192: 9.2 us cold, the flag-in-data
+// kernel 20.4) and by memory above (8 ranks, 512 rows: 53 us for 209 MB).
 #pragma once
 
 #include "../coll/bulk_kernels.cuh"

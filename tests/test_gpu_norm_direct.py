@@ -10,7 +10,7 @@ HALF_ULP = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
 
 
 @pytest.mark.parametrize("world", [1, 2, 4, 8])
-@pytest.mark.parametrize("rows,hidden", [(1, 8), (1, 264), (3, 1032), (16, 8192), (100, 4104), (300, 5128), (512, 8192), (2, 32768), (200, 12296)])
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (1, 264), (3, 1032), (16, 8192), (100, 4104), (300, 5128), (512, 8192), (2, 32768), (200, 12296), (1, 40960)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_direct(world, rows, hidden, dtype):
     g = torch.Generator(device="cuda").manual_seed(rows + hidden)

@@ -441,7 +441,7 @@ def run(args, json_out, state):
                 "global_batch": emu_world,
                 "seq_len": n,
                 "parallelism": (f"{world} GPUs, one rank per GPU over NVLink" if multi
-                                else f"{emu_world} ranks emulated on 1 GPU (one cooperative launch; peer traffic stays in L2/HBM, no NVLink)"),
+                                else f"{emu_world} ranks emulated on 1 GPU (one launch; peer traffic stays in L2/HBM, no NVLink)"),
                 "algo": f"{args.algo} -> {headline_algo}",
                 "buffers": f"{nbuf} rotating buffers = {nbuf * nbytes >> 20} MiB > 126 MiB L2, in place, symmetric heap (no staging copy)",
                 "busbw": "bytes/time*2(n-1)/n, device time by CUDA events, max over ranks",

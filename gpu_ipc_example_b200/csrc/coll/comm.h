@@ -92,6 +92,7 @@ class Comm {
   const SymmHeap& heap(int local = 0) const { return *heaps_[size_t(local)]; }
   UnixMesh* mesh() const { return mesh_; }
   int sm_count() const { return sm_count_; }
+  int max_ctas() const { return max_ctas_; }  // 0: no limit
 
   // ins / outs hold nlocal() pointers (one per local rank).  nelems counts 16-bit
   // elements of one rank's buffer.  in == out means in place.

@@ -105,7 +105,7 @@ CollInfo direct_norm(Comm& comm, DType t, const FusedNormPtrs* ptrs, int64_t row
 }  // namespace
 
 bool direct_norm_takes(const Comm& comm, int64_t hidden) {
-  return comm.nlocal() == comm.world() && hidden > 0 && hidden % 8 == 0 && direct_norm_lookup<__half>(comm.world(), 1) != nullptr &&
+  return comm.nlocal() == comm.world() && comm.max_ctas() == 0 && hidden > 0 && hidden % 8 == 0 && direct_norm_lookup<__half>(comm.world(), 1) != nullptr &&
          hidden / 8 <= kDirectNormMaxParts * direct_norm_cta_vecs(comm.world());
 }
 
@@ -117,7 +117,7 @@ CollInfo fused_allreduce_residual_rmsnorm(Comm& comm, DType t, const FusedNormPt
     for (const void* p : {ptrs[i].x, ptrs[i].residual, ptrs[i].gamma, static_cast<const void*>(ptrs[i].out),
                           static_cast<const void*>(ptrs[i].residual_out)})
       B200_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, "fused all-reduce + RMSNorm needs 16-byte aligned tensors");
-  // Every rank is driven by this process: no exchange (an explicit CTA count asks for the kernel with it).  8 ranks, 16 rows
+  // Every rank is driven by this process: no exchange (an explicit CTA count, or a limit on them, asks for the kernel with it).  8 ranks, 16 rows
   // of 8192: 9.2 us against 20.4 (device time, cold cache).
   if (ctas_req == 0 && direct_norm_takes(comm, hidden)) return direct_norm(comm, t, ptrs, rows, hidden, eps, stream);
   KernelFn fn = t == DType::F16 ? pick_world<__half, __half, kEpiNorm>(N) : pick_world<__nv_bfloat16, __nv_bfloat16, kEpiNorm>(N);

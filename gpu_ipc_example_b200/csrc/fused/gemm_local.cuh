@@ -61,7 +61,8 @@ struct LocalGemmArgs {
   int band;      // m-tiles visited before the next W tile
   int splits;    // K splits = pairs per cluster
   int stages;
-  int early_w;   // the first stages' W loads go out before the wait for the previous kernel
+  int early_w;   // the first stages' W loads go out before the wait for the previous kernel: as in the decode-sized kernel,
+                 // a weight is not what the kernels right before this one in the stream write
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {

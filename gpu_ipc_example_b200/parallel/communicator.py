@@ -68,6 +68,7 @@ class Communicator:
         self.world = self._C.world(handle)
         self.nlocal = self._C.nlocal(handle)
         self.rank = self._C.rank(handle, 0)
+        self._direct = self.nlocal == self.world  # this process drives every rank: nothing has to be exchanged
         self._info = None  # the launch report of the last call, as the native code gives it
         ops = torch.ops.b200ipc
         self._all_reduce_lists, self._all_gather_lists = ops.all_reduce_lists.default, ops.all_gather_lists.default
@@ -94,6 +95,7 @@ class Communicator:
         h = C.comm_create(rank, world, device, job_id, instance, staging_bytes, nvls, timeout_ms, backing, device_seq,
                           first_seq, max_ctas, bootstrap_timeout_ms)
         comm = cls(h, False)
+        comm._direct &= max_ctas == 0  # the kernels without an exchange take the whole GPU
         if os.environ.get("B200IPC_SELFTEST", "0") not in ("", "0") and world > 1:
             comm.self_test()  # falls back to the 8-byte-granule formats if a 64-byte segment is ever seen torn
         return comm
@@ -116,7 +118,9 @@ class Communicator:
         """All `world` ranks emulated on one GPU (one cooperative launch per collective)."""
         C = load()
         h = C.comm_create_virtual(world, device, staging_bytes, timeout_ms, device_seq, first_seq, max_ctas)
-        return cls(h, True)
+        comm = cls(h, True)
+        comm._direct &= max_ctas == 0
+        return comm
 
     def close(self):
         if self._h is not None:
@@ -203,7 +207,7 @@ class Communicator:
         xs = self._lists(x)
         rs = self._lists(residual)
         gs = self._lists(gamma)
-        if ctas == 0 and self.nlocal == self.world:
+        if ctas == 0 and self._direct:
             both, info = self._ar_rmsnorm_lists(xs, rs, gs, eps, self._h)
             if both:
                 self._info = info
@@ -277,7 +281,7 @@ class Communicator:
         xs = [t.contiguous() for t in self._lists(x)]
         ws = [t.contiguous() for t in self._lists(weight)]
         M, N = xs[0].shape[0], ws[0].shape[0] * (64 if ws[0].dim() == 4 else 1)  # 4-D: packed by pack_weight
-        local = fused is None and ctas == 0 and self.nlocal == self.world and ws[0].dim() == 2
+        local = fused is None and ctas == 0 and self._direct and ws[0].dim() == 2
         if fused is None:
             fused = not (32 < M <= 256 and self.world >= 4 and not self._virtual and ws[0].dim() == 2
                          and residual is not None and gamma is not None)
@@ -362,7 +366,7 @@ class Communicator:
             # weight that wants a gradient
             fits = fused or (N % 64 == 0 and K % 8 == 0 and not any(t.data_ptr() % 16 for t in xs + ws)
                              and not (torch.is_grad_enabled() and any(t.requires_grad for t in ws)))
-            if fits and ctas == 0 and self.nlocal == self.world:
+            if fits and ctas == 0 and self._direct:
                 outs = [torch.empty(M, N, dtype=t.dtype, device=t.device) for t in xs]
                 v = self._local_ag_gemm(xs, ws, outs, self._h)
                 self._info = v

@@ -103,3 +103,22 @@ def test_the_kernels_with_the_exchange(world, M):
                 torch.testing.assert_close(s.double(), y, atol=2e-3, rtol=2e-3)
                 want = s.double() * torch.rsqrt(s.double().pow(2).mean(-1, keepdim=True) + 1e-5) * gam.double()
                 torch.testing.assert_close(o.double(), want, atol=2e-3, rtol=2e-3)
+
+
+def test_a_limit_on_ctas_is_kept():
+    """A communicator that may use a few SMs only (the others belong to work on another stream) keeps the kernels that can be
+    told so."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    with Communicator.virtual(2, 0, staging_bytes=64 << 20, max_ctas=8) as comm:
+        xs = [_rand(g, torch.float16, 64, 512) for _ in range(2)]
+        ws = [_rand(g, torch.float16, 1024, 512, scale=0.02) for _ in range(2)]
+        res, gam = [_rand(g, torch.float16, 64, 1024)] * 2, [_rand(g, torch.float16, 1024)] * 2
+        comm.linear_allreduce(xs, ws, res, gam)
+        assert comm.last_info.ctas <= 8
+        comm.allreduce_residual_rmsnorm(res, res, gam)
+        assert comm.last_info.ctas <= 8 and comm.last_info.sched == "oneshot"
+        outs = comm.allgather_linear(xs, ws)
+        assert comm.last_info.ctas <= 8  # the all-gather's
+        torch.cuda.synchronize()
+        comm.check()
+        torch.testing.assert_close(outs[0].double(), torch.cat(xs).double() @ ws[0].double().t(), atol=2e-3, rtol=2e-3)

@@ -2,13 +2,14 @@
 // scheduled while its predecessor in the stream is still running, once every CTA of the predecessor
 // has executed pdl_launch_dependents() (or exited).  Its CTAs become resident on SMs the predecessor
 // has left, run whatever does not depend on the predecessor (barrier set-up, tensor-memory
-// allocation, WEIGHT prefetch), and block in pdl_wait() until the predecessor has completed and its
+// allocation, a prefetch of weights to L2), and block in pdl_wait() until the predecessor has completed and its
 // memory is visible.  A decode step is a chain of ~7 short kernels per layer; this takes launch
 // latency and prologues off the critical path.
 //
 // Rules followed by every kernel that is launched this way:
 //   * pdl_wait() comes before the first access to anything an earlier kernel may have written or
-//     may still read (activations, flags, counters, scratch);
+//     may still read (activations, flags, counters, scratch; weights too: a caller may have made them with the
+//     kernel right in front).  A prefetch to L2 is not such an access: nothing is read through it;
 //   * kernels without pdl_wait() are never launched with the attribute;
 //   * cooperative launches (several emulated ranks on one GPU) do not take the attribute: the two
 //     instructions are then no-ops.

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
   int kb_per = (kb_total + splits - 1) / splits;
   kb_per = (kb_per + kDecKSub - 1) / kDecKSub * kDecKSub;
   const uint64_t timeout_ns = me.timeout_ns;
-  pdl_launch_dependents();  // the next kernel may set itself up (and prefetch its weights) while this one runs
+  pdl_launch_dependents();  // the next kernel may set itself up (and prefetch its weights to L2) while this one runs
   constexpr uint32_t kTmemCols = 2 * kDecXRows;
   constexpr uint32_t kSubBytes = uint32_t(kDecTileRows + kDecXRows) * kGemmBK * 2;
 
@@ -98,28 +98,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
   const CUtensorMap* tw = &args.tma_b[blockIdx.y];
   const char* wp = static_cast<const char*>(args.w_packed[blockIdx.y]);
   constexpr uint32_t kBlk = 64 * kGemmBK * 2;
+  auto packed_block = [&](int tile, int rb, int kb) {
+    return wp + (size_t(tile * (kDecTileRows / 64) + rb) * size_t(args.packed_kblocks) + size_t(kb)) * kBlk;
+  };
   auto load_w = [&](int st, int sub, int tile, int kb) {
     if (wp) {
-      for (int rb = 0; rb < kDecTileRows / 64; ++rb)
-        bulk_load(s.a[st][sub] + rb * kBlk,
-                  wp + (size_t(tile * (kDecTileRows / 64) + rb) * size_t(args.packed_kblocks) + size_t(kb)) * kBlk, kBlk, &s.full[st]);
+      for (int rb = 0; rb < kDecTileRows / 64; ++rb) bulk_load(s.a[st][sub] + rb * kBlk, packed_block(tile, rb, kb), kBlk, &s.full[st]);
     } else {
       tma_load_2d(s.a[st][sub], tw, &s.full[st], kb * kGemmBK, tile * kDecTileRows);
     }
   };
-  // The weights do not depend on the kernel before this one: the producer fills the ring with the W halves of
-  // its first stages before it waits for that kernel; the X halves follow after the wait.
-  uint32_t npre = 0;
+  // Whether the weights come from the kernels before this one is not known here, so no load goes out before the wait.  The
+  // W halves of the ring's first stages are brought to L2 meanwhile.
   if (warp == 0 && int(blockIdx.x) < units && elect_one()) {
     const int u = int(blockIdx.x);
     const int tile = u / splits, ks = u % splits;
     const int kb0 = ks * kb_per;
     int kb1 = kb0 + kb_per;
     if (kb1 > kb_total) kb1 = kb_total;
-    for (int kb = kb0; kb < kb1 && npre < uint32_t(kDecStages); kb += kDecKSub, ++npre) {
-      const int nsub = (kb1 - kb) < kDecKSub ? (kb1 - kb) : kDecKSub;
-      mbar_expect_tx(&s.full[npre], kSubBytes * uint32_t(nsub));
-      for (int sub = 0; sub < nsub; ++sub) load_w(int(npre), sub, tile, kb + sub);
+    if (kb1 > kb0 + kDecStages * kDecKSub) kb1 = kb0 + kDecStages * kDecKSub;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (wp) {
+        for (int rb = 0; rb < kDecTileRows / 64; ++rb) bulk_prefetch(packed_block(tile, rb, kb), kBlk);
+      } else {
+        tma_prefetch_2d(tw, kb * kGemmBK, tile * kDecTileRows);
+      }
     }
   }
   pdl_wait();  // everything below may read what earlier kernels wrote (activations, flags, counters, the fp32 product)
@@ -138,14 +141,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
           const int st = int(it % kDecStages);
           const uint32_t ph = (it / kDecStages) & 1u;
           const int nsub = (kb1 - kb) < kDecKSub ? (kb1 - kb) : kDecKSub;
-          const bool w_done = it < npre;  // this stage's W halves are already on their way
-          if (!w_done) {
-            if (!mbar_wait(&s.empty[st], ph ^ 1u, abort_flag, timeout_ns)) break;
-            mbar_expect_tx(&s.full[st], kSubBytes * uint32_t(nsub));
-          }
+          if (!mbar_wait(&s.empty[st], ph ^ 1u, abort_flag, timeout_ns)) break;
+          mbar_expect_tx(&s.full[st], kSubBytes * uint32_t(nsub));
           for (int sub = 0; sub < nsub; ++sub) {
             tma_load_2d(s.b[st][sub], tx, &s.full[st], (kb + sub) * kGemmBK, 0);
-            if (!w_done) load_w(st, sub, tile, kb + sub);
+            load_w(st, sub, tile, kb + sub);
           }
         }
       }

@@ -115,7 +115,7 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   args.n_tiles = int(ceil_div64(args.N, kLocWRows));
   args.splits = p.splits;
   args.stages = local_stages(p.bn, p.splits);
-  args.early_w = p.bn == 32 ? 1 : 0;
+  args.warm_w = p.bn == 32 ? 1 : 0;
   const int64_t mt_all = int64_t(args.shards) * p.m_tiles;
   // as many m-tiles side by side as keep their X rows in a quarter of L2 while the W tiles pass by
   const int64_t x_bytes = int64_t(p.bn) * args.K * 2 * args.segs;

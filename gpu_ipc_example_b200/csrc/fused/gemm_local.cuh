@@ -61,8 +61,7 @@ struct LocalGemmArgs {
   int band;      // m-tiles visited before the next W tile
   int splits;    // K splits = pairs per cluster
   int stages;
-  int early_w;   // the first stages' W loads go out before the wait for the previous kernel: as in the decode-sized kernel,
-                 // a weight is not what the kernels right before this one in the stream write
+  int warm_w;    // the first stages' W boxes are brought to L2 before the wait for the previous kernel
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -229,15 +228,12 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
         tma_load_2d_pair(dst + uint32_t(i * args.merged_rows) * 128u, k.x + side * per_side + i, full_pair + st * 8, k.col, 0);
     }
   };
-  uint32_t npre = 0;
-  if (args.early_w && warp == 0 && cluster < total && elect_one()) {
+  // No load before the wait: W may be what the kernel before this one writes (the entry points themselves copy a strided one).
+  if (args.warm_w && warp == 0 && cluster < total && elect_one()) {
     const LocTile t = loc_tile(args, cluster);
     KPos k = first_k(t);
-    for (int kb = kb0; kb < kb1 && npre < uint32_t(stages); kb += KSUB, ++npre) {
-      const int nsub = KSUB == 1 ? 1 : min(KSUB, kb1 - kb);
-      if (side == 0) mbar_expect_tx(&full[npre], 2 * blk_bytes * uint32_t(nsub));
-      for (int sub = 0; sub < nsub; ++sub, next_k(k)) load_w(npre, sub, k, t);
-    }
+    if (t.n0 + side * 128 < N)
+      for (int kb = kb0; kb < min(kb1, kb0 + stages * KSUB); ++kb, next_k(k)) tma_prefetch_2d(k.w, k.col, t.n0 + side * 128);
   }
   pdl_wait();
   pdl_launch_dependents();  // after the wait: whoever starts early finds everything before this kernel complete
@@ -251,15 +247,12 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
 #pragma unroll 1
         for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
           const int nsub = KSUB == 1 ? 1 : min(KSUB, kb1 - kb);
-          const bool w_done = it < npre;  // this stage's W halves are already on their way
-          if (!w_done) {
-            if (!mbar_wait(&empty[st], ph, abort_flag, timeout_ns)) break;
-            if (side == 0) mbar_expect_tx(&full[st], 2 * blk_bytes * uint32_t(nsub));
-          }
+          if (!mbar_wait(&empty[st], ph, abort_flag, timeout_ns)) break;
+          if (side == 0) mbar_expect_tx(&full[st], 2 * blk_bytes * uint32_t(nsub));
 #pragma unroll
           for (int sub = 0; sub < KSUB; ++sub) {
             if (sub >= nsub) break;
-            if (!w_done) load_w(st, sub, k, t);
+            load_w(st, sub, k, t);
             load_x(st, sub, k, t);
             next_k(k);
           }

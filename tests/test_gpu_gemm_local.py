@@ -122,3 +122,40 @@ def test_a_limit_on_ctas_is_kept():
         torch.cuda.synchronize()
         comm.check()
         torch.testing.assert_close(outs[0].double(), torch.cat(xs).double() @ ws[0].double().t(), atol=2e-3, rtol=2e-3)
+
+
+@pytest.mark.parametrize("producer", ["strided", "norm"])
+@pytest.mark.parametrize("call", ["linear_allreduce", "linear_allreduce packed", "linear_allreduce exchange", "linear", "allgather_linear"])
+@pytest.mark.parametrize("world", [1, 2])
+def test_weight_made_by_the_kernel_right_before(world, call, producer):
+    """The kernels are launched while their predecessor may still run, so a weight that it writes must not be loaded before
+    the wait for it: the copy of a strided weight inside the call, and a weight that is the output of a kernel which lets its
+    dependents start before it stores.  The buffers come back from call to call with other values in them."""
+    M, K, N = 16, 1024, 4096
+    g = torch.Generator(device="cuda").manual_seed(0)
+    with Communicator.virtual(world, 0, staging_bytes=96 << 20) as comm:
+        for _ in range(10):
+            xs = [_rand(g, torch.float16, M, K) for _ in range(world)]
+            base = [_rand(g, torch.float16, N, K, scale=0.02) for _ in range(world)]
+            gam = [_rand(g, torch.float16, K, scale=0.02) for _ in range(world)]
+            ws = [b.t().contiguous().t() for b in base]  # [N, K], not contiguous
+            torch.cuda.synchronize()
+            if producer == "norm":
+                ws = comm.allreduce_residual_rmsnorm(base, base, gam)[0]
+            if call == "linear_allreduce":
+                outs = comm.linear_allreduce(xs, ws)
+            elif call == "linear_allreduce packed":
+                outs = comm.linear_allreduce(xs, [comm.pack_weight(w) for w in ws])
+            elif call == "linear_allreduce exchange":
+                outs = comm.linear_allreduce(xs, ws, fused=True)
+            elif call == "linear":
+                outs = comm.linear(xs, ws)
+            else:
+                outs = comm.allgather_linear(xs, ws)
+            torch.cuda.synchronize()
+            comm.check()
+            part = [x.double() @ w.double().t() for x, w in zip(xs, ws)]
+            for i, o in enumerate(outs):
+                want = torch.cat(xs).double() @ ws[i].double().t() if call == "allgather_linear" else part[i] if call == "linear" else sum(part)
+                # one rounding per rank and one of the sum, of values of a few units
+                torch.testing.assert_close(o.double(), want, atol=4e-3, rtol=2 * HALF_ULP[torch.float16])

@@ -24,7 +24,6 @@
 
 #include "../mem/symm_heap.h"
 #include "kernel_table.h"
-#include "tuner.h"
 
 namespace b200ipc {
 
@@ -108,8 +107,7 @@ class Comm {
   // Size -> algorithm choice used for AlgoSpec::automatic: the measured table of tuner.h unless
   // set_thresholds() installed explicit cut-offs (0, 0 restores the table).
   // `direct`: an emulated world whose buffers the barrier-based kernel can use as they are.
-  AlgoSpec choose_all_reduce(size_t bytes, bool symmetric, bool direct = false, uint32_t flags = 0) const;
-  size_t flag_max_bytes(EmuOp op, uint32_t flags) const;
+  AlgoSpec choose_all_reduce(size_t bytes, bool symmetric, bool direct = false) const;
   void set_thresholds(size_t oneshot_max_bytes, size_t ll_max_bytes) {
     oneshot_max_bytes_ = oneshot_max_bytes;
     ll_max_bytes_ = ll_max_bytes;
@@ -193,6 +191,7 @@ class Comm {
   void common_init(const CommOptions& opt);
   CollInfo launch_ll(LLOpId op, AlgoSpec algo, DType t, const void* const* ins, void* const* outs, size_t nelems,
                      LaunchGeom geom, cudaStream_t stream, uint32_t flags);
+  bool auto_direct(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems, uint32_t flags) const;
   bool bulk_direct_ok(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems) const;
   CollInfo launch_bulk(BulkModeId mode, bool nvls, DType t, const void* const* ins, void* const* outs, size_t nelems,
                        LaunchGeom geom, cudaStream_t stream, uint32_t flags);

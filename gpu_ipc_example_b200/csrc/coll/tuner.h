@@ -58,29 +58,6 @@ inline const TuneRow* tune_table(int world, bool symmetric, int* rows) {
   return symmetric ? w2_sym : w2_user;
 }
 
-// Emulated worlds (all ranks on one GPU), calls whose ranks meet at a barrier (flags given, or a communicator that was moved to
-// the 8-byte-granule formats; others take the direct kernel at every size): the input size in bytes up to which the
-// flag-in-data kernels are used; above it the barrier-based kernel that reads and writes the callers' own buffers (BulkPlace::Direct).  There is no link whose hops
-// a flag-in-data message saves, and its rings are extra passes over the same L2 and HBM; what it saves is the barrier.
-// Device time on one B200, fp16, flag-in-data against direct:
-//   all-reduce      2 ranks  512 KiB 3.3 / 3.4 us,  1 MiB 4.7 / 3.4,  16 MiB 25.8 / 8.4
-//                   4 ranks   64 KiB 3.3 / 3.5,   256 KiB 4.0 / 3.5,  16 MiB 102 / 19
-//                   8 ranks    8 KiB 4.4 / 4.2,    64 KiB 5.3 / 4.2,  16 MiB 282 / 50
-//   reduce-scatter  2 ranks  512 KiB 3.0 / 3.3,     1 MiB 3.5 / 3.5,   8 MiB 11.2 / 4.9
-//                   4 ranks  128 KiB 3.2 / 3.3,   256 KiB 3.4 / 3.3,   8 MiB 11.2 / 6.3 (direct both)
-//                   8 ranks   16 KiB 4.0 / 3.6,     2 MiB 21.5 / 6
-//   all-gather      2 ranks  512 KiB 3.2 / 3.5,     2 MiB 5.7 / 4.2 (per rank)
-//                   4 ranks   16 KiB 3.8 / 3.4,     1 MiB 8.9 / 5.7
-//                   8 ranks    8 KiB 7.6 / 4.2,     1 MiB 59 / 13.4
-enum class EmuOp : int { AllReduce, ReduceScatter, AllGather };
-inline size_t emulated_flag_max_bytes(EmuOp op, int world) {
-  switch (op) {
-    case EmuOp::AllReduce: return world >= 8 ? 8 * KiB : (world >= 4 ? 64 * KiB : 512 * KiB);
-    case EmuOp::ReduceScatter: return world >= 8 ? 0 : (world >= 4 ? 128 * KiB : 512 * KiB);
-    default: return world >= 4 ? 0 : 512 * KiB;
-  }
-}
-
 // CTAs of the in-switch (NVLS) all-reduce.  Measured on 8 GPUs with 4, 8, 12, 16, 24, 32 and 148 CTAs from 1 MiB
 // to 512 MiB: 8 CTAs were the fastest at every size (16 MiB: 49.2 us against 59.0 with 32; 512 MiB: 1120 us
 // against 1175 with 148) - the switch's reduction path is saturated by a few hundred loads in flight, and every

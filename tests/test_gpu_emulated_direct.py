@@ -91,7 +91,7 @@ def test_overlapping_buffers_are_staged(comm):
 
 
 @pytest.mark.parametrize("nbytes", [8 << 10, (8 << 10) + 2, 64 << 10, (64 << 10) + 2, 512 << 10, (512 << 10) + 2, 4 << 20])
-def test_auto_on_both_sides_of_the_cut_offs(comm, nbytes):
+def test_auto_at_any_size(comm, nbytes):
     w, n = comm.world, nbytes // 2
     xs = _inputs(w, n, seed=4)
     want = torch.stack([x.float() for x in xs]).sum(0)
@@ -104,3 +104,38 @@ def test_auto_on_both_sides_of_the_cut_offs(comm, nbytes):
         _close(outs[r], want)
         assert torch.equal(gathered[r], torch.cat([x[:n // 2 * 2] for x in xs]))
         _close(scattered[r], want[:n // w * w][r * (n // w):(r + 1) * (n // w)])
+
+
+@pytest.mark.parametrize("nbytes", [4 << 10, 96 << 10, 1 << 20, 12 << 20])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_auto_rounds_after_each_add_where_the_flag_asks_for_it(comm, nbytes, dtype):
+    """Every element is a chain of adds in T.  The schedules take the ranks in rank order, from a rank of their choice."""
+    w, n = comm.world, nbytes // 2
+    xs = _inputs(w, n, dtype, seed=5)
+
+    def chains(vs):
+        for order in (vs, vs[::-1]):
+            for r in range(w):
+                s = order[r]
+                for k in range(1, w):
+                    s = s + order[(r + k) % w]
+                yield s
+
+    def is_chain(got, vs):
+        ok = torch.zeros_like(got, dtype=torch.bool)
+        for s in chains(vs):
+            ok |= got == s
+        return bool(ok.all())
+
+    # two ranks have one add; for more, a sum in fp32 is seen
+    assert is_chain(sum(x.float() for x in xs).to(dtype), xs) == (w == 2)
+    outs = comm.all_reduce([x.clone() for x in xs], [torch.empty_like(x) for x in xs], flags=1)
+    torch.cuda.synchronize()
+    comm.check()
+    assert all(torch.equal(o, outs[0]) for o in outs) and is_chain(outs[0], xs)
+    if nbytes <= 8 << 20:  # up to here `auto` has a reduce-scatter that looks at the flag
+        m = n // (2 * w) * 2 * w
+        outs = comm.reduce_scatter([x[:m].clone() for x in xs], flags=1)
+        torch.cuda.synchronize()
+        comm.check()
+        assert is_chain(torch.cat(outs), [x[:m] for x in xs])

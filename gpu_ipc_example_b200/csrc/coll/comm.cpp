@@ -640,10 +640,10 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
 // whose hops a flag-in-data message saves, and its rings are extra passes over the same L2 and HBM.  Device time on one
 // B200, fp16, flag-in-data against direct: all-reduce 8 ranks 2 KiB 7.2 / 4.6 us (cold), 64 KiB 5.3 / 4.2, 16 MiB 282 / 50;
 // reduce-scatter 8 ranks 2 MiB 21.5 / 6; all-gather 8 ranks 1 MiB 59 / 13.4.  The direct kernel sums in fp32 and sends no messages,
-// so a call whose flags say how sums are rounded or that ranks stay silent keeps the kernels that look at them; a communicator
-// that was moved to the 8-byte-granule formats keeps using those.
+// so a call whose flags say how sums are rounded or that ranks stay silent keeps the kernels that look at them, and so does
+// one whose waits are to be traced; a communicator that was moved to the 8-byte-granule formats keeps using those.
 bool Comm::auto_direct(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems, uint32_t flags) const {
-  return flags == 0 && !safe_protos_ && bulk_direct_ok(mode, ins, outs, nelems);
+  return flags == 0 && !trace_wires_ && !safe_protos_ && bulk_direct_ok(mode, ins, outs, nelems);
 }
 
 AlgoSpec Comm::choose_all_reduce(size_t bytes, bool symmetric, bool direct) const {

@@ -70,3 +70,15 @@ def test_trace_ring_records_every_completed_wait():
         comm.all_reduce(xs, None, "simple_pcie_p", ctas=2, warps=4)
         torch.cuda.synchronize()
         assert comm.trace_events(0)[1] == total  # nothing added once tracing is off
+
+
+def test_auto_has_waits_to_record_while_tracing():
+    with Communicator.virtual(4, 0, staging_bytes=8 << 20) as comm:
+        comm.set_trace(True)
+        xs = [torch.randn(4096, device="cuda").half() for _ in range(4)]
+        comm.all_reduce(xs)
+        comm.reduce_scatter(xs)
+        comm.all_gather(xs)
+        torch.cuda.synchronize()
+        comm.check()
+        assert comm.trace_events(0)[1] >= 3 * 3  # a wait for each other rank in each of the three

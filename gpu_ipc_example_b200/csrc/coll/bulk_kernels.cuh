@@ -23,11 +23,11 @@ enum class BulkMode : int { AllReduce = 0, ReduceScatter = 1, AllGather = 2 };
 // aux[1] bits
 constexpr uint64_t kBulkCopyIn = 1;   // stage `in` into the symmetric buffer first
 constexpr uint64_t kBulkCopyOut = 2;  // copy the result from the symmetric buffer to `out`
-constexpr uint64_t kBulkNoMeet = 4;   // Direct: the ranks do not meet (the launch need not be cooperative)
 
 // Where the ranks' data lives.  Heap: at one offset of every rank's symmetric heap.  Direct: in the callers' own
 // buffers, which every rank of an emulated world can address (the launch arguments hold all of them), so that
-// nothing is staged.
+// nothing is staged and the ranks do not meet: they are block rows of one launch, which starts when every input is in place
+// and whose end is the point that whoever comes after it waits for.  `auto` takes it there; "bulk" by name is Heap.
 enum class BulkPlace : int { Heap = 0, Direct = 1 };
 
 __device__ __forceinline__ void st_release_sys_u32(uint32_t* p, uint32_t v) {
@@ -208,7 +208,7 @@ __device__ __forceinline__ void st_stream_u4(void* p, uint4 v) { __stcs(reinterp
 // Streaming stores: 22.9 -> 19.2 us at 8 MiB x 8, level elsewhere; streaming loads lose where the producer left the
 // inputs in L2 (reduce-scatter of 8 MiB 9.0 -> 12.0 us).
 template <typename T, int N, BulkMode M>
-__device__ __forceinline__ void bulk_direct_body(const KArgs& args, int r, int64_t shard_elems, int64_t valid, bool mute) {
+__device__ __forceinline__ void bulk_direct_body(const KArgs& args, int r, int64_t shard_elems, int64_t valid) {
   constexpr int kU = M == BulkMode::AllGather ? 4 : bulk_unroll(N, false);
   const int tid = int(threadIdx.x);
   const int nthreads = int(blockDim.x);
@@ -217,7 +217,6 @@ __device__ __forceinline__ void bulk_direct_body(const KArgs& args, int r, int64
   auto in16 = [&](int q) { return static_cast<const uint16_t*>(args.v[q].in); };
   auto out16 = [&](int q) { return static_cast<uint16_t*>(args.v[q].out); };
   if (M == BulkMode::AllGather) {
-    if (mute) return;
     const uint16_t* src = in16(r);
     int64_t head = (8 - (e0 & 7)) & 7;  // elements in front of the first vector that is aligned in the destination
     if (head > valid) head = valid;
@@ -275,7 +274,7 @@ __device__ __forceinline__ void bulk_direct_body(const KArgs& args, int r, int64
         const uint4 res = acc8_pack<T>(a);
         if (M == BulkMode::ReduceScatter) {
           st_stream_u4(out16(r) + i * 8, res);
-        } else if (!mute) {
+        } else {
 #pragma unroll
           for (int q = 0; q < N; ++q) st_stream_u4(out16(q) + e0 + i * 8, res);
         }
@@ -303,7 +302,7 @@ __device__ __forceinline__ void bulk_direct_body(const KArgs& args, int r, int64
       const T res = T(a);
       if (M == BulkMode::ReduceScatter) {
         reinterpret_cast<T*>(out16(r))[e] = res;
-      } else if (!mute) {
+      } else {
 #pragma unroll
         for (int q = 0; q < N; ++q) reinterpret_cast<T*>(out16(q))[o0 + e] = res;
       }
@@ -352,6 +351,10 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
     int64_t v = nelems - int64_t(s) * shard_elems;
     return v < 0 ? 0 : (v > shard_elems ? shard_elems : v);
   };
+  if constexpr (P == BulkPlace::Direct) {
+    bulk_direct_body<T, N, M>(args, r, shard_elems, valid(r));
+    return;
+  }
   // A slab is blockDim consecutive vectors; slab j belongs to CTA j % gridDim.x on every rank
   // and a CTA keeps kU of its slabs in flight.
   const int64_t ntiles = (shard_vec + nthreads - 1) / nthreads;
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
   uint16_t* out16 = static_cast<uint16_t*>(me.out);
 
   // ---- phase 0: stage the input ------------------------------------------------
-  if (P == BulkPlace::Heap && M != BulkMode::AllGather && copy_in) {
+  if (M != BulkMode::AllGather && copy_in) {
     for (int s = 0; s < N; ++s) {
       const int64_t nv = valid(s);
       for (int64_t tile = b; tile < ntiles; tile += int64_t(G) * kU)
@@ -376,14 +379,10 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
   }
   // Every rank has arrived (so it has left the previous collective and, for the
   // reducing modes, its input is in place) before any remote access.
-  // (Direct: all ranks are block rows of this one launch, which starts when every input is in place, and a rank only
-  // reads and writes its own shard of the buffers.  The barrier is for ranks that were told to send nothing.)
-  if ((P == BulkPlace::Heap || (me.aux[1] & kBulkNoMeet) == 0) && !cta_rank_barrier(me, lay, bar + 1, 10, /*publish=*/copy_in)) return;
+  if (!cta_rank_barrier(me, lay, bar + 1, 10, /*publish=*/copy_in)) return;
 
   // ---- phase 1: the collective ---------------------------------------------------
-  if constexpr (P == BulkPlace::Direct) {
-    bulk_direct_body<T, N, M>(args, r, shard_elems, valid(r), (me.flags & kMuteSends) != 0);
-  } else if (M == BulkMode::AllGather) {
+  if (M == BulkMode::AllGather) {
     const uint16_t* src16 = copy_in ? in16 : reinterpret_cast<const uint16_t*>(my_buf + int64_t(r) * shard_vec * 16);
     for (int64_t tile = b; tile < ntiles; tile += int64_t(G) * kU) {
       uint4 v[kU];
@@ -462,11 +461,10 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
   }
 
   // ---- phase 2: everyone's loads and stores are done ---------------------------------
-  // (Direct: all ranks are block rows of this one launch, whose end is that point for whoever comes after it.)
-  if (P == BulkPlace::Heap && !cta_rank_barrier(me, lay, bar + 2, 11, /*publish=*/true)) return;
+  if (!cta_rank_barrier(me, lay, bar + 2, 11, /*publish=*/true)) return;
 
   // ---- phase 3: hand the result to the caller ----------------------------------------
-  if (P == BulkPlace::Heap && M != BulkMode::ReduceScatter && copy_out) {
+  if (M != BulkMode::ReduceScatter && copy_out) {
     for (int s = 0; s < N; ++s) {
       const int64_t nv = valid(s);
       for (int64_t tile = b; tile < ntiles; tile += int64_t(G) * kU)

@@ -502,7 +502,7 @@ CollInfo Comm::launch_ll(LLOpId op, AlgoSpec algo, DType t, const void* const* i
 // ----------------------------------------------------------------------------
 // Large messages
 // ----------------------------------------------------------------------------
-// Whether the barrier-based kernel can work on the callers' own buffers: all ranks live in this process (their buffers
+// Whether the large-message kernel can work on the callers' own buffers: all ranks live in this process (their buffers
 // are in one launch's arguments and one address space), everything is 16-byte aligned, and no output overlaps an
 // input except as the collective's in-place form (the staged form has read all inputs before it writes).
 bool Comm::bulk_direct_ok(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems) const {
@@ -524,11 +524,10 @@ bool Comm::bulk_direct_ok(BulkModeId mode, const void* const* ins, void* const* 
   return true;
 }
 
-CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* const* ins, void* const* outs,
+CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, bool direct, DType t, const void* const* ins, void* const* outs,
                            size_t nelems, LaunchGeom geom, cudaStream_t stream, uint32_t flags) {
   const int N = world_;
   if (nvls) B200_REQUIRE(has_nvls(), "NVLS was not set up for this communicator: " << heaps_[0]->nvls_note());
-  const bool direct = !nvls && bulk_direct_ok(mode, ins, outs, nelems);
   KernelFn fn = direct ? bulk_direct_kernel_lookup(mode, t, N) : bulk_kernel_lookup(mode, t, N, nvls);
   B200_REQUIRE(fn != nullptr, "no kernel for world size " << N << " (supported: 2, 4, 8)");
   const HeapLayout& lay = heaps_[0]->layout();
@@ -549,7 +548,7 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
   const size_t sym_bytes = size_t(shard_vec) * 16 * size_t(N);
   const bool exact = (mode == BulkModeId::AllReduce) ? (nelems % (8 * size_t(N)) == 0) : (shard_elems % 8 == 0);
 
-  // An emulated world works on the callers' buffers as they are (`direct`).  Else: zero-copy when the caller's
+  // `direct` works on the callers' buffers as they are.  Else: zero-copy when the caller's
   // buffers already live in the symmetric heap at the same offset on every rank and the shards are vector-exact.
   //   all-reduce: in place on a symmetric buffer
   //   reduce-scatter: symmetric input
@@ -592,6 +591,7 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
   }
 
   const int threads = kBulkThreadsPerCta;
+  // the direct form's CTAs wait for nobody; for them this is one full wave
   int cap = std::min(resident_ctas(fn, threads, 0), kMaxBarrierCtas);
   B200_REQUIRE(cap >= 1, "bulk kernel does not fit on the device");
   const int64_t tile_vec = int64_t(threads);  // a slab: one vector per thread; a CTA keeps kU slabs in flight
@@ -611,14 +611,13 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, DType t, const void* cons
 
   KArgs args;
   fill_views(&args, ins, outs, nelems, flags);
-  const bool meet = !direct || (flags & kMuteSends) != 0;
-  const uint32_t bar = meet ? take_barrier() : 0;
+  const uint32_t bar = direct ? 0 : take_barrier();
   for (int i = 0; i < nlocal(); ++i) {
     args.v[i].bar_seq = bar;
     args.v[i].aux[0] = sym_off;
-    args.v[i].aux[1] = copy_flags | (meet ? 0 : kBulkNoMeetBit);
+    args.v[i].aux[1] = copy_flags;
   }
-  launch(fn, ctas, threads, &args, 0, stream, false, meet);
+  launch(fn, ctas, threads, &args, 0, stream, false, /*meet=*/!direct);
 
   CollInfo info;
   info.sched = nvls ? SchedKind::Nvls : SchedKind::Bulk;
@@ -697,10 +696,12 @@ CollInfo Comm::all_reduce(AlgoSpec algo, DType t, const void* const* ins, void* 
     info.sched = SchedKind::OneShot;
     return info;
   }
+  bool direct = false;
   if (algo.automatic) {
     bool symmetric = true;
     for (int i = 0; i < nlocal(); ++i) symmetric &= (ins[i] == outs[i]) && sym_offset_of(ins[i], i) != SIZE_MAX;
-    algo = choose_all_reduce(nelems * 2, symmetric, auto_direct(BulkModeId::AllReduce, ins, outs, nelems, extra_flags));
+    direct = auto_direct(BulkModeId::AllReduce, ins, outs, nelems, extra_flags);
+    algo = choose_all_reduce(nelems * 2, symmetric, direct);
   }
   for (int i = 0; i < nlocal(); ++i) {
     B200_REQUIRE((reinterpret_cast<uintptr_t>(ins[i]) & 3) == 0 && (reinterpret_cast<uintptr_t>(outs[i]) & 3) == 0,
@@ -712,8 +713,8 @@ CollInfo Comm::all_reduce(AlgoSpec algo, DType t, const void* const* ins, void* 
     case SchedKind::Ring: return launch_ll(LLOpId::ArRing, algo, t, ins, outs, nelems, geom, stream, extra_flags);
     case SchedKind::Bisect: return launch_ll(LLOpId::ArBisect, algo, t, ins, outs, nelems, geom, stream, extra_flags);
     case SchedKind::OneShot: return launch_ll(LLOpId::ArOneShot, algo, t, ins, outs, nelems, geom, stream, extra_flags);
-    case SchedKind::Bulk: return launch_bulk(BulkModeId::AllReduce, false, t, ins, outs, nelems, geom, stream, extra_flags);
-    default: return launch_bulk(BulkModeId::AllReduce, true, t, ins, outs, nelems, geom, stream, extra_flags);
+    case SchedKind::Bulk: return launch_bulk(BulkModeId::AllReduce, false, direct, t, ins, outs, nelems, geom, stream, extra_flags);
+    default: return launch_bulk(BulkModeId::AllReduce, true, false, t, ins, outs, nelems, geom, stream, extra_flags);
   }
 }
 
@@ -728,10 +729,11 @@ CollInfo Comm::all_gather(AlgoSpec algo, DType t, const void* const* ins, void* 
     info.sched = SchedKind::Ring;
     return info;
   }
+  bool direct = false;
   if (algo.automatic) {
     algo = AlgoSpec{};
     const size_t bytes = nelems * 2;
-    const bool direct = nelems % 2 == 0 && auto_direct(BulkModeId::AllGather, ins, outs, nelems, extra_flags);
+    direct = nelems % 2 == 0 && auto_direct(BulkModeId::AllGather, ins, outs, nelems, extra_flags);
     // two ranks: the direct flag-in-data push moves the same bytes as any other form and needs no
     // barrier; measured ahead of the barrier-based kernels and of NCCL up to 64 MiB per rank
     // measured on 8 GPUs (bytes per rank): the direct push wins up to 1 MiB (23 us against NCCL's 47), the
@@ -750,7 +752,8 @@ CollInfo Comm::all_gather(AlgoSpec algo, DType t, const void* const* ins, void* 
     }
   }
   if (algo.sched == SchedKind::Bulk || algo.sched == SchedKind::Nvls)
-    return launch_bulk(BulkModeId::AllGather, algo.sched == SchedKind::Nvls, t, ins, outs, nelems, geom, stream, extra_flags);
+    return launch_bulk(BulkModeId::AllGather, algo.sched == SchedKind::Nvls, direct, t, ins, outs, nelems, geom, stream,
+                       extra_flags);
   B200_REQUIRE(algo.sched == SchedKind::Ring, "all-gather runs on the ring, direct, bulk or nvls schedules");
   return launch_ll(algo.direct_allgather ? LLOpId::AgDirect : LLOpId::AgRing, algo, t, ins, outs, nelems, geom, stream,
                    extra_flags);
@@ -768,9 +771,10 @@ CollInfo Comm::reduce_scatter(AlgoSpec algo, DType t, const void* const* ins, vo
     return info;
   }
   const bool was_auto = algo.automatic;
+  bool direct = false;
   if (algo.automatic) {
     algo = AlgoSpec{};
-    const bool direct = nelems % size_t(world_) == 0 && auto_direct(BulkModeId::ReduceScatter, ins, outs, nelems, extra_flags);
+    direct = nelems % size_t(world_) == 0 && auto_direct(BulkModeId::ReduceScatter, ins, outs, nelems, extra_flags);
     // small inputs: one flag-in-data push to each slice's owner, no barrier
     if (direct) {
       algo.sched = SchedKind::Bulk;
@@ -795,7 +799,7 @@ CollInfo Comm::reduce_scatter(AlgoSpec algo, DType t, const void* const* ins, vo
   }
   B200_REQUIRE(algo.sched == SchedKind::Bulk || algo.sched == SchedKind::Nvls,
                "reduce-scatter runs on the parallel (flag-in-data), bulk or nvls schedules");
-  return launch_bulk(BulkModeId::ReduceScatter, algo.sched == SchedKind::Nvls, t, ins, outs, nelems, geom, stream,
+  return launch_bulk(BulkModeId::ReduceScatter, algo.sched == SchedKind::Nvls, direct, t, ins, outs, nelems, geom, stream,
                      extra_flags);
 }
 

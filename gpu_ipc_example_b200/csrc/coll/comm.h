@@ -193,7 +193,8 @@ class Comm {
                      LaunchGeom geom, cudaStream_t stream, uint32_t flags);
   bool auto_direct(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems, uint32_t flags) const;
   bool bulk_direct_ok(BulkModeId mode, const void* const* ins, void* const* outs, size_t nelems) const;
-  CollInfo launch_bulk(BulkModeId mode, bool nvls, DType t, const void* const* ins, void* const* outs, size_t nelems,
+  // direct: on the callers' own buffers (bulk_direct_ok)
+  CollInfo launch_bulk(BulkModeId mode, bool nvls, bool direct, DType t, const void* const* ins, void* const* outs, size_t nelems,
                        LaunchGeom geom, cudaStream_t stream, uint32_t flags);
 
   int world_ = 1;

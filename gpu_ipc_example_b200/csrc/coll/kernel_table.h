@@ -33,6 +33,5 @@ constexpr int bulk_unroll(int world, bool nvls) { return nvls ? 8 : (world >= 8 
 // Bits of RankView::aux[1] for the bulk kernels.
 constexpr uint64_t kBulkCopyInBit = 1;   // stage the caller's input into the symmetric buffer
 constexpr uint64_t kBulkCopyOutBit = 2;  // copy the result from the symmetric buffer to the caller
-constexpr uint64_t kBulkNoMeetBit = 4;   // callers' own buffers: no barrier between the ranks
 
 }  // namespace b200ipc

@@ -13,7 +13,7 @@ static_assert(int(LLOpId::ArParallel) == int(LLOp::ArParallel) && int(LLOpId::Ag
                   int(LLOpId::RsParallel) == int(LLOp::RsParallel),
               "LLOpId must mirror LLOp");
 static_assert(kBulkThreadsPerCta == kBulkThreads, "thread count mismatch");
-static_assert(kBulkCopyInBit == kBulkCopyIn && kBulkCopyOutBit == kBulkCopyOut && kBulkNoMeetBit == kBulkNoMeet, "flag mismatch");
+static_assert(kBulkCopyInBit == kBulkCopyIn && kBulkCopyOutBit == kBulkCopyOut, "flag mismatch");
 
 #define B200_DECLARE(OP)                                             \
   template <> LLKernelFn ll_lookup<LLOp::OP, __half>(ProtoKind, int); \

@@ -31,9 +31,9 @@ def test_all_reduce(comm, n, dtype):
     xs = _inputs(comm.world, n, dtype)
     want = torch.stack([x.float() for x in xs]).sum(0)
     outs = [torch.full_like(x, 9) for x in xs]
-    comm.all_reduce(xs, outs, "bulk")
+    comm.all_reduce(xs, outs)
     assert comm.last_info.sched == "bulk" and not comm.last_info.staged
-    comm.all_reduce(xs, None, "bulk")  # in place
+    comm.all_reduce(xs)  # in place
     torch.cuda.synchronize()
     comm.check()
     for x, o in zip(xs, outs):
@@ -41,13 +41,13 @@ def test_all_reduce(comm, n, dtype):
         assert torch.equal(x, o)
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 8, 12, 23, 4096, 4097, 70001, 70006, 262144 + 2])
+@pytest.mark.parametrize("n", [2, 4, 6, 8, 12, 22, 4096, 4098, 70002, 70006, 262144 + 2])
 def test_all_gather(comm, n):
     xs = _inputs(comm.world, n, seed=1)
     want = torch.cat(xs)
     outs = [torch.zeros(comm.world * n + 16, device="cuda", dtype=torch.float16) for _ in xs]
     got = [o[:comm.world * n] for o in outs]
-    comm.all_gather(xs, got, "allgather_bulk")
+    comm.all_gather(xs, got)
     assert comm.last_info.sched == "bulk" and not comm.last_info.staged
     torch.cuda.synchronize()
     comm.check()
@@ -57,7 +57,7 @@ def test_all_gather(comm, n):
         parts = [g[r * n:(r + 1) * n] for r, g in enumerate(got)]
         for r, p in enumerate(parts):
             p.copy_(xs[r] + 1)
-        comm.all_gather(parts, got, "allgather_bulk")
+        comm.all_gather(parts, got)
         torch.cuda.synchronize()
         comm.check()
         assert all(torch.equal(g, want + 1) for g in got)
@@ -68,7 +68,7 @@ def test_all_gather(comm, n):
 def test_reduce_scatter(comm, slice_, dtype):
     xs = _inputs(comm.world, comm.world * slice_, dtype, seed=2)
     want = torch.stack([x.float() for x in xs]).sum(0)
-    outs = comm.reduce_scatter(xs, None, "bulk")
+    outs = comm.reduce_scatter(xs)
     assert comm.last_info.sched == "bulk" and not comm.last_info.staged
     torch.cuda.synchronize()
     comm.check()
@@ -76,18 +76,51 @@ def test_reduce_scatter(comm, slice_, dtype):
         _close(o, want[r * slice_:(r + 1) * slice_])
 
 
-def test_overlapping_buffers_are_staged(comm):
-    """An output that lies inside an input, but not where the in-place form has it."""
-    n = 8 * comm.world * 1000
+def test_overlapping_buffers_take_another_kernel(comm):
+    """An output that lies inside an input, but not where the in-place form has it.  Above what the flag-in-data kernels take
+    (8 MiB), so the inputs are staged."""
+    n = 8 * 600000
     xs = _inputs(comm.world, n, seed=3)
     want = torch.stack([x.float() for x in xs]).sum(0)
     outs = [x[:n // comm.world] for x in xs]
-    comm.reduce_scatter(xs, outs, "bulk")
+    comm.reduce_scatter(xs, outs)
     assert comm.last_info.staged
     torch.cuda.synchronize()
     comm.check()
     for r, o in enumerate(outs):
         _close(o, want[r * (n // comm.world):(r + 1) * (n // comm.world)])
+
+
+@pytest.mark.parametrize("n", [8, 4096 * 8 + 8, 1234568])
+def test_by_name_it_is_the_kernel_with_the_barrier(comm, n):
+    """What one process per GPU runs: staged from plain buffers, zero-copy on the symmetric heap."""
+    w = comm.world
+    xs = _inputs(w, n, seed=6)
+    want = torch.stack([x.float() for x in xs]).sum(0)
+    outs = comm.all_reduce(xs, [torch.empty_like(x) for x in xs], "bulk")
+    assert comm.last_info.staged
+    gathered = comm.all_gather(xs, None, "allgather_bulk")
+    assert comm.last_info.staged
+    scattered = comm.reduce_scatter([x[:n // (8 * w) * 8 * w] for x in xs], None, "bulk") if n >= 8 * w else None
+    if scattered:
+        assert comm.last_info.staged
+    sym = comm.empty([n // (8 * w) * 8 * w], torch.float16) if n >= 8 * w else None
+    if sym:
+        for s, x in zip(sym, xs):
+            s.copy_(x[:s.numel()])
+        barrier = comm.last_info.first_flag  # the number of its barrier: the direct kernel takes none
+        comm.all_reduce(sym, None, "bulk")
+        assert not comm.last_info.staged and comm.last_info.first_flag > barrier
+    torch.cuda.synchronize()
+    comm.check()
+    for r in range(w):
+        _close(outs[r], want)
+        assert torch.equal(gathered[r], torch.cat(xs))
+        if scattered:
+            m = scattered[r].numel()
+            _close(scattered[r], want[r * m:(r + 1) * m])
+            _close(sym[r], want[:sym[r].numel()])
+    comm.free_symmetric()
 
 
 @pytest.mark.parametrize("nbytes", [8 << 10, (8 << 10) + 2, 64 << 10, (64 << 10) + 2, 512 << 10, (512 << 10) + 2, 4 << 20])

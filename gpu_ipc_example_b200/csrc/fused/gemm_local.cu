@@ -160,7 +160,9 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
 }
 
 void check_local(Comm& comm, int64_t M, int64_t N, int64_t K) {
-  B200_REQUIRE(comm.nlocal() == comm.world() && comm.world() <= kMaxRanks, "every rank must be driven by this process");
+  B200_REQUIRE(comm.nlocal() == comm.world(), "every rank must be driven by this process");
+  const int W = comm.world();
+  B200_REQUIRE(W == 1 || W == 2 || W == 4 || W == 8, "world size must be 1, 2, 4 or 8");  // a tile of merged shards is cut in powers of two
   B200_REQUIRE(M > 0 && N > 0 && K > 0, "empty GEMM");
   B200_REQUIRE(N % 64 == 0, "N must be a multiple of 64");
   B200_REQUIRE(K % 8 == 0, "K must be a multiple of 8");

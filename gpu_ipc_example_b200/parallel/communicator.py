@@ -68,7 +68,8 @@ class Communicator:
         self.world = self._C.world(handle)
         self.nlocal = self._C.nlocal(handle)
         self.rank = self._C.rank(handle, 0)
-        self._direct = self.nlocal == self.world  # this process drives every rank: nothing has to be exchanged
+        # this process drives every rank: nothing has to be exchanged (the kernels for that take these worlds)
+        self._direct = self.nlocal == self.world and self.world in (1, 2, 4, 8)
         self._info = None  # the launch report of the last call, as the native code gives it
         ops = torch.ops.b200ipc
         self._all_reduce_lists, self._all_gather_lists = ops.all_reduce_lists.default, ops.all_gather_lists.default

@@ -159,3 +159,17 @@ def test_weight_made_by_the_kernel_right_before(world, call, producer):
                 want = torch.cat(xs).double() @ ws[i].double().t() if call == "allgather_linear" else part[i] if call == "linear" else sum(part)
                 # one rounding per rank and one of the sum, of values of a few units
                 torch.testing.assert_close(o.double(), want, atol=4e-3, rtol=2 * HALF_ULP[torch.float16])
+
+
+@pytest.mark.parametrize("world", [3, 5, 6, 7])
+def test_other_world_sizes_are_refused(world):
+    """A communicator can be made for them, the kernels are for 1, 2, 4 and 8."""
+    with Communicator.virtual(world, 0, staging_bytes=16 << 20) as comm:
+        xs = [torch.zeros(8, 128, device="cuda").half() for _ in range(world)]
+        ws = [torch.zeros(64, 128, device="cuda").half() for _ in range(world)]
+        outs = [torch.zeros(8 * world, 64, device="cuda").half() for _ in range(world)]
+        for call in (lambda: comm.allgather_linear(xs, ws), lambda: comm.linear_allreduce(xs, ws),
+                     lambda: torch.ops.b200ipc.local_ag_gemm(xs, ws, outs, comm._h),
+                     lambda: torch.ops.b200ipc.local_gemm_ar(xs, ws, [], [], [o[:8] for o in outs], [], 1e-5, False, comm._h)):
+            with pytest.raises(RuntimeError, match="world size"):
+                call()

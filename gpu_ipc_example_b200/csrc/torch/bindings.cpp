@@ -345,6 +345,20 @@ std::vector<int64_t> fused_ar_scale_cast(std::vector<at::Tensor> ins, std::vecto
   return info_vec(info);
 }
 
+// What the GEMM + all-reduce kernels read and write as [M, N] or [N] values of x's type, whatever the tensors' own shapes.
+void check_epilogue_tensors(const at::Tensor& x, const std::vector<at::Tensor>& residuals, const std::vector<at::Tensor>& gammas,
+                            const std::vector<at::Tensor>& outs, const std::vector<at::Tensor>& res_outs, int64_t M, int64_t N) {
+  auto each = [&](const std::vector<at::Tensor>& ts, int64_t numel, const char* what) {
+    for (const at::Tensor& t : ts)
+      TORCH_CHECK(t.numel() == numel && t.scalar_type() == x.scalar_type(), "b200ipc: ", what, " must hold ", numel, " elements of ",
+                  x.scalar_type(), ", got ", t.sizes(), " of ", t.scalar_type());
+  };
+  each(residuals, M * N, "residual");
+  each(gammas, N, "gamma");
+  each(outs, M * N, "output");
+  each(res_outs, M * N, "residual output");
+}
+
 // Row-parallel linear + all-reduce (+ residual + RMSNorm).  xs: [M, K] per rank, ws: [N, K] per rank
 // (nn.Linear layout); outs / res_outs / workspaces are symmetric tensors.  residuals / gammas /
 // res_outs may be empty lists.
@@ -371,11 +385,11 @@ std::vector<int64_t> fused_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::T
     TORCH_CHECK(ws[0].size(1) == K, "b200ipc: weight must be [N, K] with the same K as x");
   }
   GemmArWorkspace need = gemm_ar_workspace(c.world(), M, N);
+  check_epilogue_tensors(xs[0], residuals, gammas, outs, res_outs, M, N);
   std::vector<GemmArPtrs> p(size_t(c.nlocal()));
   for (int i = 0; i < c.nlocal(); ++i) {
-    TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes() && outs[i].numel() == M * N,
-                "b200ipc: shape mismatch between ranks");
-    TORCH_CHECK(xs[i].scalar_type() == ws[i].scalar_type() && xs[i].scalar_type() == outs[i].scalar_type(), "b200ipc: dtype mismatch");
+    TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes(), "b200ipc: shape mismatch between ranks");
+    TORCH_CHECK(xs[i].scalar_type() == xs[0].scalar_type() && ws[i].scalar_type() == xs[0].scalar_type(), "b200ipc: dtype mismatch");
     TORCH_CHECK(size_t(workspaces[i].numel() * workspaces[i].element_size()) >= need.total(), "b200ipc: workspace too small, need ",
                 need.total(), " bytes");
     p[size_t(i)].x = xs[i].data_ptr();
@@ -432,11 +446,11 @@ std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::T
   TORCH_CHECK(xs[0].dim() == 2 && ws[0].dim() == 2, "b200ipc: x must be [M, K] and weight [N, K] (or packed)");
   const int64_t M = xs[0].size(0), K = xs[0].size(1), N = ws[0].size(0);
   TORCH_CHECK(ws[0].size(1) == K, "b200ipc: weight must be [N, K] with the same K as x");
+  check_epilogue_tensors(xs[0], residuals, gammas, outs, res_outs, M, N);
   std::vector<GemmArPtrs> p(size_t(c.nlocal()));
   for (int i = 0; i < c.nlocal(); ++i) {
-    TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes() && outs[i].numel() == M * N,
-                "b200ipc: shape mismatch between ranks");
-    TORCH_CHECK(xs[i].scalar_type() == ws[i].scalar_type() && xs[i].scalar_type() == outs[i].scalar_type(), "b200ipc: dtype mismatch");
+    TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes(), "b200ipc: shape mismatch between ranks");
+    TORCH_CHECK(xs[i].scalar_type() == xs[0].scalar_type() && ws[i].scalar_type() == xs[0].scalar_type(), "b200ipc: dtype mismatch");
     p[size_t(i)].x = xs[i].data_ptr();
     p[size_t(i)].w = ws[i].data_ptr();
     p[size_t(i)].residual = residuals.empty() ? nullptr : residuals[i].data_ptr();

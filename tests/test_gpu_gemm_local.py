@@ -173,3 +173,27 @@ def test_other_world_sizes_are_refused(world):
                      lambda: torch.ops.b200ipc.local_gemm_ar(xs, ws, [], [], [o[:8] for o in outs], [], 1e-5, False, comm._h)):
             with pytest.raises(RuntimeError, match="world size"):
                 call()
+
+
+@pytest.mark.parametrize("fused", [None, True])
+def test_operands_of_the_epilogue_are_checked(fused):
+    """A residual that would have to be broadcast, a gamma of another length, 32-bit ones: refused, not read out of range or as
+    16-bit values.  Any shape with the right number of elements is taken, as before."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    M, K, N = 8, 128, 256
+    with Communicator.virtual(2, 0, staging_bytes=16 << 20) as comm:
+        xs, ws = [_rand(g, torch.float16, M, K) for _ in range(2)], [_rand(g, torch.float16, N, K, scale=0.02) for _ in range(2)]
+        res, gam = _rand(g, torch.float16, M, N), _rand(g, torch.float16, N)
+        for r, ga in ((res[0], gam), (res[:1], gam), (res.float(), gam), (res, gam[:64]), (res, gam.float())):
+            for bad in (0, 1):  # either rank's
+                rs, gs = [res, res], [gam, gam]
+                rs[bad], gs[bad] = r.contiguous(), ga.contiguous()
+                with pytest.raises(RuntimeError, match="must hold"):
+                    comm.linear_allreduce(xs, ws, rs, gs, fused=fused)
+        with pytest.raises(RuntimeError, match="dtype"):
+            comm.linear_allreduce(xs, [ws[0], ws[1].bfloat16()], [res] * 2, [gam] * 2, fused=fused)
+        want = comm.linear_allreduce(xs, ws, [res] * 2, [gam] * 2, fused=fused)[0][0].clone()
+        got = comm.linear_allreduce(xs, ws, [res.view(2, M // 2, N)] * 2, [gam.view(1, N)] * 2, fused=fused)[0][0]
+        torch.cuda.synchronize()
+        comm.check()
+        assert torch.equal(got, want)

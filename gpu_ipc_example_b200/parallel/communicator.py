@@ -364,8 +364,9 @@ class Communicator:
         if fused is None:
             fused = M >= 4096 or self.world == 1
             # below 4096 rows the pair of calls also takes what the kernel does not: any N and K, unaligned rows, a
-            # weight that wants a gradient
+            # vector for a weight, ranks with weights of different heights, a weight that wants a gradient
             fits = fused or (N % 64 == 0 and K % 8 == 0 and not any(t.data_ptr() % 16 for t in xs + ws)
+                             and ws[0].dim() == 2 and all(t.shape == ws[0].shape for t in ws)
                              and not (torch.is_grad_enabled() and any(t.requires_grad for t in ws)))
             if fits and ctas == 0 and self._direct:
                 outs = [torch.empty(M, N, dtype=t.dtype, device=t.device) for t in xs]

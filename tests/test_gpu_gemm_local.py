@@ -67,14 +67,19 @@ def test_gather_linear(world, rows, K, N, dtype):
 
 
 def test_what_the_kernel_does_not_take_still_runs():
-    """Below 4096 rows an all-gather followed by the framework's matmul took any N and K, unaligned rows and a weight that
-    wants a gradient; it still does."""
+    """Below 4096 rows an all-gather followed by the framework's matmul took any N and K, unaligned rows, weights of
+    uneven heights, a vector, and a weight that wants a gradient; it still does."""
     g = torch.Generator(device="cuda").manual_seed(0)
     with Communicator.virtual(2, 0, staging_bytes=32 << 20) as comm:
         for K, N, off in ((128, 40, 0), (36, 64, 0), (128, 64, 1)):
             flat = [_rand(g, torch.float16, 8 * K + 8) for _ in range(2)]
             xs = [f[off:off + 8 * K].view(8, K) for f in flat]
             ws = [_rand(g, torch.float16, N, K, scale=0.02) for _ in range(2)]
+            for o, w in zip(comm.allgather_linear(xs, ws), ws):
+                torch.testing.assert_close(o.double(), torch.cat(xs).double() @ w.double().t(), atol=2e-3, rtol=2e-3)
+        xs = [_rand(g, torch.float16, 8, 128) for _ in range(2)]
+        for shapes in (((64, 128), (128, 128)), ((128,), (128,))):  # uneven heights, a vector
+            ws = [_rand(g, torch.float16, *s, scale=0.02) for s in shapes]
             for o, w in zip(comm.allgather_linear(xs, ws), ws):
                 torch.testing.assert_close(o.double(), torch.cat(xs).double() @ w.double().t(), atol=2e-3, rtol=2e-3)
         ws = [w.detach().requires_grad_() for w in (_rand(g, torch.float16, 64, 128), _rand(g, torch.float16, 64, 128))]

@@ -432,6 +432,19 @@ std::vector<int64_t> fused_ag_gemm(std::vector<at::Tensor> xs, std::vector<at::T
   return info_vec(info);
 }
 
+// Replaces operands that overlap an output by copies of them.  A residual may lie exactly where its own rank's result goes.
+void keep_apart(std::vector<at::Tensor>& ts, const std::vector<at::Tensor>& outs, bool in_place_ok) {
+  for (size_t i = 0; i < ts.size(); ++i) {
+    const char* a = static_cast<const char*>(ts[i].data_ptr());
+    for (size_t j = 0; j < outs.size(); ++j) {
+      const char* b = static_cast<const char*>(outs[j].data_ptr());
+      if (a + ts[i].nbytes() <= b || b + outs[j].nbytes() <= a || (in_place_ok && i == j && a == b)) continue;
+      ts[i] = ts[i].clone();
+      break;
+    }
+  }
+}
+
 // The same two layers with every rank in this process (a world of one or an emulated one): no workspace, outputs anywhere.
 std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::Tensor> ws, std::vector<at::Tensor> residuals,
                                    std::vector<at::Tensor> gammas, std::vector<at::Tensor> outs, std::vector<at::Tensor> res_outs,
@@ -447,6 +460,14 @@ std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::T
   const int64_t M = xs[0].size(0), K = xs[0].size(1), N = ws[0].size(0);
   TORCH_CHECK(ws[0].size(1) == K, "b200ipc: weight must be [N, K] with the same K as x");
   check_epilogue_tensors(xs[0], residuals, gammas, outs, res_outs, M, N);
+  c10::cuda::CUDAGuard guard(c.device());
+  // A tile is stored while others still read x (the kernel with the exchange stores after the last of them), and an output of
+  // two calls ago, which may be x now, is where this call's goes.
+  for (const std::vector<at::Tensor>* o : {&outs, &res_outs}) {
+    keep_apart(xs, *o, false);
+    keep_apart(ws, *o, false);
+    keep_apart(residuals, *o, true);
+  }
   std::vector<GemmArPtrs> p(size_t(c.nlocal()));
   for (int i = 0; i < c.nlocal(); ++i) {
     TORCH_CHECK(xs[i].sizes() == xs[0].sizes() && ws[i].sizes() == ws[0].sizes(), "b200ipc: shape mismatch between ranks");
@@ -458,7 +479,6 @@ std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::T
     p[size_t(i)].out = outs[i].data_ptr();
     p[size_t(i)].res_out = res_outs.empty() ? nullptr : res_outs[i].data_ptr();
   }
-  c10::cuda::CUDAGuard guard(c.device());
   return info_vec(local_gemm_allreduce(c, dtype_of(xs[0]), p.data(), M, N, K, float(eps), with_norm,
                                        at::cuda::getCurrentCUDAStream(c.device())));
 }

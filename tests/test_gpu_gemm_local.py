@@ -202,3 +202,32 @@ def test_operands_of_the_epilogue_are_checked(fused):
         torch.cuda.synchronize()
         comm.check()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("world,M", [(1, 16), (1, 300), (2, 16), (2, 300)])
+def test_inputs_that_lie_where_the_outputs_go(world, M):
+    """Outputs take turns on two sets of buffers.  A result that is used twice is the second time an input at the place that the
+    call writes; so is a residual of which every rank holds one rank's copy."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    N = 1024
+    ws = [[_rand(g, torch.float16, N, N, scale=0.02) for _ in range(world)] for _ in range(3)]
+    with Communicator.virtual(world, 0, staging_bytes=64 << 20) as comm:
+        a = comm.linear_allreduce([_rand(g, torch.float16, M, N) for _ in range(world)], ws[0])
+        was = [t.clone() for t in a]
+        comm.linear_allreduce(a, ws[1])
+        c = comm.linear_allreduce(a, ws[2])
+        assert c[0].data_ptr() == a[0].data_ptr()
+        want = sum(t.double() @ w.double().t() for t, w in zip(was, ws[2]))
+        for o in c:
+            _close(o, want, torch.float16)
+        xs = [_rand(g, torch.float16, M, N) for _ in range(world)]
+        r = comm.linear_allreduce(xs, ws[0], [was[0]] * world)[1]
+        r0 = r[0].clone()
+        comm.linear_allreduce(xs, ws[1], r)
+        s = comm.linear_allreduce(xs, ws[2], [r[0]] * world)[1]
+        assert s[0].data_ptr() == r[0].data_ptr()
+        want = sum(t.double() @ w.double().t() for t, w in zip(xs, ws[2])) + r0.double()
+        for o in s:
+            _close(o, want, torch.float16)
+        torch.cuda.synchronize()
+        comm.check()

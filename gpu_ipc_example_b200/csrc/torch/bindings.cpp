@@ -565,11 +565,13 @@ at::Tensor rope_decode_attention_op(at::Tensor qkv, at::Tensor kcache, at::Tenso
   return out;
 }
 
-// RMSNorm(x) * gamma for [rows, hidden]
+// RMSNorm(x) * gamma for [rows, hidden], hidden a multiple of 8; operands that are strided or not 16-byte aligned are copied.
 at::Tensor rmsnorm_op(at::Tensor x, at::Tensor gamma, double eps) {
-  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && gamma.is_contiguous() && x.dim() == 2 && gamma.numel() == x.size(1) && x.size(1) % 8 == 0 &&
-                  gamma.scalar_type() == x.scalar_type() && fits_kernels(x) && fits_kernels(gamma),
-              "b200ipc: rmsnorm takes contiguous, 16-byte aligned [rows, hidden] tensors, hidden a multiple of 8");
+  TORCH_CHECK(x.is_cuda() && gamma.device() == x.device() && x.dim() == 2 && gamma.numel() == x.size(1) && x.size(1) % 8 == 0 &&
+                  gamma.scalar_type() == x.scalar_type(),
+              "b200ipc: rmsnorm takes [rows, hidden] and gamma [hidden] of one type on one device, hidden a multiple of 8");
+  x = aligned(x);
+  gamma = aligned(gamma);
   at::Tensor out = at::empty_like(x);
   c10::cuda::CUDAGuard guard(x.device());
   add_rmsnorm(dtype_of(x), x.data_ptr(), nullptr, gamma.data_ptr(), out.data_ptr(), nullptr, x.size(0), int(x.size(1)), float(eps),

@@ -66,3 +66,17 @@ def test_rmsnorm(rows, hidden, dtype):
     want = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * gam.double()
     u = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8  # one rounding
     torch.testing.assert_close(torch.ops.b200ipc.rmsnorm(x, gam, 1e-5).double(), want, atol=1e-6, rtol=1.01 * u)
+
+
+def test_rmsnorm_of_strided_and_unaligned_operands():
+    load()
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x, gam = torch.randn(5, 64, device="cuda", generator=g).half(), torch.randn(64, device="cuda", generator=g).half()
+    want = torch.ops.b200ipc.rmsnorm(x, gam, 1e-5)
+    shifted = torch.zeros(72, device="cuda").half()
+    shifted[1:65] = gam
+    spread = torch.zeros(64, 2, device="cuda").half()
+    spread[:, 1] = gam
+    for ga in (shifted[1:65], spread[:, 1]):
+        assert torch.equal(torch.ops.b200ipc.rmsnorm(x, ga, 1e-5), want)
+        assert torch.equal(torch.ops.b200ipc.rmsnorm(x.t().contiguous().t(), ga, 1e-5), want)

@@ -99,12 +99,14 @@ def test_add_rmsnorm(dtype, hidden):
     torch.testing.assert_close(out.float(), s * torch.rsqrt(s.pow(2).mean(-1, keepdim=True) + 1e-5) * gam.float(), **tol)
 
 
-def test_allreduce_residual_rmsnorm_prefill_sized():
-    """Above the one-shot limit the call becomes an all-reduce plus one fused add + RMSNorm kernel; same result."""
+@pytest.mark.parametrize("max_ctas", [0, 148])
+def test_allreduce_residual_rmsnorm_prefill_sized(max_ctas):
+    """Above the one-shot limit the call becomes an all-reduce plus one fused add + RMSNorm kernel; same result.  That is the
+    route of one process per GPU, and of an emulated world with a limit on CTAs; without one that takes one kernel."""
     from gpu_ipc_example_b200 import Communicator
 
     world, rows, hidden = 4, 512, 2048  # 2 MiB per rank
-    with Communicator.virtual(world, 0, staging_bytes=64 << 20) as comm:
+    with Communicator.virtual(world, 0, staging_bytes=64 << 20, max_ctas=max_ctas) as comm:
         g = torch.Generator(device="cuda").manual_seed(5)
         parts = [torch.randn(rows, hidden, device="cuda", generator=g).half() for _ in range(world)]
         keep = [p.clone() for p in parts]

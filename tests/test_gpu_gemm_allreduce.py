@@ -1,6 +1,7 @@
 """The tcgen05/TMA row-parallel GEMM fused with its all-reduce (and residual + RMSNorm), against a
-plain PyTorch fp32 reference.  World sizes above one are emulated on the single GPU (one cooperative
-launch, block rows are ranks), which exercises the peer stores, flags and the delivery counter."""
+plain PyTorch fp32 reference.  World sizes above one are emulated on the single GPU.  fused=True is the kernel that one process
+per GPU runs (one cooperative launch, block rows are ranks), which exercises the peer stores, flags and the delivery
+counter; fused=None is what a process that drives every rank takes, the GEMM without an exchange."""
 import pytest
 import torch
 
@@ -24,12 +25,19 @@ def _ref(xs, ws):
     return torch.stack([(x.float() @ w.float().t()).to(dtype).float() for x, w in zip(xs, ws)]).sum(0)
 
 
+def _check_kernel(comm, fused):
+    # the kernels with the exchange are 12 warps, the one without 10
+    assert comm.last_info.warps == (12 if fused else 10)
+
+
+@pytest.mark.parametrize("fused", [None, True])
 @pytest.mark.parametrize("world", [1, 2, 4, 8])
-def test_gemm_allreduce_plain(world):
+def test_gemm_allreduce_plain(world, fused):
     with Communicator.virtual(world, 0, staging_bytes=96 << 20) as comm:
         for (M, K, N) in ((128, 256, 256), (1, 512, 1024), (16, 448, 512), (300, 512, 1024), (2048, 448, 1024)):
             xs, ws, _, _ = _mk(world, M, K, N, torch.float16, seed=M)
-            outs = comm.linear_allreduce(xs, ws)
+            outs = comm.linear_allreduce(xs, ws, fused=fused)
+            _check_kernel(comm, fused)
             torch.cuda.synchronize()
             comm.check()
             want = _ref(xs, ws)
@@ -67,19 +75,23 @@ def test_every_split_of_k_has_work(M, K, N):
     with Communicator.virtual(1, 0, staging_bytes=64 << 20) as comm:
         for rep in range(2):
             xs, ws, _, _ = _mk(1, M, K, N, torch.float16, seed=rep)
-            outs = comm.linear_allreduce(xs, ws)
-            torch.cuda.synchronize()
-            comm.check()
-            torch.testing.assert_close(outs[0].float(), xs[0].float() @ ws[0].float().t(), atol=4e-3, rtol=2e-3)
+            want = xs[0].float() @ ws[0].float().t()
+            for outs in (comm.linear_allreduce(xs, ws, fused=True), comm.linear(xs, ws)):
+                assert comm.last_info.sched == "oneshot" and comm.last_info.warps == 12
+                torch.cuda.synchronize()
+                comm.check()
+                torch.testing.assert_close(outs[0].float(), want, atol=4e-3, rtol=2e-3)
 
 
-@pytest.mark.parametrize("world", [1, 8])
+@pytest.mark.parametrize("fused", [None, True])
+@pytest.mark.parametrize("world", [1, 4, 8])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_gemm_allreduce_residual_rmsnorm(world, dtype):
+def test_gemm_allreduce_residual_rmsnorm(world, dtype, fused):
     with Communicator.virtual(world, 0, staging_bytes=96 << 20) as comm:
         for (M, K, N) in ((1, 448, 8192), (16, 448, 8192), (128, 448, 8192), (200, 256, 1024)):
             xs, ws, res, gam = _mk(world, M, K, N, dtype, seed=7 + M)
-            out, new_res = comm.linear_allreduce(xs, ws, [res] * world, [gam] * world, 1e-5)
+            out, new_res = comm.linear_allreduce(xs, ws, [res] * world, [gam] * world, 1e-5, fused=fused)
+            _check_kernel(comm, fused)
             torch.cuda.synchronize()
             comm.check()
             s = (_ref(xs, ws) + res.float()).to(dtype).float()
@@ -90,24 +102,28 @@ def test_gemm_allreduce_residual_rmsnorm(world, dtype):
                 torch.testing.assert_close(o.float(), want, **tol)
 
 
-def test_repeated_calls_reuse_the_workspace():
+@pytest.mark.parametrize("fused", [None, True])
+def test_repeated_calls_reuse_the_workspace(fused):
     with Communicator.virtual(4, 0, staging_bytes=64 << 20) as comm:
         for it in range(6):
             xs, ws, res, gam = _mk(4, 64, 256, 512, torch.float16, seed=it)
-            out, new_res = comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4)
+            out, new_res = comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4, fused=fused)
+            _check_kernel(comm, fused)
             torch.cuda.synchronize()
             comm.check()
             s = (_ref(xs, ws) + res.float()).half().float()
             torch.testing.assert_close(new_res[3].float(), s, atol=4e-2, rtol=2e-2)
 
 
-def test_result_of_one_call_is_the_residual_of_the_next():
+@pytest.mark.parametrize("fused", [None, True])
+def test_result_of_one_call_is_the_residual_of_the_next(fused):
     """Calls of one shape alternate between two sets of output buffers: a decoder chains them without copies."""
     with Communicator.virtual(2, 0, staging_bytes=64 << 20) as comm:
         xs, ws, res, gam = _mk(2, 16, 256, 512, torch.float16, seed=11)
-        _, r1 = comm.linear_allreduce(xs, ws, [res] * 2, [gam] * 2)
-        _, r2 = comm.linear_allreduce(xs, ws, r1, [gam] * 2)
-        out3, r3 = comm.linear_allreduce(xs, ws, r2, [gam] * 2)
+        _, r1 = comm.linear_allreduce(xs, ws, [res] * 2, [gam] * 2, fused=fused)
+        _, r2 = comm.linear_allreduce(xs, ws, r1, [gam] * 2, fused=fused)
+        out3, r3 = comm.linear_allreduce(xs, ws, r2, [gam] * 2, fused=fused)
+        _check_kernel(comm, fused)
         torch.cuda.synchronize()
         comm.check()
         assert r1[0].data_ptr() != r2[0].data_ptr() and r1[0].data_ptr() == r3[0].data_ptr()
@@ -121,18 +137,20 @@ def test_result_of_one_call_is_the_residual_of_the_next():
         torch.testing.assert_close(out3[0].float(), want, atol=6e-2, rtol=2e-2)
 
 
-def test_graph_replay_with_device_side_counters():
+@pytest.mark.parametrize("M,fused", [(32, None), (32, True), (64, True)])
+def test_graph_replay_with_device_side_counters(M, fused):
     with Communicator.virtual(4, 0, staging_bytes=64 << 20, device_seq=True) as comm:
-        xs, ws, res, gam = _mk(4, 32, 256, 512, torch.float16, seed=3)
+        xs, ws, res, gam = _mk(4, M, 256, 512, torch.float16, seed=3)
         s = (_ref(xs, ws) + res.float()).half().float()
         stream = torch.cuda.Stream()
         with torch.cuda.stream(stream):
-            comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4)  # allocates the workspace outside the capture
+            comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4, fused=fused)  # allocates the workspace outside the capture
+            _check_kernel(comm, fused)
             stream.synchronize()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=stream):
-                out, new_res = comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4)
-                out, new_res = comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4)
+                out, new_res = comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4, fused=fused)
+                out, new_res = comm.linear_allreduce(xs, ws, [res] * 4, [gam] * 4, fused=fused)
             for _ in range(3):
                 for t in new_res:
                     t.zero_()

@@ -8,9 +8,10 @@ from gpu_ipc_example_b200.parallel import ColumnParallelLinear, RowParallelLinea
 pytestmark = pytest.mark.gpu
 
 
-def test_row_and_column_parallel_layers():
+@pytest.mark.parametrize("max_ctas", [0, 148])  # a limit on CTAs: the kernels with the exchange
+def test_row_and_column_parallel_layers(max_ctas):
     world, M, K, N = 4, 64, 512, 512
-    with Communicator.virtual(world, 0, staging_bytes=64 << 20) as comm:
+    with Communicator.virtual(world, 0, staging_bytes=64 << 20, max_ctas=max_ctas) as comm:
         g = torch.Generator(device="cuda").manual_seed(0)
         x = torch.randn(M, K, device="cuda", generator=g).half()
         w = (torch.randn(N, K, device="cuda", generator=g) * 0.03).half()
@@ -58,11 +59,12 @@ def test_functional_api_with_a_world_of_one():
         ops.shutdown()
 
 
-def test_functional_api_on_an_emulated_world_of_four():
+@pytest.mark.parametrize("max_ctas", [0, 148])
+def test_functional_api_on_an_emulated_world_of_four(max_ctas):
     """The torch.distributed-shaped functions with real exchanges behind them: every argument is a list with
     one tensor per emulated rank."""
     world = 4
-    comm = Communicator.virtual(world, 0, staging_bytes=32 << 20)
+    comm = Communicator.virtual(world, 0, staging_bytes=32 << 20, max_ctas=max_ctas)
     ops.init(comm)
     try:
         g = torch.Generator(device="cuda").manual_seed(4)

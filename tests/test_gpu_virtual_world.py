@@ -260,14 +260,18 @@ def test_auto_picks_by_size(comm):
     comm.set_thresholds(0, 0)
 
 
-def test_fused_allreduce_residual_rmsnorm(comm):
+@pytest.mark.parametrize("ctas", [0, 8])
+def test_fused_allreduce_residual_rmsnorm(comm, ctas):
+    """A given number of CTAs asks for the kernel with the exchange; without one these worlds take the kernel without."""
     for rows, hidden in ((1, 8192), (4, 8192), (32, 8192), (16, 1024), (3, 4104)):
         xs = [t.view(rows, hidden) for t in _inputs(comm.world, rows * hidden, torch.float16, seed=3)]
         res = [torch.randn(rows, hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(11)).half()
                for _ in range(comm.world)]
         gam = [torch.rand(hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(12)).half() + 0.5
                for _ in range(comm.world)]
-        outs, new_res = comm.allreduce_residual_rmsnorm(xs, res, gam, 1e-5)
+        outs, new_res = comm.allreduce_residual_rmsnorm(xs, res, gam, 1e-5, ctas=ctas)
+        if 2 * rows * hidden <= comm.fused_oneshot_max_bytes:  # above: an all-reduce and a kernel behind it
+            assert comm.last_info.sched == ("oneshot" if ctas else "bulk")
         torch.cuda.synchronize()
         comm.check()
         s = torch.stack([x.float() for x in xs]).sum(0) + res[0].float()

@@ -7,9 +7,9 @@
 
 For N > 1 run it under `python -m torch.distributed.run --nproc-per-node N ... bench.py --gpus N ...`
 (one rank per GPU); when started without a launcher's environment it re-launches itself that way.
-With N = 1 there is no peer, so the world is emulated: 8 ranks on the one GPU, one cooperative
-launch per all-reduce, "peer" traffic through L2/HBM instead of NVLink - the same kernels and
-protocol, a different wire.  That is stated in `config.parallelism`.
+With N = 1 there is no peer, so the world is emulated: 8 ranks on the one GPU, one launch per all-reduce.  `auto` takes a
+kernel there that reads and writes every rank's buffer through L2/HBM: no rank waits for another, and the number says
+nothing about N > 1 (`--algo bulk` times the kernel with the exchange).  That is stated in `config.parallelism`.
 
 A step is one all-reduce of the reference's default problem: 8 Mi fp16 elements (16 MiB) per rank
 (`-n 8MB`, main.cpp:179, 45).  Rank 0 prints one JSON line; `value` is the NCCL-convention bus
@@ -441,7 +441,8 @@ def run(args, json_out, state):
                 "global_batch": emu_world,
                 "seq_len": n,
                 "parallelism": (f"{world} GPUs, one rank per GPU over NVLink" if multi
-                                else f"{emu_world} ranks emulated on 1 GPU (one launch; peer traffic stays in L2/HBM, no NVLink)"),
+                                else f"{emu_world} ranks emulated on 1 GPU (one launch over all ranks' buffers in L2/HBM; no NVLink"
+                                + ("; no exchange between ranks is measured)" if args.algo == "auto" else ")")),
                 "algo": f"{args.algo} -> {headline_algo}",
                 "buffers": f"{nbuf} rotating buffers = {nbuf * nbytes >> 20} MiB > 126 MiB L2, in place, symmetric heap (no staging copy)",
                 "busbw": "bytes/time*2(n-1)/n, device time by CUDA events, max over ranks",

@@ -97,7 +97,7 @@ void usage() {
       "  -o, --out-of-place  write to a separate output buffer\n"
       "      --iters K       timed launches (default 1)\n"
       "      --np N          fork N ranks from this process\n"
-      "      --virtual N     emulate N ranks on one GPU (one cooperative launch)\n"
+      "      --virtual N     emulate N ranks on one GPU (auto then exchanges nothing)\n"
       "      --nvls          set up the NVSwitch multicast mapping\n"
       "      --ref-accum     round to the element type after every add, like the reference\n"
       "      --random        N(0,1) / U(-1,1) data instead of the (i%%32)*(rank+1) pattern\n"

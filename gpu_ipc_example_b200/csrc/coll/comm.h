@@ -4,8 +4,9 @@
 //
 // A communicator drives either ONE rank of a multi-process world (one process
 // per GPU; peers mapped through the heap) or ALL ranks of a "virtual world" on a
-// single GPU (one cooperative launch whose block rows are the ranks) - the
-// second form exists so that every protocol can be exercised on one GPU.
+// single GPU (one launch whose block rows are the ranks, cooperative where they
+// wait on one another) - the second form exists so that every protocol can be
+// exercised on one GPU; what `auto` picks there exchanges nothing.
 //
 // Capability parity: launch geometry and sequence-number advance
 // (allreduce.hpp:37-74, 238-269; allgather.hpp:31-70), the -a name table
@@ -106,7 +107,7 @@ class Comm {
 
   // Size -> algorithm choice used for AlgoSpec::automatic: the measured table of tuner.h unless
   // set_thresholds() installed explicit cut-offs (0, 0 restores the table).
-  // `direct`: an emulated world whose buffers the barrier-based kernel can use as they are.
+  // `direct`: an emulated world whose buffers the large-message kernel is to use as they are (auto_direct).
   AlgoSpec choose_all_reduce(size_t bytes, bool symmetric, bool direct = false) const;
   void set_thresholds(size_t oneshot_max_bytes, size_t ll_max_bytes) {
     oneshot_max_bytes_ = oneshot_max_bytes;
@@ -154,7 +155,7 @@ class Comm {
   int resident_ctas(KernelFn fn, int threads, size_t smem);
   uint32_t take_seq(uint32_t advance);
   uint32_t take_barrier();
-  // Launch with caller-built parameters (cooperative when this communicator drives several ranks).
+  // Launch with caller-built parameters (cooperative when this communicator drives several ranks that meet).
   // pdl: the kernel executes griddepcontrol.wait before it touches anything an earlier kernel wrote, so it may be
   // launched with programmatic stream serialisation (single-rank launches only; see common/pdl.h)
   // meet: block rows (emulated ranks) wait on one another inside the kernel, so that all have to be resident.

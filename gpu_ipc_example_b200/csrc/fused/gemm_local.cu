@@ -62,7 +62,8 @@ int resident_clusters(const void* fn, int device, int splits) {
 // Microseconds that a plan takes apart from what all plans share (launch, first loads).  Fitted to one B200: a k block of a
 // pair 0.08 + 0.0012 BN (K = 8192, M = 2048, N = 7168: BN = 160 166 us, 224 170, 256 197, 128 197); the epilogue of a
 // tile 0.5 + 0.0133 BN, hidden behind the next tile's MMAs where there is one; handing partial sums between the pairs of a
-// cluster 1.4 + 0.006 BN (K = 1024, M = 16, N = 8192: one split 15.4 us, two 17.4; K = 3584: 18.6 and 14.5 back to back).
+// cluster 1.4 + 0.006 BN (K = 1024, M = 16, N = 8192: one split 15.4 us, two 17.4; K = 3584: 18.6 and 14.5 back to back; both
+// taken with the first W loads ahead of the wait for the kernel in front, 15.5 with a prefetch to L2 there).
 double plan_cost(int64_t tiles, int64_t room, int64_t kb_total, int bn, int splits) {
   const double waves = double(ceil_div64(tiles, room));
   const double main = double(ceil_div64(kb_total, splits)) * (0.08 + 0.0012 * bn);

@@ -7,17 +7,16 @@ Per layer there are exactly two all-reduces (after the attention output projecti
 down projection); each is fused with the residual add and the RMSNorm that follows it, in one of
 three ways (`fusion=`):
 
-  "gemm"       the row-parallel projection itself is part of the kernel: tcgen05/TMA GEMM whose
-               epilogue reduce-scatters into the peers, owner reduce + residual + RMSNorm, all-gather
-               (`Communicator.linear_allreduce`)
-  "allreduce"  cuBLAS projection, then one one-shot all-reduce + residual + RMSNorm kernel
-               (`Communicator.allreduce_residual_rmsnorm`)
+  "gemm"       the row-parallel projection itself is part of the kernel (`Communicator.linear_allreduce`): on several GPUs a
+               tcgen05/TMA GEMM with the exchange, residual and RMSNorm in it; where one process drives every rank, a
+               GEMM over all ranks' K with the residual in its epilogue, and a norm kernel behind it
+  "allreduce"  cuBLAS projection, then one all-reduce + residual + RMSNorm kernel (`Communicator.allreduce_residual_rmsnorm`)
   "nccl"       the baseline: cuBLAS projection, `torch.distributed.all_reduce`, separate add and norm
 
-What lies between the GEMMs and the collectives runs in three hand-written kernels when the head
-dimension is 128 (`kernels=True`, the default there): rotary embedding fused with the KV-cache append and
-attention of the new token over the cache (grouped-query, split over the context), SiLU(gate) * up; the first norm
-and the arg-max over the logits are one kernel each.
+What lies between the GEMMs and the collectives runs in two hand-written kernels per layer when the head
+dimension is 128 (`kernels=True`, the default there): rotary embedding, KV-cache append and attention of the new token
+over the cache (grouped-query, split over the context) in one, SiLU(gate) * up in the other; the first norm and the
+arg-max over the logits are one kernel each.
 With `kernels=False` the same steps are plain PyTorch ops (the reference path of the tests).
 
 The reference has no model code; its smoke script all-reduces decode-sized fp16 activations the way a

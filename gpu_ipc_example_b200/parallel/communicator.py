@@ -116,7 +116,12 @@ class Communicator:
     @classmethod
     def virtual(cls, world: int, device: int = 0, *, staging_bytes: int = 64 << 20, timeout_ms: int = 2000,
                 device_seq: bool = False, first_seq: int = 1, max_ctas: int = 0) -> "Communicator":
-        """All `world` ranks emulated on one GPU (one cooperative launch per collective)."""
+        """All `world` ranks emulated on one GPU, one launch per collective.
+
+        Nothing has to be exchanged there: `auto`, `allreduce_residual_rmsnorm`, `linear_allreduce` and `allgather_linear`
+        take kernels that read and write every rank's tensors directly.  The kernels that one process per GPU runs (one
+        cooperative launch whose block rows are the ranks) run for an algorithm by name, a call with `flags`, `ctas=` of the norm, `fused=True`,
+        a packed weight, and on communicators with `max_ctas`."""
         C = load()
         h = C.comm_create_virtual(world, device, staging_bytes, timeout_ms, device_seq, first_seq, max_ctas)
         comm = cls(h, True)
@@ -247,8 +252,12 @@ class Communicator:
         """Re-lays a row-parallel weight [N, K] (nn.Linear layout, N a multiple of 64) for `linear_allreduce`:
         [N / 64, K blocks, 64, 64], every 64 x 64 block stored as the 128-byte-swizzled shared-memory image the
         tensor core reads (16-byte chunk c of row r sits at chunk c ^ (r % 8)), K zero-padded to a multiple of
-        256.  Done once at load time; the kernel then streams the weight with one contiguous bulk copy per
-        stage, which is worth most at decode sizes where the layer is bound by reading the weight."""
+        256.  Done once at load time; the kernel with the exchange then streams the weight with one contiguous bulk copy
+        per stage, which is worth most at decode sizes where the layer is bound by reading the weight.
+
+        For one process per GPU.  Where one process drives every rank, plain weights take the GEMM without an exchange, which does
+        not know this layout and is ahead (K = 3584, N = 8192 with norm, 16 rows 17.3 us against 19.2 packed, 64 rows 19.4
+        against 30.0)."""
         N, K = weight.shape
         if N % 64:
             raise ValueError("pack_weight needs N to be a multiple of 64")
@@ -264,7 +273,7 @@ class Communicator:
     def linear_allreduce(self, x: TensorOrList, weight: TensorOrList, residual: Optional[TensorOrList] = None,
                          gamma: Optional[TensorOrList] = None, eps: float = 1e-5, *, ctas: int = 0,
                          fused: Optional[bool] = None):
-        """Row-parallel linear layer fused with its all-reduce in one tcgen05/TMA kernel.
+        """Row-parallel linear layer fused with its all-reduce on tcgen05/TMA kernels.
 
         fused=None picks: where this communicator drives every rank (a world of one, an emulated world) nothing has
         to be exchanged, so plain weights take ONE GEMM over the ranks' concatenated K (fp32 sum, one rounding) and a
@@ -274,11 +283,11 @@ class Communicator:
         or an explicit `ctas`, takes the kernel with the exchange.
 
         x: [M, K_local], weight: [N, K_local] (nn.Linear layout) of this rank, or that weight packed once by
-        `pack_weight` (faster, most of all at decode sizes).  Returns
+        `pack_weight` (for one process per GPU).  Returns
         `y = all_reduce(x @ weight.T)` when neither residual nor gamma is given, else the pair
         `(RMSNorm(y + residual) * gamma, y + residual)`.  Outputs live in the symmetric heap; calls of one shape
         alternate between two sets of them, so a result stays valid through the next call of that shape (it may
-        be that call's residual) and is overwritten by the one after."""
+        be that call's residual) and is overwritten by the one after (which may still have it as an input)."""
         xs = [t.contiguous() for t in self._lists(x)]
         ws = [t.contiguous() for t in self._lists(weight)]
         M, N = xs[0].shape[0], ws[0].shape[0] * (64 if ws[0].dim() == 4 else 1)  # 4-D: packed by pack_weight
@@ -348,7 +357,7 @@ class Communicator:
         return out
 
     def allgather_linear(self, x_shard: TensorOrList, weight: TensorOrList, *, ctas: int = 0, fused: Optional[bool] = None):
-        """Column-parallel linear layer on row-sharded activations, all-gather fused into the GEMM kernel.
+        """Column-parallel linear layer on row-sharded activations, the all-gather fused into the GEMM kernel where one pays.
 
         fused=None picks: where this communicator drives every rank (a world of one, an emulated world) the GEMM reads the
         shards where they are.  On several GPUs the fused kernel from 4096 gathered rows up (level with cuBLAS + NCCL at

@@ -1,9 +1,8 @@
 """Tensor-parallel linear layers on top of the fused kernels (inference; no autograd).
 
 `RowParallelLinear` holds a K-slice of the weight and returns the all-reduced product, optionally with
-the residual add and RMSNorm that follow it in a decoder block, from one kernel.  `ColumnParallelLinear`
-holds an N-slice; with `gather_input=True` its input is row-sharded and the all-gather is fused into
-the GEMM.  Both work on one rank per process or on all ranks of an emulated world (lists of tensors).
+the residual add and RMSNorm that follow it in a decoder block, from one call.  `ColumnParallelLinear`
+holds an N-slice; with `gather_input=True` its input is row-sharded (`Communicator.allgather_linear`).  Both work on one rank per process or on all ranks of an emulated world (lists of tensors).
 """
 from __future__ import annotations
 
@@ -17,8 +16,9 @@ from .communicator import Communicator
 class RowParallelLinear:
     def __init__(self, comm: Communicator, weight, fused: str = "gemm"):
         """weight: [N, K_local] (nn.Linear layout) or a list with one such tensor per local rank.
-        fused: "gemm" = tcgen05 GEMM + reduce-scatter epilogue kernel; "allreduce" = library GEMM followed by
-        the one-shot all-reduce (+ residual + RMSNorm) kernel."""
+        fused: "gemm" = `Communicator.linear_allreduce` (tcgen05 GEMM with the collective in its kernel, or without an
+        exchange where one process drives every rank); "allreduce" = library GEMM followed by the all-reduce (+ residual +
+        RMSNorm) call."""
         assert fused in ("gemm", "allreduce")
         self.comm, self.weight, self.fused = comm, weight, fused
 
@@ -39,7 +39,7 @@ class RowParallelLinear:
 class ColumnParallelLinear:
     def __init__(self, comm: Communicator, weight, gather_input: bool = False):
         """weight: [N_local, K] or a list of those.  gather_input: the input arrives row-sharded
-        ([M / world, K] per rank) and is all-gathered inside the GEMM kernel."""
+        ([M / world, K] per rank) and goes through `Communicator.allgather_linear`."""
         self.comm, self.weight, self.gather_input = comm, weight, gather_input
 
     def __call__(self, x):

@@ -115,6 +115,7 @@ def ninja_text(with_torch: bool = True) -> str:
     core_objs.append(cu("fused/gemm_ar.cu"))
     core_objs.append(cu("fused/gemm_local.cu"))
     core_objs.append(cu("model/decode_ops.cu"))
+    core_objs.append(cu("model/decode_step.cu"))
 
     lib = f"{PKG}/libb200ipc.so"
     w(f"build {lib}: link_so {' '.join(core_objs)}")
@@ -169,7 +170,7 @@ def build(with_torch: bool = True, verbose: bool = False, jobs: int | None = Non
 def cuda_units():
     """(source, extra flags) of every CUDA translation unit of the library."""
     units = [("coll/ll_inst.cu", f"-DB200_LL_OP={op} -DB200_LL_T={ty}") for op in LL_OPS for ty in LL_TYPES.values()]
-    units += [(src, "") for src in ("coll/bulk_inst.cu", "fused/fused_ops.cu", "fused/gemm_ar.cu", "fused/gemm_local.cu", "model/decode_ops.cu",
+    units += [(src, "") for src in ("coll/bulk_inst.cu", "fused/fused_ops.cu", "fused/gemm_ar.cu", "fused/gemm_local.cu", "model/decode_ops.cu", "model/decode_step.cu",
                                     "capi/no_alloc.cu")]
     return units
 

@@ -9,29 +9,12 @@
 // activations of a tensor-parallel LLM (script/gpu_inference_test.py:29-45).
 #include "decode_ops.h"
 
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include "../common/check.h"
 #include "../common/pdl.h"
+#include "decode_math.cuh"
 
 namespace b200ipc {
 namespace {
-
-template <typename T>
-struct Num;
-template <>
-struct Num<__half> {
-  using T2 = __half2;
-  __device__ static float2 up(T2 v) { return __half22float2(v); }
-  __device__ static T2 down(float a, float b) { return __floats2half2_rn(a, b); }
-};
-template <>
-struct Num<__nv_bfloat16> {
-  using T2 = __nv_bfloat162;
-  __device__ static float2 up(T2 v) { return __bfloat1622float2(v); }
-  __device__ static T2 down(float a, float b) { return __floats2bfloat162_rn(a, b); }
-};
 
 // Every kernel of this file starts with pdl_launch_dependents() + pdl_wait() and is launched with programmatic
 // stream serialisation: its CTAs can be resident before the previous kernel of the step has drained.
@@ -48,11 +31,6 @@ void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t s
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1u : 0u;
   B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
-}
-
-// Pair (x1, x2) turned by an angle.  Spelled out so that every kernel that rotates gives the same bits.
-__device__ __forceinline__ float2 rope_pair(float x1, float x2, float sn, float cs) {
-  return make_float2(fmaf(x1, cs, -__fmul_rn(x2, sn)), fmaf(x2, cs, __fmul_rn(x1, sn)));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -115,34 +93,9 @@ __global__ void rope_kv_append_kernel(T* qkv, T* kcache, T* vcache, int hq, int 
 // Warps merge in shared memory, splits through a workspace; the last CTA of a (batch, KV head)
 // to arrive writes the result.
 // ---------------------------------------------------------------------------------------------
-constexpr int kAttnD = 128;
 constexpr int kAttnThreads = 128;
 constexpr int kAttnWarps = kAttnThreads / 32;
 constexpr int kAttnTile = 16;  // positions per warp step
-
-template <typename T>
-__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                          uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_16816<__half>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                                  uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-template <>
-__device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                                         uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-template <typename T>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  const typename Num<T>::T2 v = Num<T>::down(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 
 // 16 words of a 256-byte row: the 16-byte chunks c, c+4, c+8, c+12
 template <typename T>
@@ -439,15 +392,6 @@ __global__ void silu_mul_kernel(const T* gu, T* act, int64_t rows, int F) {
 // 16032 columns: 16 us before).
 // ---------------------------------------------------------------------------------------------
 constexpr int kArgmaxThreads = 512;
-struct Best {
-  float v;
-  int i;
-};
-__device__ __forceinline__ Best better(Best a, Best b) {
-  const bool na = a.v != a.v, nb = b.v != b.v;
-  const bool take_b = nb ? (!na || b.i < a.i) : (!na && (b.v > a.v || (b.v == a.v && b.i < a.i)));
-  return take_b ? b : a;
-}
 template <typename T>
 __global__ void __launch_bounds__(kArgmaxThreads) row_argmax_kernel(const T* x, float* values, int64_t* indices, int cols) {
   using T2 = typename Num<T>::T2;

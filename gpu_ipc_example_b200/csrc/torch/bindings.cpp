@@ -27,6 +27,7 @@
 #include "../common/check.h"
 #include "../fused/fused_ops.h"
 #include "../model/decode_ops.h"
+#include "../model/decode_step.h"
 
 namespace {
 
@@ -589,6 +590,71 @@ std::tuple<at::Tensor, at::Tensor> row_argmax_op(at::Tensor x) {
   return {v, i};
 }
 
+int64_t step_workspace_bytes(int64_t comm_id, int64_t batch, int64_t layers, int64_t hidden, int64_t hq, int64_t hkv, int64_t ffn, int64_t vocab,
+                             int64_t max_ctx) {
+  Comm& c = get(comm_id);
+  const DecodeStepShape s{int(batch), int(layers), int(hidden), int(hq), int(hkv), int(ffn), int(vocab), int(max_ctx)};
+  return decode_step_takes(c, s, 1) ? int64_t(decode_step_workspace_bytes(c, s)) : 0;
+}
+
+// One decode step as one kernel: [ids, hidden states of every rank], or nothing where that kernel does not take the call and
+// the general route has to.  h: the tokens' embeddings, overwritten; lists in [layer][rank] order.
+std::vector<at::Tensor> decode_step_op(at::Tensor h, const std::vector<at::Tensor>& wqkv, const std::vector<at::Tensor>& wo,
+                                       const std::vector<at::Tensor>& wgu, const std::vector<at::Tensor>& wdown,
+                                       const std::vector<at::Tensor>& kcache, const std::vector<at::Tensor>& vcache,
+                                       const std::vector<at::Tensor>& head, const std::vector<at::Tensor>& gamma_attn,
+                                       const std::vector<at::Tensor>& gamma_mlp, at::Tensor gamma_final, at::Tensor workspace, int64_t hq,
+                                       int64_t hkv, int64_t pos, double eps, double theta, int64_t comm_id) {
+  Comm& c = get(comm_id);
+  const size_t W = size_t(c.world()), L = gamma_mlp.size(), n = L * W;
+  if (h.dim() != 2 || L == 0 || gamma_attn.size() != L || head.size() != W || !(theta > 0)) return {};
+  for (const auto* list : {&wqkv, &wo, &wgu, &wdown, &kcache, &vcache})
+    if (list->size() != n) return {};
+  if (wgu[0].dim() != 2 || kcache[0].dim() != 4 || head[0].dim() != 2) return {};
+  const int64_t B = h.size(0), H = h.size(1), F = wgu[0].size(0) / 2, V = head[0].size(0), ctx = kcache[0].size(2), D = 128;
+  if (h.scalar_type() != at::kHalf && h.scalar_type() != at::kBFloat16) return {};
+  const DecodeStepShape s{int(B), int(L), int(H), int(hq), int(hkv), int(F), int(V), int(ctx)};
+  if (!decode_step_takes(c, s, int(pos))) return {};
+  auto takes = [&](const at::Tensor& t, at::IntArrayRef sizes) {
+    return t.is_cuda() && t.get_device() == c.device() && t.scalar_type() == h.scalar_type() && t.sizes() == sizes && fits_kernels(t);
+  };
+  if (!takes(h, {B, H}) || !takes(gamma_final, {H})) return {};
+  DecodeStepPtrs p;
+  for (size_t i = 0; i < n; ++i) {
+    if (!takes(wqkv[i], {(hq + 2 * hkv) * D, H}) || !takes(wo[i], {H, hq * D}) || !takes(wgu[i], {2 * F, H}) || !takes(wdown[i], {H, F}) ||
+        !takes(kcache[i], {B, hkv, ctx, D}) || !takes(vcache[i], {B, hkv, ctx, D}))
+      return {};
+    p.wqkv.push_back(wqkv[i].data_ptr());
+    p.wo.push_back(wo[i].data_ptr());
+    p.wgu.push_back(wgu[i].data_ptr());
+    p.wdown.push_back(wdown[i].data_ptr());
+    p.kcache.push_back(kcache[i].data_ptr());
+    p.vcache.push_back(vcache[i].data_ptr());
+  }
+  for (size_t l = 0; l < L; ++l) {
+    if (!takes(gamma_attn[l], {H}) || !takes(gamma_mlp[l], {H})) return {};
+    p.gamma_attn.push_back(gamma_attn[l].data_ptr());
+    p.gamma_mlp.push_back(gamma_mlp[l].data_ptr());
+  }
+  p.gamma_final = gamma_final.data_ptr();
+  p.h = h.data_ptr();
+  c10::cuda::CUDAGuard guard(c.device());
+  std::vector<at::Tensor> out{at::empty({B}, h.options().dtype(at::kLong))};
+  for (size_t r = 0; r < W; ++r) {
+    if (!takes(head[r], {V, H})) return {};
+    p.head.push_back(head[r].data_ptr());
+    out.push_back(at::empty({B, H}, h.options()));
+    p.hidden_out.push_back(out.back().data_ptr());
+  }
+  p.ids = out[0].data_ptr<int64_t>();
+  TORCH_CHECK(workspace.is_cuda() && workspace.get_device() == c.device() && workspace.is_contiguous() &&
+                  size_t(workspace.nbytes()) >= decode_step_workspace_bytes(c, s) && (reinterpret_cast<uintptr_t>(workspace.data_ptr()) & 255) == 0,
+              "b200ipc: decode step workspace too small or not 256-byte aligned");
+  p.workspace = workspace.data_ptr();
+  decode_step(c, dtype_of(h), s, p, int(pos), float(eps), float(theta), at::cuda::getCurrentCUDAStream(c.device()));
+  return out;
+}
+
 // (RMSNorm(x + residual) * gamma, x + residual) for [rows, hidden] tensors
 std::vector<at::Tensor> add_rmsnorm_op(at::Tensor x, at::Tensor residual, at::Tensor gamma, double eps) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && residual.is_contiguous() && gamma.is_contiguous() && x.dim() == 2 &&
@@ -646,6 +712,9 @@ TORCH_LIBRARY(b200ipc, m) {
         &decode_attention_op);
   m.def("rope_decode_attention(Tensor qkv, Tensor(a!) kcache, Tensor(b!) vcache, Tensor(c!) workspace, int hq, int hkv, int pos, "
         "int splits, float theta) -> Tensor", &rope_decode_attention_op);
+  m.def("decode_step(Tensor(a!) h, Tensor[] wqkv, Tensor[] wo, Tensor[] wgu, Tensor[] wdown, Tensor[] kcache, Tensor[] vcache, Tensor[] head, "
+        "Tensor[] gamma_attn, Tensor[] gamma_mlp, Tensor gamma_final, Tensor workspace, int hq, int hkv, int pos, float eps, float theta, "
+        "int comm) -> Tensor[]", &decode_step_op);
   m.def("rmsnorm(Tensor x, Tensor gamma, float eps) -> Tensor", &rmsnorm_op);
   m.def("row_argmax(Tensor x) -> (Tensor, Tensor)", &row_argmax_op);
   m.def("silu_mul(Tensor gate_up) -> Tensor", &silu_mul_op);
@@ -698,6 +767,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                 int64_t(l.staging_off),  int64_t(l.staging_bytes), int64_t(l.total_bytes)};
   });
   m.def("gemm_ar_workspace_bytes", &gemm_ar_workspace_bytes);
+  m.def("decode_step_workspace_bytes", &step_workspace_bytes);
   m.def("attention_splits", &attention_splits);
   m.def("attention_workspace_bytes", &attention_workspace_bytes);
   m.def("algo_names", &algo_names_help);

@@ -5,9 +5,15 @@
 // Capability parity: the reference's framework smoke test drives an all-reduce
 // of fp16 activations through a torch process group (script/gpu_inference_test.py:
 // 21-45); here the same call lands in this library's kernels.
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 #include <torch/library.h>
 
@@ -679,6 +685,214 @@ at::Tensor silu_mul_op(at::Tensor gate_up) {
   return act;
 }
 
+// ---- the list calls of Communicator, past the dispatcher -----------------------------------------------------------------
+// A small collective is bound by its call: through torch.ops the lists of an 8-rank world cost about 7 us before the launch,
+// as CPython calls 2.  A call comes this way only where nothing listens on the way there and its tensors are plain ones: no
+// mode or transform, no profiler, no subclass or wrapper.  Everything else, arguments that do not fit included, gives None,
+// and Communicator makes the call through the operator, which does what it always did.
+bool nothing_listens() {
+  const auto& tls = c10::impl::tls_local_dispatch_key_set();
+  return ((tls.included_ - c10::default_included_set).raw_repr() & ~c10::full_backend_mask) == 0 && !at::impl::torch_function_mode_enabled() &&
+         !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::hasCallbacks();
+}
+
+bool plain_list(PyObject* o, std::vector<at::Tensor>* ts) {
+  static const c10::DispatchKeySet plain =
+      c10::DispatchKeySet({c10::DispatchKey::Dense, c10::DispatchKey::AutogradFunctionality, c10::DispatchKey::ADInplaceOrView}) |
+      c10::autocast_dispatch_keyset;
+  if (!PyList_CheckExact(o)) return false;
+  const Py_ssize_t n = PyList_GET_SIZE(o);
+  ts->reserve(size_t(n));
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* item = PyList_GET_ITEM(o, i);
+    if (!THPVariable_CheckExact(item)) return false;
+    const at::Tensor& t = THPVariable_Unpack(item);
+    if (!t.defined() || !t.is_cuda() || ((t.key_set() - plain).raw_repr() & ~c10::full_backend_mask) != 0) return false;
+    ts->push_back(t);
+  }
+  return true;
+}
+
+// Arguments of a call, taken one after the other; `ok` is false once one was not what was asked for.
+struct FastArgs {
+  PyObject* const* args;
+  Py_ssize_t n, at = 0;
+  bool ok;
+  FastArgs(PyObject* const* a, Py_ssize_t count, Py_ssize_t want) : args(a), n(count), ok(count == want && nothing_listens()) {}
+  std::vector<at::Tensor> list() {
+    std::vector<at::Tensor> ts;
+    if (ok) ok = plain_list(args[at++], &ts);
+    return ts;
+  }
+  int64_t integer() {
+    if (!ok) return 0;
+    PyObject* o = args[at++];
+    const long long v = PyLong_CheckExact(o) ? PyLong_AsLongLong(o) : -1;
+    if (!PyLong_CheckExact(o) || (v == -1 && PyErr_Occurred())) {
+      PyErr_Clear();
+      ok = false;
+    }
+    return v;
+  }
+  double real() {
+    if (!ok) return 0;
+    PyObject* o = args[at++];
+    if (!PyFloat_CheckExact(o)) ok = false;
+    return ok ? PyFloat_AS_DOUBLE(o) : 0;
+  }
+  bool boolean() {
+    if (!ok) return false;
+    PyObject* o = args[at++];
+    ok = PyBool_Check(o);
+    return o == Py_True;
+  }
+  std::string text() {
+    if (!ok) return {};
+    Py_ssize_t len = 0;
+    PyObject* o = args[at++];
+    const char* s = PyUnicode_CheckExact(o) ? PyUnicode_AsUTF8AndSize(o, &len) : nullptr;
+    if (s == nullptr) {
+      PyErr_Clear();
+      ok = false;
+      return {};
+    }
+    return std::string(s, size_t(len));
+  }
+};
+
+PyObject* report(const std::vector<int64_t>& v) {
+  PyObject* t = PyTuple_New(Py_ssize_t(v.size()));
+  if (t == nullptr) return nullptr;
+  for (size_t i = 0; i < v.size(); ++i) {
+    PyObject* x = PyLong_FromLongLong(v[i]);
+    if (x == nullptr) {
+      Py_DECREF(t);
+      return nullptr;
+    }
+    PyTuple_SET_ITEM(t, Py_ssize_t(i), x);
+  }
+  return t;
+}
+
+template <typename F>
+auto without_gil(F&& f) {
+  py::gil_scoped_release release;
+  return f();
+}
+
+PyObject* fast_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  FastArgs a(args, n, 7);
+  const auto ins = a.list(), outs = a.list();
+  const int64_t comm = a.integer();
+  const std::string algo = a.text();
+  const int64_t ctas = a.integer(), warps = a.integer(), flags = a.integer();
+  if (!a.ok) Py_RETURN_NONE;
+  return report(without_gil([&] { return all_reduce_lists(ins, outs, comm, algo, ctas, warps, flags); }));
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* fast_all_gather(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  FastArgs a(args, n, 7);
+  const auto ins = a.list(), outs = a.list();
+  const int64_t comm = a.integer();
+  const std::string algo = a.text();
+  const int64_t ctas = a.integer(), warps = a.integer(), flags = a.integer();
+  if (!a.ok) Py_RETURN_NONE;
+  return report(without_gil([&] { return all_gather_lists(ins, outs, comm, algo, ctas, warps, flags); }));
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* fast_reduce_scatter(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  FastArgs a(args, n, 6);
+  const auto ins = a.list(), outs = a.list();
+  const int64_t comm = a.integer();
+  const std::string algo = a.text();
+  const int64_t ctas = a.integer(), flags = a.integer();
+  if (!a.ok) Py_RETURN_NONE;
+  return report(without_gil([&] { return reduce_scatter_lists(ins, outs, comm, algo, ctas, flags); }));
+  END_HANDLE_TH_ERRORS
+}
+
+// (outs, residual outs, launch report), or None
+PyObject* fast_ar_rmsnorm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  FastArgs a(args, n, 5);
+  const auto xs = a.list(), residuals = a.list(), gammas = a.list();
+  const double eps = a.real();
+  const int64_t comm = a.integer();
+  if (!a.ok) Py_RETURN_NONE;
+  auto r = without_gil([&] { return ar_rmsnorm_lists(xs, residuals, gammas, eps, comm); });
+  std::vector<at::Tensor>& both = std::get<0>(r);
+  if (both.empty()) Py_RETURN_NONE;
+  const size_t half = both.size() / 2;
+  PyObject* result = PyTuple_New(3);
+  if (result == nullptr) return nullptr;
+  for (int part = 0; part < 2; ++part) {
+    PyObject* list = PyList_New(Py_ssize_t(half));
+    if (list == nullptr) {
+      Py_DECREF(result);
+      return nullptr;
+    }
+    PyTuple_SET_ITEM(result, part, list);
+    for (size_t i = 0; i < half; ++i) {
+      PyObject* t = THPVariable_Wrap(std::move(both[size_t(part) * half + i]));
+      if (t == nullptr) {
+        Py_DECREF(result);
+        return nullptr;
+      }
+      PyList_SET_ITEM(list, Py_ssize_t(i), t);
+    }
+  }
+  PyObject* info = report(std::get<1>(r));
+  if (info == nullptr) {
+    Py_DECREF(result);
+    return nullptr;
+  }
+  PyTuple_SET_ITEM(result, 2, info);
+  return result;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* fast_local_gemm_ar(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  FastArgs a(args, n, 9);
+  auto xs = a.list(), ws = a.list(), residuals = a.list(), gammas = a.list(), outs = a.list(), res_outs = a.list();
+  const double eps = a.real();
+  const bool with_norm = a.boolean();
+  const int64_t comm = a.integer();
+  if (!a.ok) Py_RETURN_NONE;
+  return report(without_gil([&] {
+    return local_gemm_ar(std::move(xs), std::move(ws), std::move(residuals), std::move(gammas), std::move(outs), std::move(res_outs), eps, with_norm,
+                         comm);
+  }));
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* fast_local_ag_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  FastArgs a(args, n, 4);
+  auto xs = a.list(), ws = a.list(), outs = a.list();
+  const int64_t comm = a.integer();
+  if (!a.ok) Py_RETURN_NONE;
+  return report(without_gil([&] { return local_ag_gemm(std::move(xs), std::move(ws), std::move(outs), comm); }));
+  END_HANDLE_TH_ERRORS
+}
+
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyMethodDef fast_method(const char* name) {
+  return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(F)), METH_FASTCALL, nullptr};
+}
+PyMethodDef g_fast_methods[] = {fast_method<fast_all_reduce>("fast_all_reduce"),
+                                fast_method<fast_all_gather>("fast_all_gather"),
+                                fast_method<fast_reduce_scatter>("fast_reduce_scatter"),
+                                fast_method<fast_ar_rmsnorm>("fast_ar_rmsnorm"),
+                                fast_method<fast_local_gemm_ar>("fast_local_gemm_ar"),
+                                fast_method<fast_local_ag_gemm>("fast_local_ag_gemm"),
+                                {nullptr, nullptr, 0, nullptr}};
+
 int64_t gemm_ar_workspace_bytes(int64_t world, int64_t M, int64_t N) { return int64_t(gemm_ar_workspace(int(world), M, N).total()); }
 
 }  // namespace
@@ -723,6 +937,7 @@ TORCH_LIBRARY(b200ipc, m) {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "b200ipc native extension";
+  if (PyModule_AddFunctions(m.ptr(), g_fast_methods) != 0) throw py::error_already_set();
   m.def("comm_create", &comm_create);
   m.def("comm_create_virtual", &comm_create_virtual);
   m.def("comm_destroy", &comm_destroy);

@@ -75,6 +75,10 @@ class Communicator:
         self._all_reduce_lists, self._all_gather_lists = ops.all_reduce_lists.default, ops.all_gather_lists.default
         self._reduce_scatter_lists, self._ar_rmsnorm_lists = ops.reduce_scatter_lists.default, ops.ar_rmsnorm_lists.default
         self._local_gemm_ar, self._local_ag_gemm = ops.local_gemm_ar.default, ops.local_ag_gemm.default
+        # the same past the dispatcher; they answer None where a call has to go through the operator
+        C = self._C
+        self._fast_all_reduce, self._fast_all_gather, self._fast_reduce_scatter = C.fast_all_reduce, C.fast_all_gather, C.fast_reduce_scatter
+        self._fast_ar_rmsnorm, self._fast_local_gemm_ar, self._fast_local_ag_gemm = C.fast_ar_rmsnorm, C.fast_local_gemm_ar, C.fast_local_ag_gemm
         # largest input (bytes per rank) the one-shot all-reduce + residual + RMSNorm kernel is used for
         self.fused_oneshot_max_bytes = 256 << 10
 
@@ -176,7 +180,8 @@ class Communicator:
         """Sum over ranks.  In place unless `out` is given.  Stream-ordered on the current stream."""
         ins = self._lists(x)
         outs = ins if out is None else self._lists(out)
-        self._info = self._all_reduce_lists(ins, [] if out is None else outs, self._h, algo, ctas, warps, flags)
+        call = (ins, [] if out is None else outs, self._h, algo, ctas, warps, flags)
+        self._info = self._fast_all_reduce(*call) or self._all_reduce_lists(*call)
         return self._ret(x, outs)
 
     def all_gather(self, x: TensorOrList, out: Optional[TensorOrList] = None, algo: str = "allgather_auto", *,
@@ -187,7 +192,8 @@ class Communicator:
             outs = [torch.empty((self.world * t.shape[0],) + tuple(t.shape[1:]), dtype=t.dtype, device=t.device) for t in ins]
         else:
             outs = self._lists(out)
-        self._info = self._all_gather_lists(ins, outs, self._h, algo, ctas, warps, flags)
+        call = (ins, outs, self._h, algo, ctas, warps, flags)
+        self._info = self._fast_all_gather(*call) or self._all_gather_lists(*call)
         return self._ret(x, outs)
 
     def reduce_scatter(self, x: TensorOrList, out: Optional[TensorOrList] = None, algo: str = "auto", *, ctas: int = 0,
@@ -198,7 +204,8 @@ class Communicator:
             outs = [torch.empty((t.shape[0] // self.world,) + tuple(t.shape[1:]), dtype=t.dtype, device=t.device) for t in ins]
         else:
             outs = self._lists(out)
-        self._info = self._reduce_scatter_lists(ins, outs, self._h, algo, ctas, flags)
+        call = (ins, outs, self._h, algo, ctas, flags)
+        self._info = self._fast_reduce_scatter(*call) or self._reduce_scatter_lists(*call)
         return self._ret(x, outs)
 
     def allreduce_residual_rmsnorm(self, x: TensorOrList, residual: TensorOrList, gamma: TensorOrList, eps: float = 1e-5,
@@ -214,6 +221,10 @@ class Communicator:
         rs = self._lists(residual)
         gs = self._lists(gamma)
         if ctas == 0 and self._direct:
+            fast = self._fast_ar_rmsnorm(xs, rs, gs, eps, self._h)
+            if fast:
+                outs, res_outs, self._info = fast
+                return self._ret(x, outs), self._ret(x, res_outs)
             both, info = self._ar_rmsnorm_lists(xs, rs, gs, eps, self._h)
             if both:
                 self._info = info
@@ -317,9 +328,9 @@ class Communicator:
         with_norm = gamma is not None
         want_res = residual is not None
         if local:
-            v = self._local_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
-                                                L(out), L(res_out) if want_res else [], eps, with_norm, self._h)
-            self._info = v
+            call = (xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [], L(out),
+                    L(res_out) if want_res else [], eps, with_norm, self._h)
+            self._info = self._fast_local_gemm_ar(*call) or self._local_gemm_ar(*call)
             return (out, res_out) if with_norm or want_res else out
         v = torch.ops.b200ipc.fused_gemm_ar(xs, ws, self._lists(residual) if want_res else [], self._lists(gamma) if with_norm else [],
                                             L(out), L(res_out) if want_res else [], L(wsp), eps, with_norm, self._h, ctas, False)
@@ -379,8 +390,8 @@ class Communicator:
                              and not (torch.is_grad_enabled() and any(t.requires_grad for t in ws)))
             if fits and ctas == 0 and self._direct:
                 outs = [torch.empty(M, N, dtype=t.dtype, device=t.device) for t in xs]
-                v = self._local_ag_gemm(xs, ws, outs, self._h)
-                self._info = v
+                call = (xs, ws, outs, self._h)
+                self._info = self._fast_local_ag_gemm(*call) or self._local_ag_gemm(*call)
                 return self._ret(x_shard, outs)
         if not fused:
             gathered = self.all_gather(xs if self._virtual else xs[0], None, "allgather_auto")

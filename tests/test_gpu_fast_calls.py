@@ -1,0 +1,79 @@
+"""The list calls past the dispatcher: where a mode, a profiler or a subclass would see the operator, the operator is what runs,
+and both ways give the same results, launch reports and errors."""
+import pytest
+import torch
+from torch.utils._python_dispatch import TorchDispatchMode
+
+from gpu_ipc_example_b200 import Communicator
+
+pytestmark = pytest.mark.gpu
+
+
+class Seen(TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.names = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.names.append(str(func))
+        return func(*args, **(kwargs or {}))
+
+
+class Sub(torch.Tensor):
+    pass
+
+
+def _calls(comm, xs, ws, res, gam):
+    W = comm.world
+    yield "all_reduce", lambda: comm.all_reduce(xs, [torch.empty_like(t) for t in xs])
+    yield "all_reduce in place", lambda: comm.all_reduce([t.clone() for t in xs])
+    yield "all_gather", lambda: comm.all_gather(xs, [t.new_empty(W * t.shape[0], t.shape[1]) for t in xs])
+    yield "reduce_scatter", lambda: comm.reduce_scatter(xs, [t.new_empty(t.shape[0] // W, t.shape[1]) for t in xs])
+    yield "norm", lambda: sum(comm.allreduce_residual_rmsnorm(xs, res, gam), [])
+    yield "linear", lambda: [t.clone() for t in sum(comm.linear_allreduce(xs, ws, res, gam), [])]
+    yield "gather_linear", lambda: comm.allgather_linear(xs, ws)
+
+
+@pytest.mark.parametrize("world", [2, 8])
+def test_both_ways_agree(world):
+    g = torch.Generator(device="cuda").manual_seed(world)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).half()
+    xs, ws = [rnd(16, 512) for _ in range(world)], [rnd(512, 512) for _ in range(world)]
+    res, gam = [rnd(16, 512)] * world, [rnd(512)] * world
+    with Communicator.virtual(world, 0, staging_bytes=64 << 20) as comm:
+        for name, call in _calls(comm, xs, ws, res, gam):
+            fast, info = call(), comm.last_info
+            seen = Seen()
+            with seen:
+                slow = call()
+            assert comm.last_info == info, name
+            for a, b in zip(fast, slow):
+                assert torch.equal(a, b), name
+        subs = [t.as_subclass(Sub) for t in xs]
+        for a, b in zip(comm.all_reduce(subs, [torch.empty_like(t) for t in xs]), comm.all_reduce(xs, [torch.empty_like(t) for t in xs])):
+            assert torch.equal(a, b)
+        with torch.profiler.profile() as prof:
+            comm.all_reduce(xs, [torch.empty_like(t) for t in xs])
+        assert any("b200ipc::all_reduce_lists" in e.name for e in prof.events())
+        torch.cuda.synchronize()
+        comm.check()
+
+
+def test_errors_are_the_operators():
+    with Communicator.virtual(2, 0, staging_bytes=16 << 20) as comm:
+        a = [torch.zeros(64, device="cuda").half() for _ in range(2)]
+        for ins, outs, kw in ((a, [torch.zeros(64, device="cuda").half(), torch.zeros(32, device="cuda").half()], {}),  # sizes
+                              (a, a, dict(algo="no such algorithm")), ([t.float() for t in a], None, {}), ([t.cpu() for t in a], None, {}),
+                              (a, None, dict(ctas="one")), ([a[0], None], None, {})):
+            errors = []
+            for listen in (False, True):
+                with pytest.raises((RuntimeError, TypeError, ValueError)) as e:
+                    if listen:
+                        with Seen():
+                            comm.all_reduce(ins, outs, **kw)
+                    else:
+                        comm.all_reduce(ins, outs, **kw)
+                errors.append((e.type, str(e.value).split("\n")[0]))
+            assert errors[0] == errors[1]
+        out = comm.all_reduce(a, None)  # the communicator still works
+        assert torch.equal(out[0], a[0])

@@ -617,7 +617,7 @@ CollInfo Comm::launch_bulk(BulkModeId mode, bool nvls, bool direct, DType t, con
     args.v[i].aux[0] = sym_off;
     args.v[i].aux[1] = copy_flags;
   }
-  launch(fn, ctas, threads, &args, 0, stream, false, /*meet=*/!direct);
+  launch(fn, ctas, threads, &args, 0, stream, /*pdl=*/direct, /*meet=*/!direct);
 
   CollInfo info;
   info.sched = nvls ? SchedKind::Nvls : SchedKind::Bulk;

@@ -8,6 +8,7 @@
 #include "../common/check.h"
 #include "fused_ops.h"
 #include "gemm_local.cuh"
+#include "gemm_stream.cuh"
 #include "tensor_map.h"
 
 namespace b200ipc {
@@ -160,6 +161,85 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   info->launches = 1;
 }
 
+const void* stream_kernel(DType t, int bn) {
+  if (t == DType::F16)
+    return bn == 16 ? reinterpret_cast<const void*>(&gemm_stream_kernel<__half, 16>) : reinterpret_cast<const void*>(&gemm_stream_kernel<__half, 32>);
+  return bn == 16 ? reinterpret_cast<const void*>(&gemm_stream_kernel<__nv_bfloat16, 16>)
+                  : reinterpret_cast<const void*>(&gemm_stream_kernel<__nv_bfloat16, 32>);
+}
+
+// Accumulator columns and K split of the weight-streaming kernel; bn = 0 where the tiles of gemm_local.cuh are taken.
+struct StreamPlan {
+  int bn = 0, splits = 1;
+};
+
+// `columns`: the rows of X, with their padding between shards; `exact`: the accumulator has just these.  As many splits as there
+// are places for CTAs (two on an SM), with at least eight blocks of K and four rows to finish for each; a narrow layer pads its rows
+// to 32 for an eighth split (8 rows x 8192 x 1280: four splits 13.1 us, eight 9.6, the other kernel 11.4).  That one keeps what
+// it measured ahead or level in (with norm, this kernel / that one): more than 16 rows for a CTA to finish (24 rows x 448 x 4864
+// 8.2 us / 7.8), weights of which the part fetched ahead is next to nothing (470 MB: 81 / 80).
+StreamPlan plan_stream(const Comm& comm, int64_t columns, bool exact, int64_t tiles, int64_t kb_total) {
+  StreamPlan p;
+  if (columns > kStrMaxRows || (exact && columns != 16 && columns != 32)) return p;
+  if (tiles * kb_total * kStrTileBytes > (int64_t(192) << 20)) return p;
+  int bn = columns <= 16 ? 16 : 32;
+  auto room = [&](int splits) { return tiles * splits <= 2 * comm.sm_count() && kb_total >= 8 * splits; };
+  while (p.splits < 8 && bn / (2 * p.splits) >= 4 && room(2 * p.splits)) p.splits *= 2;
+  if (bn == 16 && p.splits == 4 && !exact && room(8)) {
+    bn = 32;
+    p.splits = 8;
+  }
+  if (std::min<int64_t>(bn / p.splits, columns) <= 16) p.bn = bn;
+  return p;
+}
+
+void launch_stream(Comm& comm, StreamGemmArgs& args, DType t, const StreamPlan& p, const void* const* xs, const void* const* ws,
+                   cudaStream_t stream, CollInfo* info) {
+  const int W = comm.world();
+  const void* fn = stream_kernel(t, p.bn);
+  args.n_tiles = int(ceil_div64(args.N, kStrWRows));
+  args.splits = p.splits;
+  const int64_t ctas = int64_t(args.n_tiles) * args.groups * p.splits;
+  const int slab = (p.splits - 1) * (p.bn / p.splits) * 128 * 4;
+  args.stages = std::min(kStrMaxStages, (kStrSmemBudget - 1024 - slab) / (kStrTileBytes + p.bn * kGemmBK * 2));
+  args.warm = int(kStrWarmBytes / (ctas * kStrTileBytes));
+  for (int r = 0; r < W; ++r) {
+    encode_tile_map(&args.tma_x[r], t, xs[r], uint64_t(args.rows), uint64_t(args.K), uint32_t(args.merged ? args.merged_rows : p.bn));
+    encode_tile_map(&args.tma_w[r], t, ws[r], uint64_t(args.N), uint64_t(args.K), kStrWRows);
+    args.w[r] = ws[r];
+  }
+  KArgs views;
+  comm.fill_views(&views, nullptr, nullptr, 0, 0);
+  args.status = views.v[0].status;
+  args.abort_word = reinterpret_cast<uint32_t*>(views.v[0].heap + views.lay.ctrl_off + kCtrlAbortOff);
+  args.timeout_ns = views.v[0].timeout_ns;
+  args.rank = views.v[0].rank;
+  B200_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrSmemBudget));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(ctas));
+  cfg.blockDim = dim3(kStrThreads);
+  cfg.dynamicSmemBytes = kStrSmemBudget;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(p.splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2u : 1u;
+  void* params[] = {&args};
+  B200_CUDA_CHECK(cudaLaunchKernelExC(&cfg, fn, params));
+  comm.note_launch();
+  info->sched = SchedKind::Bulk;
+  info->proto = ProtoKind::LL512;
+  info->ctas = int(ctas);
+  info->warps = kStrThreads / 32;
+  info->nwires = info->ctas * info->warps;
+  info->steps = 1;
+  info->launches = 1;
+}
+
 void check_local(Comm& comm, int64_t M, int64_t N, int64_t K) {
   B200_REQUIRE(comm.nlocal() == comm.world(), "every rank must be driven by this process");
   const int W = comm.world();
@@ -176,13 +256,25 @@ CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64
                               bool with_norm, cudaStream_t stream) {
   check_local(comm, M, N, K);
   const int W = comm.world();
+  const int64_t kb = ceil_div64(K, kGemmBK) * W;
+  const StreamPlan stream_plan = plan_stream(comm, M, false, ceil_div64(N, kStrWRows), kb);
   LocalGemmArgs args;
-  std::memset(&args, 0, sizeof(args));
-  args.rows = int(M);
-  args.N = int(N);
-  args.K = int(K);
-  args.segs = W;
-  args.shards = args.groups = 1;
+  StreamGemmArgs sargs;
+  if (stream_plan.bn) {
+    std::memset(&sargs, 0, sizeof(sargs));
+    sargs.rows = int(M);
+    sargs.N = int(N);
+    sargs.K = int(K);
+    sargs.segs = W;
+    sargs.groups = 1;
+  } else {
+    std::memset(&args, 0, sizeof(args));
+    args.rows = int(M);
+    args.N = int(N);
+    args.K = int(K);
+    args.segs = W;
+    args.shards = args.groups = 1;
+  }
   RowNormArgs norm;
   std::memset(&norm, 0, sizeof(norm));
   norm.N = int(N);
@@ -196,16 +288,20 @@ CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64
     if (with_norm) B200_REQUIRE(p.gamma != nullptr, "RMSNorm needs gamma");
     xs[i] = p.x;
     ws[i] = p.w;
-    args.residual[i] = p.residual;
-    args.sum[i] = p.res_out ? p.res_out : p.out;
-    args.copy[i] = (p.res_out && !with_norm) ? p.out : nullptr;
-    norm.sum[i] = args.sum[i];
+    void* sum = p.res_out ? p.res_out : p.out;
+    void* copy = (p.res_out && !with_norm) ? p.out : nullptr;
+    (stream_plan.bn ? sargs.residual : args.residual)[i] = p.residual;
+    (stream_plan.bn ? sargs.sum : args.sum)[i] = sum;
+    (stream_plan.bn ? sargs.copy : args.copy)[i] = copy;
+    norm.sum[i] = sum;
     norm.gamma[i] = p.gamma;
     norm.out[i] = p.out;
   }
-  const int64_t kb = ceil_div64(K, kGemmBK) * W;
   CollInfo info;
-  launch_local(comm, args, t, plan_local(t, comm.device(), M, 1, 1, N, kb, 0), xs, ws, stream, &info);
+  if (stream_plan.bn)
+    launch_stream(comm, sargs, t, stream_plan, xs, ws, stream, &info);
+  else
+    launch_local(comm, args, t, plan_local(t, comm.device(), M, 1, 1, N, kb, 0), xs, ws, stream, &info);
   if (with_norm) {
     // two vectors a thread where there are too few rows to fill the GPU otherwise
     const int threads = M * W <= 2 * comm.sm_count() ? 512 : 256;
@@ -243,6 +339,9 @@ CollInfo local_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64
       bn_only = int(per_shard * W);
     }
   }
+  // the weight-streaming kernel's tile: all shards side by side, in whole swizzle blocks of eight rows
+  const int64_t stream_rows = W > 1 ? ceil_div64(M / W, 8) * 8 : M;
+  const StreamPlan stream_plan = plan_stream(comm, stream_rows * W, W > 1, ceil_div64(N, kStrWRows) * W, ceil_div64(K, kGemmBK));
   const void* xs[kMaxRanks];
   const void* ws[kMaxRanks];
   for (int i = 0; i < W; ++i) {
@@ -252,6 +351,22 @@ CollInfo local_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64
     args.sum[i] = ptrs[i].out;
   }
   CollInfo info;
+  if (stream_plan.bn) {
+    StreamGemmArgs sargs;
+    std::memset(&sargs, 0, sizeof(sargs));
+    sargs.rows = args.rows;
+    sargs.N = args.N;
+    sargs.K = args.K;
+    sargs.segs = 1;
+    sargs.groups = W;
+    if (W > 1) {
+      sargs.merged = W;
+      sargs.merged_rows = int(stream_rows);
+    }
+    for (int i = 0; i < W; ++i) sargs.sum[i] = ptrs[i].out;
+    launch_stream(comm, sargs, t, stream_plan, xs, ws, stream, &info);
+    return info;
+  }
   launch_local(comm, args, t, plan_local(t, comm.device(), M / W, args.shards, W, N, ceil_div64(K, kGemmBK), bn_only), xs, ws, stream, &info);
   return info;
 }

@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(512) row_norm_kernel(const __grid_constant__ R
   const uint4* gamma = static_cast<const uint4*>(args.gamma[q]);
   const int step = int(blockDim.x);
   const bool in_regs = nvec <= U * step;
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const uint4* src = static_cast<const uint4*>(args.sum[q]) + size_t(blockIdx.x) * nvec;
   uint4* dst = static_cast<uint4*>(args.out[q]) + size_t(blockIdx.x) * nvec;
   uint4 x[U], g[U];

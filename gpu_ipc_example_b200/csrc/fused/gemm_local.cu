@@ -161,12 +161,12 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   info->launches = 1;
 }
 
-const void* stream_kernel(DType t, int bn) {
-  if (t == DType::F16)
-    return bn == 16 ? reinterpret_cast<const void*>(&gemm_stream_kernel<__half, 16>) : reinterpret_cast<const void*>(&gemm_stream_kernel<__half, 32>);
-  return bn == 16 ? reinterpret_cast<const void*>(&gemm_stream_kernel<__nv_bfloat16, 16>)
-                  : reinterpret_cast<const void*>(&gemm_stream_kernel<__nv_bfloat16, 32>);
+template <typename T>
+const void* stream_kernel_of(int bn) {
+  return bn == 16 ? reinterpret_cast<const void*>(&gemm_stream_kernel<T, 16>)
+         : bn == 32 ? reinterpret_cast<const void*>(&gemm_stream_kernel<T, 32>) : reinterpret_cast<const void*>(&gemm_stream_kernel<T, 64>);
 }
+const void* stream_kernel(DType t, int bn) { return t == DType::F16 ? stream_kernel_of<__half>(bn) : stream_kernel_of<__nv_bfloat16>(bn); }
 
 // Accumulator columns and K split of the weight-streaming kernel; bn = 0 where the tiles of gemm_local.cuh are taken.
 struct StreamPlan {
@@ -177,19 +177,20 @@ struct StreamPlan {
 // are places for CTAs (two on an SM), with at least eight blocks of K and four rows to finish for each; a narrow layer pads its rows
 // to 32 for an eighth split (8 rows x 8192 x 1280: four splits 13.1 us, eight 9.6, the other kernel 11.4).  That one keeps what
 // it measured ahead or level in (with norm, this kernel / that one): more than 16 rows for a CTA to finish (24 rows x 448 x 4864
-// 8.2 us / 7.8), weights of which the part fetched ahead is next to nothing (470 MB: 81 / 80).
+// 8.2 us / 7.8), more than 32 rows where that leaves places empty (48 x 3584 x 8192, 256 CTAs 17.0 / 18.7; 48 x 3000 x 5120, 160
+// CTAs 15.2 / 14.0), weights of which the part fetched ahead is next to nothing (470 MB: 81 / 80).
 StreamPlan plan_stream(const Comm& comm, int64_t columns, bool exact, int64_t tiles, int64_t kb_total) {
   StreamPlan p;
-  if (columns > kStrMaxRows || (exact && columns != 16 && columns != 32)) return p;
+  if (columns > kStrMaxRows || (exact && columns != 16 && columns != 32 && columns != 64)) return p;
   if (tiles * kb_total * kStrTileBytes > (int64_t(192) << 20)) return p;
-  int bn = columns <= 16 ? 16 : 32;
+  int bn = columns <= 16 ? 16 : columns <= 32 ? 32 : 64;
   auto room = [&](int splits) { return tiles * splits <= 2 * comm.sm_count() && kb_total >= 8 * splits; };
   while (p.splits < 8 && bn / (2 * p.splits) >= 4 && room(2 * p.splits)) p.splits *= 2;
   if (bn == 16 && p.splits == 4 && !exact && room(8)) {
     bn = 32;
     p.splits = 8;
   }
-  if (std::min<int64_t>(bn / p.splits, columns) <= 16) p.bn = bn;
+  if (std::min<int64_t>(bn / p.splits, columns) <= 16 && (bn < 64 || tiles * p.splits >= 200)) p.bn = bn;
   return p;
 }
 

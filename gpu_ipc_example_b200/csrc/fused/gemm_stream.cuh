@@ -1,13 +1,13 @@
-// The linear layers of gemm_local.cuh for the few rows of a decode step: at most 32 rows of X, so that what counts is the
+// The linear layers of gemm_local.cuh for the few rows of a decode step: at most 64 rows of X, so that what counts is the
 // stream of W from memory.  As there, every rank's operands are in one address space and nothing is exchanged.
 //
-// One tile per CTA (cluster): 128 rows of W (the tensor core's M side) and all rows of X, padded to 16 or 32 (its N side).  K is
+// One tile per CTA (cluster): 128 rows of W (the tensor core's M side) and all rows of X, padded to 16, 32 or 64 (its N side).  K is
 // split over the CTAs of a cluster until tiles x splits fill the places; every CTA hands its fp32 partial sums for a share of the
 // rows of X to the CTA that owns them (st.async, counted on the receiver's barrier), and the owner adds them in a fixed order.
 //
 // What bounds it is the chain around the stream: launch and first loads 4.5 us, split sum, epilogue and exit 4, norm 2.6 of the
 // 17.2 us that 16 rows x 3584 x 8192 with norm took in the kernel of gemm_local.cuh, one launch after the other.  So this one is
-// cut to let the next launch in: 106 KB of shared memory, 72 or 80 registers x 320 threads and 32 columns of tensor memory leave
+// cut to let the next launch in: 106 KB of shared memory, 72 or 80 registers x 320 threads and 64 columns of tensor memory leave
 // room for a second CTA on the SM, and dependents are let go at once.  The next kernel's CTAs set up and bring the first 24 MB of
 // W to L2 as soon as there is room for them, while this kernel's stragglers or its norm are at work.  Now 14.0 us (one row 17.0 ->
 // 13.0, 32 rows 17.9 -> 15.0, 2048 x 6016 12.0 -> 10.0, 8192 x 7168 26.0 -> 23.3, back to back).  With less of W fetched ahead the
@@ -20,8 +20,8 @@ namespace b200ipc {
 
 constexpr int kStrThreads = 320;  // warp 0: TMA, warp 1: MMA, warps 2-5 and 6-9: two epilogue groups
 constexpr int kStrWRows = 128;
-constexpr int kStrMaxRows = 32;   // rows of X
-constexpr int kStrTmemCols = 32;  // accumulator columns
+constexpr int kStrMaxRows = 64;   // rows of X
+constexpr int kStrTmemCols = 64;  // accumulator columns
 constexpr int kStrMaxStages = 8;
 constexpr int kStrSmemBudget = 106 * 1024;
 constexpr int kStrTileBytes = kStrWRows * kGemmBK * 2;  // a stage's block of W
@@ -50,20 +50,18 @@ struct StreamGemmArgs {
   int warm;         // k blocks of W that a CTA brings to L2 before the wait for the previous kernel
 };
 
-// 2, 4, 8 or 16 accumulator columns of the warp's 32 lanes
+// 2, 4 or 8 accumulator columns of the warp's 32 lanes
 template <int O>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[O]) {
   if constexpr (O == 2)
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
   else if constexpr (O == 4)
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
-  else if constexpr (O == 8)
-    tmem_ld_8cols(taddr, r);
   else
-    tmem_ld_16cols(taddr, r);
+    tmem_ld_8cols(taddr, r);
 }
 
-// BN: columns of the accumulator, 16 or 32.
+// BN: columns of the accumulator: 16, 32 or 64.
 template <typename T, int BN>
 __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __grid_constant__ StreamGemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
@@ -218,7 +216,8 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
       if (splits > 1) {  // the others' shares to them, straight from the registers
         constexpr int H = BN / 2;
         uint32_t acc[H];
-        tmem_ld_cols<H>(tmem_lane + uint32_t(half * H), acc);
+#pragma unroll
+        for (int c = 0; c < H; c += 8) tmem_ld_8cols(tmem_lane + uint32_t(half * H + c), acc + c);
         tmem_ld_wait();
         uint32_t dst = 0, bar = 0;
         int o = 0;

@@ -22,7 +22,8 @@ def _close(got, want, dtype):
 # no block; ranks that meet inside a share of K; splits 0: the other kernel's side of the rule
 @pytest.mark.parametrize("world,M,K,N,splits", [
     (1, 1, 72, 4864, 1), (1, 16, 448, 4864, 1), (1, 17, 448, 4864, 0), (1, 16, 1024, 8192, 2), (1, 17, 1024, 8192, 2), (1, 16, 2048, 3136, 4),
-    (1, 5, 8192, 1280, 8), (1, 17, 2056, 6016, 4), (1, 32, 3000, 4928, 4), (1, 33, 2048, 6016, 0), (2, 15, 1000, 5120, 4), (2, 31, 1792, 8192, 4),
+    (1, 5, 8192, 1280, 8), (1, 17, 2056, 6016, 4), (1, 32, 3000, 4928, 4), (1, 33, 2048, 6464, 4), (1, 64, 2056, 6464, 4),
+    (1, 64, 2056, 6016, 0), (1, 64, 448, 4864, 0), (1, 65, 2048, 8192, 0), (2, 48, 1000, 8192, 4), (2, 15, 1000, 5120, 4), (2, 31, 1792, 8192, 4),
     (4, 3, 264, 6144, 2), (8, 16, 136, 8192, 2), (8, 24, 456, 4864, 4)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_linear(world, M, K, N, splits, dtype):

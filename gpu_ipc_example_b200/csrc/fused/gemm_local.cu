@@ -16,6 +16,7 @@ namespace {
 
 struct LocalPlan {
   int bn = 32, m_tiles = 1, splits = 1;
+  int cut = 1;  // parts that the tiles behind the last full wave are taken in
 };
 
 // k blocks per stage: two where a block holds too little work for what its barriers and its commit cost
@@ -65,11 +66,11 @@ int resident_clusters(const void* fn, int device, int splits) {
 // tile 0.5 + 0.0133 BN, hidden behind the next tile's MMAs where there is one; handing partial sums between the pairs of a
 // cluster 1.4 + 0.006 BN (K = 1024, M = 16, N = 8192: one split 15.4 us, two 17.4; K = 3584: 18.6 and 14.5 back to back; both
 // taken with the first W loads ahead of the wait for the kernel in front, 15.5 with a prefetch to L2 there).
-double plan_cost(int64_t tiles, int64_t room, int64_t kb_total, int bn, int splits) {
-  const double waves = double(ceil_div64(tiles, room));
-  const double main = double(ceil_div64(kb_total, splits)) * (0.08 + 0.0012 * bn);
-  const double epi = 0.5 + 0.0133 * bn / splits;
-  return waves * std::max(main, epi) + epi + (splits > 1 ? 1.4 + 0.006 * bn : 0);
+double plan_cost(int64_t tiles, int64_t room, int64_t kb_total, int bn, int splits, int cut) {
+  auto wave = [&](int rows) { return std::max(double(ceil_div64(kb_total, splits)) * (0.08 + 0.0012 * rows), 0.5 + 0.0133 * rows / splits); };
+  const int64_t left = tiles % room;
+  return double(tiles / room) * wave(bn) + (left ? wave(bn / cut) : 0) + 0.5 + 0.0133 * (left ? bn / cut : bn) / splits +
+         (splits > 1 ? 1.4 + 0.006 * bn : 0);
 }
 
 // The tile height and the K split of a problem.  bn_only: the tile's height is given (merged shards).
@@ -93,12 +94,19 @@ LocalPlan plan_local(DType t, int device, int64_t rows, int64_t shards, int64_t 
       const int64_t room = resident_clusters(local_kernel(t, bn), device, splits);
       if (room < 1) continue;
       if (splits > 1 && (tiles > room || kb_total < 4 * splits)) break;  // one tile per cluster, every split with work
-      const double cost = plan_cost(tiles, room, kb_total, bn, splits);
-      if (best_cost == 0 || cost < best_cost) {
-        best_cost = cost;
-        best.bn = bn;
-        best.m_tiles = int(m_tiles);
-        best.splits = splits;
+      // The last wave of tiles often fills a fraction of the GPU: cut in two or four it is over sooner (2048 rows x 3584 x 8192: 256
+      // tiles of 256 rows for 74 pairs, the last 34 in two parts each).  Tall tiles and a long K only, and for what the model gives
+      // as 4 % or more: with K = 1000 and tiles of 128 rows it measured behind.
+      for (int cut = 1; cut <= 4; cut *= 2) {
+        if (cut > 1 && (bn_only || splits > 1 || bn <= 128 || kb_total < 32 || bn % (16 * cut) || tiles <= room || tiles % room * cut > room)) continue;
+        const double cost = plan_cost(tiles, room, kb_total, bn, splits, cut) * (cut > 1 ? 1.04 : 1.0);
+        if (best_cost == 0 || cost < best_cost) {
+          best_cost = cost;
+          best.bn = bn;
+          best.m_tiles = int(m_tiles);
+          best.splits = splits;
+          best.cut = cut;
+        }
       }
     }
   }
@@ -122,8 +130,14 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   // as many m-tiles side by side as keep their X rows in a quarter of L2 while the W tiles pass by
   const int64_t x_bytes = int64_t(p.bn) * args.K * 2 * args.segs;
   args.band = int(std::min<int64_t>(mt_all, std::max<int64_t>(1, (int64_t(32) << 20) / x_bytes)));
+  const int64_t total = mt_all * args.n_tiles * args.groups;
+  const int64_t clusters = std::min<int64_t>(total, resident_clusters(fn, comm.device(), p.splits));
+  B200_REQUIRE(clusters >= 1 && (p.splits == 1 || clusters == total), "GEMM kernel does not fit on the device");
+  args.cut = p.cut;
+  args.cut_from = int(p.cut > 1 ? total - total % clusters : total);
   for (int r = 0; r < W; ++r) {
     encode_tile_map(&args.tma_x[r], t, xs[r], uint64_t(args.rows), uint64_t(args.K), uint32_t(args.merged ? args.merged_rows : p.bn / 2));
+    if (p.cut > 1) encode_tile_map(&args.tma_x_cut[r], t, xs[r], uint64_t(args.rows), uint64_t(args.K), uint32_t(p.bn / p.cut / 2));
     encode_tile_map(&args.tma_w[r], t, ws[r], uint64_t(args.N), uint64_t(args.K), 128);
   }
   KArgs views;
@@ -133,9 +147,6 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   args.timeout_ns = views.v[0].timeout_ns;
   args.rank = views.v[0].rank;
 
-  const int64_t total = mt_all * args.n_tiles * args.groups;
-  const int64_t clusters = std::min<int64_t>(total, resident_clusters(fn, comm.device(), p.splits));
-  B200_REQUIRE(clusters >= 1 && (p.splits == 1 || clusters == total), "GEMM kernel does not fit on the device");
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(clusters * 2 * p.splits));
   cfg.blockDim = dim3(kLocThreads);

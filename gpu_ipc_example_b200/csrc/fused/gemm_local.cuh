@@ -15,6 +15,9 @@
 // multicast), warp 1 of the even CTA the tcgen05.mma, warps 2-9 read the accumulator (double-buffered in tensor memory),
 // round and store.
 //
+// Many tiles: those behind the last full wave are cut in two or four along X, so that the wave which fills a fraction of the GPU
+// is a shorter one (2048 rows x 3584 x 8192 with norm, 256 tiles for 74 pairs: 127 -> 121 us at the power cap).
+//
 // Few tiles (decode, narrow layers): K is split over the pairs of a cluster of 2, 4 or 8 CTAs; after the last MMA every
 // pair hands its fp32 partial sums for a share of the rows to the pair that owns them through distributed shared
 // memory (st.async, counted on the receiver's barrier), and the owners add them in a fixed order (the result does not depend on timing) and run the epilogue.
@@ -41,6 +44,7 @@ constexpr int kLocSmemBudget = 226 * 1024;
 struct LocalGemmArgs {
   alignas(64) CUtensorMap tma_x[kMaxRanks];  // X of rank r [rows, K], box 64 x BN / 2
   alignas(64) CUtensorMap tma_w[kMaxRanks];  // W of rank r [N, K], box 64 x 128
+  alignas(64) CUtensorMap tma_x_cut[kMaxRanks];  // X of rank r, box 64 x BN / cut / 2
   const void* residual[kMaxRanks];           // [M, N] or nullptr (linear only)
   void* sum[kMaxRanks];                      // [M, N]: the result before the norm
   void* copy[kMaxRanks];                     // [M, N] or nullptr: a second copy of it
@@ -56,6 +60,7 @@ struct LocalGemmArgs {
   int merged_rows;  // rows a shard takes in such a tile: `rows` rounded up to whole swizzle blocks
   int groups;    // products with a W and an output of their own (linear: 1, gather: world)
   int bn;        // X rows per tile
+  int cut, cut_from;  // BN > 128: tiles from number cut_from on are taken in `cut` parts of BN / cut rows
   int m_tiles;   // per shard
   int n_tiles;
   int band;      // m-tiles visited before the next W tile
@@ -124,12 +129,20 @@ __device__ __forceinline__ void tmem_ld_16cols(uint32_t taddr, uint32_t (&r)[16]
 
 // Where tile t lies: (group, first X row inside the shard, shard, first W row).
 struct LocTile {
-  int group, shard, m0, n0;
+  int group, shard, m0, n0, bn;
 };
+template <bool CUT>
 __device__ __forceinline__ LocTile loc_tile(const LocalGemmArgs& a, int t) {
   const int mt_all = a.shards * a.m_tiles;
   const int per_group = mt_all * a.n_tiles;
   LocTile o;
+  o.bn = a.bn;
+  int part = 0;
+  if (CUT && t >= a.cut_from) {
+    o.bn = a.bn / a.cut;
+    part = (t - a.cut_from) % a.cut;
+    t = a.cut_from + (t - a.cut_from) / a.cut;
+  }
   o.group = t / per_group;
   int u = t % per_group;
   const int per_band = a.band * a.n_tiles;
@@ -140,7 +153,7 @@ __device__ __forceinline__ LocTile loc_tile(const LocalGemmArgs& a, int t) {
   const int m = band * a.band + u % width;
   o.n0 = (u / width) * kLocWRows;
   o.shard = m / a.m_tiles;
-  o.m0 = (m % a.m_tiles) * a.bn;
+  o.m0 = (m % a.m_tiles) * a.bn + part * o.bn;
   return o;
 }
 
@@ -167,7 +180,8 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   const int kb_seg = (args.K + kGemmBK - 1) / kGemmBK;  // columns past K read as zeros
   const int kb_total = kb_seg * args.segs;
   const int kb0 = int(int64_t(kb_total) * split / splits), kb1 = int(int64_t(kb_total) * (split + 1) / splits);
-  const int total = args.groups * args.shards * args.m_tiles * args.n_tiles;
+  const int tiles = args.groups * args.shards * args.m_tiles * args.n_tiles;
+  const int total = KSUB > 1 ? tiles : args.cut_from + (tiles - args.cut_from) * args.cut;
   const uint64_t timeout_ns = args.timeout_ns;
   volatile int* abort_flag = &s_abort;
 
@@ -205,7 +219,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   };
   auto first_k = [&](const LocTile& t) {
     const int seg = kb0 / kb_seg;
-    return KPos{&args.tma_w[args.groups > 1 ? t.group : seg], &args.tma_x[args.shards > 1 ? t.shard : seg], (kb0 - seg * kb_seg) * kGemmBK};
+    return KPos{&args.tma_w[args.groups > 1 ? t.group : seg], &(KSUB > 1 || t.bn == bn ? args.tma_x : args.tma_x_cut)[args.shards > 1 ? t.shard : seg], (kb0 - seg * kb_seg) * kGemmBK};
   };
   auto next_k = [&](KPos& k) {
     k.col += kGemmBK;
@@ -221,7 +235,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   auto load_x = [&](uint32_t st, int sub, const KPos& k, const LocTile& t) {
     const uint32_t dst = ring_addr + st * stage_bytes + uint32_t(sub) * blk_bytes + a_bytes;
     if (args.merged == 0) {
-      tma_load_2d_pair(dst, k.x, full_pair + st * 8, k.col, t.m0 + side * (bn / 2));
+      tma_load_2d_pair(dst, k.x, full_pair + st * 8, k.col, t.m0 + side * (t.bn / 2));
     } else {
       const int per_side = args.merged / 2;
       for (int i = 0; i < per_side; ++i)
@@ -230,7 +244,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   };
   // No load before the wait: W may be what the kernel before this one writes (the entry points themselves copy a strided one).
   if (args.warm_w && warp == 0 && cluster < total && elect_one()) {
-    const LocTile t = loc_tile(args, cluster);
+    const LocTile t = loc_tile<KSUB == 1>(args, cluster);
     KPos k = first_k(t);
     if (t.n0 + side * 128 < N)
       for (int kb = kb0; kb < min(kb1, kb0 + stages * KSUB); ++kb, next_k(k)) tma_prefetch_2d(k.w, k.col, t.n0 + side * 128);
@@ -242,13 +256,14 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
     if (elect_one()) {
       uint32_t it = 0, st = 0, ph = 1;
       for (int tt = cluster; tt < total && !*abort_flag; tt += nclusters) {
-        const LocTile t = loc_tile(args, tt);
+        const LocTile t = loc_tile<KSUB == 1>(args, tt);
         KPos k = first_k(t);
+        const uint32_t tile_bytes = 2 * (a_bytes + uint32_t(t.bn / 2) * kGemmBK * 2);  // a k block of both CTAs
 #pragma unroll 1
         for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
           const int nsub = KSUB == 1 ? 1 : min(KSUB, kb1 - kb);
           if (!mbar_wait(&empty[st], ph, abort_flag, timeout_ns)) break;
-          if (side == 0) mbar_expect_tx(&full[st], 2 * blk_bytes * uint32_t(nsub));
+          if (side == 0) mbar_expect_tx(&full[st], tile_bytes * uint32_t(nsub));
 #pragma unroll
           for (int sub = 0; sub < KSUB; ++sub) {
             if (sub >= nsub) break;
@@ -271,11 +286,11 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
     }
   } else if (warp == 1) {
     if (side == 0 && elect_one()) {
-      const uint32_t idesc = make_idesc<T>(kLocWRows, bn);
       const uint16_t mask = uint16_t(3u << (crank & ~1u));
       uint32_t st = 0, ph = 0, i = 0;
       for (int tt = cluster; tt < total && !*abort_flag; tt += nclusters, ++i) {
         const uint32_t buf = i & 1u;
+        const uint32_t idesc = make_idesc<T>(kLocWRows, KSUB > 1 || tt < args.cut_from ? bn : bn / args.cut);
         if (!mbar_wait(&acc_empty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, timeout_ns)) break;
         tc_fence_after_sync();
         bool ok = true;
@@ -316,7 +331,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   auto out_off = [&](const LocTile& t, int c) {
     return (size_t(t.shard) * rows + size_t(t.m0 + c)) * size_t(N) + size_t(t.n0 + side * 128 + my_n);
   };
-  auto tile_rows = [&](const LocTile& t) { return args.merged ? bn : min(bn, rows - t.m0); };
+  auto tile_rows = [&](const LocTile& t) { return args.merged ? bn : min(t.bn, rows - t.m0); };
   auto rows_left = [&](const LocTile& t, int c, int cw) { return t.n0 < col_left ? min(cw, rows - t.m0 - c) : 0; };
   auto load_residual = [&](const T* res, size_t off, int left, T (&rv)[kLocChunk]) {
     if (left >= kLocChunk) {
@@ -377,7 +392,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
       const T* res0 = static_cast<const T*>(args.residual[0]);
       uint32_t i = 0;
       for (int tt = cluster; tt < total; tt += nclusters, ++i) {
-        const LocTile t = loc_tile(args, tt);
+        const LocTile t = loc_tile<KSUB == 1>(args, tt);
         const uint32_t buf = i & 1u;
         const int valid = tile_rows(t);
         T rv[kLocChunk];
@@ -413,7 +428,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
     }
   } else {
     // one tile per cluster
-    const LocTile t = loc_tile(args, cluster);
+    const LocTile t = loc_tile<KSUB == 1>(args, cluster);
     const int own = bn / splits;  // rows of X whose sums this pair finishes: a multiple of 8
     const int c_own = split * own, valid = tile_rows(t);
     const T* res0 = static_cast<const T*>(args.residual[0]);
@@ -491,7 +506,9 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
 }
 
 // out = RMSNorm(sum) * gamma for the rows of every rank (blockIdx.y); `out` may be `sum` itself.  One CTA per row; the
-// row stays in registers between the statistic and the scaling (rows of up to 4 x 8 x blockDim elements).
+// row stays in registers between the statistic and the scaling (rows of up to 4 x 8 x blockDim elements).  Behind 2048 rows of
+// 8192 it is bound by memory (15.5 us for its output, the sums that L2 writes back and those it reads again: more CTAs per SM
+// change nothing), behind few rows by its launch.
 struct RowNormArgs {
   const void* sum[kMaxRanks];
   const void* gamma[kMaxRanks];

@@ -77,6 +77,9 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves apart: every thread of the cluster's CTAs arrives once, and waits for all of them later.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
@@ -549,8 +552,10 @@ __global__ void __launch_bounds__(512) row_norm_kernel(const __grid_constant__ R
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float tot = 0.f;
-  for (int w = 0; w < (step >> 5); ++w) tot += s_part[w];
+  // at most 16 warps: their sums by shuffles, not one shared-memory load after another
+  float tot = int(threadIdx.x & 15) < (step >> 5) ? s_part[threadIdx.x & 15] : 0.f;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   const float inv = rsqrtf(tot / float(N) + args.eps);
   for (int v0 = int(threadIdx.x); v0 < nvec; v0 += U * step) {
 #pragma unroll

@@ -9,9 +9,11 @@
 // 17.2 us that 16 rows x 3584 x 8192 with norm took in the kernel of gemm_local.cuh, one launch after the other.  So this one is
 // cut to let the next launch in: 106 KB of shared memory, 72 or 80 registers x 320 threads and 64 columns of tensor memory leave
 // room for a second CTA on the SM, and dependents are let go at once.  The next kernel's CTAs set up and bring the first 24 MB of
-// W to L2 as soon as there is room for them, while this kernel's stragglers or its norm are at work.  Now 14.0 us (one row 17.0 ->
-// 13.0, 32 rows 17.9 -> 15.0, 2048 x 6016 12.0 -> 10.0, 8192 x 7168 26.0 -> 23.3, back to back).  With less of W fetched ahead the
-// memory idles between the launches (16 MB: 14.5), more takes from the stream of the kernel in front (40 MB: 15.6).
+// W to L2 as soon as there is room for them, while this kernel's stragglers or its norm are at work.  Now 13.8 us (one row 17.0 ->
+// 12.7, 32 rows 17.9 -> 14.8, 2048 x 6016 12.0 -> 9.5, 8192 x 7168 26.0 -> 23.6, back to back).  0.2 - 0.5 of that came with the
+// cluster's barrier in two halves: a warp arrives when it has sent its sums and has the others', and its stores pass while the rest
+// of the cluster gets there.  With less of W fetched ahead the memory idles between the launches (16 MB: +0.5), more takes from the
+// stream of the kernel in front (40 MB: +1.6).
 #pragma once
 
 #include "gemm_local.cuh"
@@ -235,6 +237,8 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
       }
     }
+    __syncwarp();
+    if (splits > 1) cluster_arrive();  // this warp has sent its sums and has all of the others'
     // Rows c .. c + O of this group's share.
     auto finish = [&](auto count, int c) {
       constexpr int O = decltype(count)::value;
@@ -291,11 +295,12 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
     }
   }
 
-  // ---- the cluster leaves together: nobody stores into a CTA that is gone; tensor memory goes back ---------------------
+  // ---- a CTA leaves when nobody will store into it any more; tensor memory goes back -------------------------------------
+  __syncwarp();
+  if (splits > 1 && warp < 2) cluster_arrive();
   tc_fence_before_sync();
   __syncthreads();
-  __syncwarp();
-  if (splits > 1) cluster_sync_all();
+  if (splits > 1) cluster_wait();
   tc_fence_after_sync();
   if (warp == 1) tmem_dealloc(tmem_base, kStrTmemCols);
   if (*abort_flag && threadIdx.x == 0) {

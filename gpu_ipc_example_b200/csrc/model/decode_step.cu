@@ -49,12 +49,12 @@ StepLayout step_layout(const Comm& comm, const DecodeStepShape& s) {
     return here;
   };
   l.sync = take(size_t(s.layers + 1) * kStepSyncs * kStepSyncStride * 4);
-  l.arrivals = take(size_t(z.sequences + int64_t(2 * s.layers + 1) * s.batch) * 4);
+  l.arrivals = take(size_t(z.sequences + s.batch) * 4);
+  l.squares = take(size_t(2 * s.batch) * kStepMaxParts * 4);
   l.counter_words = int(at / 4);
   l.xnorm = take(size_t(s.batch) * s.hidden * 2);
   l.attn = take(size_t(W) * s.batch * s.hq * kAttnD * 2);
   l.act = take(size_t(W) * s.batch * s.ffn * 2);
-  l.squares = take(size_t(s.batch) * kStepMaxParts * 4);
   l.part = take(size_t(z.tiles + ctas) * s.batch * kStepTileRows * 4);
   l.apart = take(std::max(size_t(z.sequences + ctas) * G * kMergeRow * 4, size_t(s.batch) * kStepMaxParts * sizeof(Best)));
   l.total = at;
@@ -107,7 +107,7 @@ void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStep
   a.act = ws + lay.act;
   a.part = reinterpret_cast<float*>(ws + lay.part);
   a.apart = reinterpret_cast<float*>(ws + lay.apart);
-  a.squares = reinterpret_cast<float*>(ws + lay.squares);
+  a.squares = reinterpret_cast<uint32_t*>(ws + lay.squares);
   a.sync = reinterpret_cast<uint32_t*>(ws + lay.sync);
   a.arrivals = reinterpret_cast<uint32_t*>(ws + lay.arrivals);
   KArgs views;

@@ -5,9 +5,10 @@
 //
 // A step is bound by what it reads once: the weights and the cache.  As a chain of kernels (eight per layer) every one of them
 // pays its launch, its first loads and its drain while the memory idles: batch 32 at 2048 tokens, hidden 8192, FFN 3584, eight
-// query heads on one KV head, 85 us per layer for 247 MB (38 us at the copy rate).  Here one CTA per SM stays for the whole step and one thread streams everything
-// the CTA will need, in order, through one ring of 16 KB stages (128 x 64 tiles of W, 64 positions of K or V): the stream does
-// not wait for the math, so while the CTAs meet between two phases the ring fills with the weights of the next.
+// query heads on one KV head, 85 us per layer for 247 MB (38 us at the copy rate).  Here one CTA per SM stays for the whole step
+// and one thread streams everything the CTA will need, in order, through one ring of 16 KB stages (128 x 64 tiles of W, 64
+// positions of K or V): the stream does not wait for the math, so while the CTAs meet between two phases the ring fills with the
+// weights of the next.
 //
 //   warp 0       stream: W tiles, K and V tiles (TMA, never waits for another CTA)
 //   warp 1       X tiles: waits until the phase's input is complete, then loads it beside the W tiles
@@ -22,12 +23,13 @@
 // CTAs wait on one another: the launch is cooperative.  Every wait is bounded; a CTA whose wait runs out stops arriving, which
 // ends the others' waits the same way.
 //
-// Measured, four layers and the head of that shape as one step: 423 us as a chain of kernels, 327 here (floor 194: 1.25 GB).
+// Measured, four layers and the head of that shape as one step: 423 us as a chain of kernels, 317 here (floor 194: 1.25 GB).
 // Two thirds of a layer are bound by the stream (gate/up and down: 6 - 7 TB/s), the rest by the chain of meetings: about 1.5 us
-// from the last CTA's store to everybody's next load, eight times a layer, attention 9 us, each norm 3.5 us.  What mattered: one
+// from the last CTA's store to everybody's next load, eight times a layer, attention 9 us, each norm 2.7 us.  What mattered: one
 // body of code for all phases (with one per phase, 320 KB of instructions, every phase ran into cold instruction caches: 528
 // us); streamed lines first to leave L2, where the partial sums and X live (348 -> 324 us); several CTAs per row of a norm.
-// Bringing tiles to L2 ahead of the ring took as much from the stream of the phase at work as it gave the next.
+// Bringing tiles to L2 ahead of the ring, by TMA or by plain prefetches of a warp of its own, 14 stages: gate/up 16.8 -> 12.7 us, but
+// every meeting slower by as much (64 sequences x 4096: 3 - 5 % behind).
 #pragma once
 
 #include "../fused/gemm_ar.cuh"
@@ -87,9 +89,9 @@ struct DecodeStepArgs {
   void* act;      // [world][batch, ffn]
   float* part;    // partial sums: [tile + CTA][batch][128]
   float* apart;   // attention: [(rank, sequence, KV head) + CTA][G][4 + 128]
-  float* squares; // sums of squares of a row's parts: [batch][kStepMaxParts]
+  uint32_t* squares;   // sums of squares of a row's parts, two norms by turns: [2][batch][kStepMaxParts]; 0 = not there yet
   uint32_t* sync;
-  uint32_t* arrivals;  // [rank, sequence, KV head], then [norm of the launch, arg-max][sequence]: CTAs that are through
+  uint32_t* arrivals;  // [rank, sequence, KV head], then for the arg-max [sequence]: CTAs that are through
   StatusBlock* status;
   uint32_t* abort_word;
   uint64_t timeout_ns;
@@ -109,6 +111,19 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p) {
 }
 __device__ __forceinline__ void red_release_gpu_add(uint32_t* p, uint32_t v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t atom_acq_rel_gpu_add(uint32_t* p, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_relaxed_gpu_or(uint32_t* p, uint32_t v) {
+  asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // Generic stores before it are seen by asynchronous (TMA) reads after it, and the other way round.
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
@@ -313,11 +328,11 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
   const int a0 = at.u0, a1 = at.u1;
   const int parts = min(max(ctas / B, 1), kStepMaxParts);  // CTAs that share a row of a norm or of the arg-max
   auto counter = [&](int l, int s) { return args.sync + (size_t(args.first_layer + l) * kStepSyncs + size_t(s)) * kStepSyncStride; };
-  // Bounded: false where the count did not arrive in time or this CTA has given up.
-  auto wait_count = [&](const uint32_t* p, uint32_t target) {
+  // Bounded: false where `there` did not become true in time or this CTA has given up.
+  auto wait_for = [&](auto there) {
     uint64_t t0 = 0;
     for (uint32_t n = 0;; ++n) {
-      if (ld_acquire_gpu_u32(p) >= target) return true;
+      if (there()) return true;
       if ((n & 63u) == 63u) {
         if (*abort_flag) return false;
         const uint64_t now = globaltimer_ns();
@@ -328,6 +343,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
     *abort_flag = 1;
     return false;
   };
+  auto wait_count = [&](const uint32_t* p, uint32_t target) { return wait_for([&]() { return ld_acquire_gpu_u32(p) >= target; }); };
 
   if (threadIdx.x == 0) {
 #pragma unroll 1
@@ -786,11 +802,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
           bool finish = true;
           if (first != last) {  // the last CTA of the sequence to arrive adds them up
             bad = compute_sync(bad);
-            if (tid == 0) {
-              __threadfence();
-              s_flag = atomicAdd(args.arrivals + seq, 1u) == uint32_t(last - first);
-              __threadfence();
-            }
+            if (tid == 0) s_flag = atom_acq_rel_gpu_add(args.arrivals + seq, 1u) == uint32_t(last - first);
             bad = compute_sync(bad);
             finish = s_flag != 0;
             if (finish && hd < G) {
@@ -905,7 +917,6 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
             s_best[cw] = best;
           }
           bad = compute_sync(bad);
-          uint32_t* arrived = args.arrivals + at.sequences + (2 * args.first_layer + (phase >> 1)) * B + b;
           if (head) {  // the last CTA of the row compares what they found
             if (cw == 0 && !bad) {
               best = warp_best(s_best[lane % kStepComputeWarps]);
@@ -913,9 +924,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
               int is_last = 0;
               if (lane == 0) {
                 found[part0] = make_float2(best.v, __int_as_float(best.i));
-                __threadfence();
-                is_last = atomicAdd(arrived, 1u) == uint32_t(parts - 1);
-                __threadfence();
+                is_last = atom_acq_rel_gpu_add(args.arrivals + at.sequences + b, 1u) == uint32_t(parts - 1);
               }
               if (__shfl_sync(0xffffffffu, is_last, 0)) {
                 const float2 f = __ldcg(found + lane % parts);
@@ -926,18 +935,24 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
             bad = compute_sync(bad);
             continue;
           }
+          // The parts' sums of squares.  A word is its own signal (sign bit set, never zero): nothing else is handed over, so there
+          // is nothing to release, and no second load behind the wait: 1.0 us, not 1.8 (with a counter and a release).  As a
+          // reduction: plain stores came up to 2 us later while the ring fills.  The other norm's words were read by all before
+          // anybody got here: cleared for the next one.
           if (cw == 0) {
-            float* sq = args.squares + size_t(b) * kStepMaxParts;
+            const int turn = phase >> 1 & 1;
+            uint32_t* sq = args.squares + (size_t(turn) * B + b) * kStepMaxParts;
             if (lane == 0 && !bad) {
               float mine = 0.f;
 #pragma unroll
               for (int w = 0; w < kStepComputeWarps; ++w) mine += s_red[w];
-              sq[part0] = mine;
-              red_release_gpu_add(arrived, 1u);
-              bad = !wait_count(arrived, uint32_t(parts));
+              red_relaxed_gpu_or(sq + part0, __float_as_uint(mine) | 0x80000000u);
+              args.squares[(size_t(turn ^ 1) * B + b) * kStepMaxParts + part0] = 0u;
             }
+            uint32_t word = 0;
+            if (lane < parts && !bad) bad = !wait_for([&]() { return (word = ld_relaxed_gpu_u32(sq + lane)) != 0u; });
             __syncwarp();
-            float tot = lane < parts ? __ldcg(sq + lane) : 0.f;
+            float tot = __uint_as_float(word & 0x7fffffffu);
 #pragma unroll
             for (int o = kStepMaxParts / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
             if (lane == 0) s_inv = rsqrtf(tot / float(args.hidden) + args.eps);

@@ -105,14 +105,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The thread may sleep this long in one try.  The default is short: warps that wait for a tile's accumulator try again and again, and
+// a GEMM at the power cap pays for that with its clock (2 x 300 rows x 1792 x 8192 24.6 -> 24.0 us, 2048 x 3584 x 8192 with norm
+// 123.0 -> 121.0, 4096 x 8192 x 7168 on two ranks 776 -> 765).
+constexpr uint32_t kMbarSleepNs = 20000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(kMbarSleepNs)
       : "memory");
   return ok != 0;
 }
@@ -122,7 +126,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   uint64_t t0 = 0;
   for (uint32_t n = 0;; ++n) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((n & 1023u) == 1023u) {
+    if ((n & 15u) == 15u) {
       if (*abort_flag) return false;
       const uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;

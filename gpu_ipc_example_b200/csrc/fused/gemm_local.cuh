@@ -508,10 +508,11 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   }
 }
 
-// out = RMSNorm(sum) * gamma for the rows of every rank (blockIdx.y); `out` may be `sum` itself.  One CTA per row; the
-// row stays in registers between the statistic and the scaling (rows of up to 4 x 8 x blockDim elements).  Behind 2048 rows of
-// 8192 it is bound by memory (15.5 us for its output, the sums that L2 writes back and those it reads again: more CTAs per SM
-// change nothing), behind few rows by its launch.
+// out = RMSNorm(sum) * gamma for the rows of every rank (blockIdx.y); `out` may be `sum` itself.  One CTA per row; rows of up to
+// 4 x 8 x blockDim elements stay in registers between the statistic and the scaling.  Behind few rows it is bound by its launch;
+// behind 2048 rows of 8192 it was by instructions: 18 per element (loads chosen by a flag beside the registers, additions of
+// zero, single fp32 operations), 72 % of the issue slots, 16.2 us cold where memory takes 8.  In a body of its own for rows in
+// registers, on pairs of fp32: 11 instructions, 13.4 - 14.6 us; 16 rows x 3584 x 8192 with its GEMM 13.7 -> 13.2 us a call.
 struct RowNormArgs {
   const void* sum[kMaxRanks];
   const void* gamma[kMaxRanks];
@@ -519,11 +520,44 @@ struct RowNormArgs {
   int N;
   float eps;
 };
+// Two fp32 operations in one instruction, each rounded as by itself.
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(d)
+      : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)), "l"(*reinterpret_cast<const uint64_t*>(&c)));
+  return *reinterpret_cast<const float2*>(&d);
+}
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)));
+  return *reinterpret_cast<const float2*>(&d);
+}
+template <typename T>
+__device__ __forceinline__ void row_norm_squares(float2& ss, uint4 x) {
+  const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = Cvt<T>::up(xs[e]);
+    ss = fma_f32x2(f, f, ss);
+  }
+}
+template <typename T>
+__device__ __forceinline__ uint4 row_norm_scale(uint4 x, uint4 g, float inv) {
+  const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, gs[4] = {g.x, g.y, g.z, g.w};
+  uint32_t ys[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 y = mul_f32x2(mul_f32x2(Cvt<T>::up(xs[e]), make_float2(inv, inv)), Cvt<T>::up(gs[e]));
+    ys[e] = Cvt<T>::down(y.x, y.y);
+  }
+  return make_uint4(ys[0], ys[1], ys[2], ys[3]);
+}
 template <typename T>
 __global__ void __launch_bounds__(512) row_norm_kernel(const __grid_constant__ RowNormArgs args) {
   constexpr int U = 4;
   __shared__ float s_part[16];
-  const int q = int(blockIdx.y), N = args.N, nvec = N / 8;
+  const int q = int(blockIdx.y), N = args.N, nvec = N / 8, tid = int(threadIdx.x);
   const uint4* gamma = static_cast<const uint4*>(args.gamma[q]);
   const int step = int(blockDim.x);
   const bool in_regs = nvec <= U * step;
@@ -532,47 +566,34 @@ __global__ void __launch_bounds__(512) row_norm_kernel(const __grid_constant__ R
   const uint4* src = static_cast<const uint4*>(args.sum[q]) + size_t(blockIdx.x) * nvec;
   uint4* dst = static_cast<uint4*>(args.out[q]) + size_t(blockIdx.x) * nvec;
   uint4 x[U], g[U];
-  float ss = 0.f;
-  for (int v0 = int(threadIdx.x); v0 < nvec; v0 += U * step) {
+  float2 ss = make_float2(0.f, 0.f);
+  if (in_regs) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int v = v0 + u * step;
-      x[u] = v < nvec ? src[v] : make_uint4(0, 0, 0, 0);
-      if (in_regs && v < nvec) g[u] = gamma[v];
-    }
+    for (int u = 0; u < U; ++u) x[u] = tid + u * step < nvec ? src[tid + u * step] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      acc8_add<T>(a, x[u]);
+    for (int u = 0; u < U; ++u)
+      if (tid + u * step < nvec) g[u] = gamma[tid + u * step];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += a[e] * a[e];
-    }
+    for (int u = 0; u < U; ++u) row_norm_squares<T>(ss, x[u]);
+  } else {
+    for (int v = tid; v < nvec; v += step) row_norm_squares<T>(ss, src[v]);
   }
+  float sum = ss.x + ss.y;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((tid & 31) == 0) s_part[tid >> 5] = sum;
   __syncthreads();
   // at most 16 warps: their sums by shuffles, not one shared-memory load after another
-  float tot = int(threadIdx.x & 15) < (step >> 5) ? s_part[threadIdx.x & 15] : 0.f;
+  float tot = (tid & 15) < (step >> 5) ? s_part[tid & 15] : 0.f;
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   const float inv = rsqrtf(tot / float(N) + args.eps);
-  for (int v0 = int(threadIdx.x); v0 < nvec; v0 += U * step) {
+  if (in_regs) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int v = v0 + u * step;
-      if (v >= nvec) continue;
-      const uint4 xv = in_regs ? x[u] : src[v];
-      const uint4 gv = in_regs ? g[u] : gamma[v];
-      const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, gs[4] = {gv.x, gv.y, gv.z, gv.w};
-      uint32_t ys[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 xf = Cvt<T>::up(xs[e]), gf = Cvt<T>::up(gs[e]);
-        ys[e] = Cvt<T>::down(xf.x * inv * gf.x, xf.y * inv * gf.y);
-      }
-      dst[v] = make_uint4(ys[0], ys[1], ys[2], ys[3]);
-    }
+    for (int u = 0; u < U; ++u)
+      if (tid + u * step < nvec) dst[tid + u * step] = row_norm_scale<T>(x[u], g[u], inv);
+  } else {
+    for (int v = tid; v < nvec; v += step) dst[v] = row_norm_scale<T>(src[v], gamma[v], inv);
   }
 }
 

@@ -9,8 +9,8 @@
 // 17.2 us that 16 rows x 3584 x 8192 with norm took in the kernel of gemm_local.cuh, one launch after the other.  So this one is
 // cut to let the next launch in: 106 KB of shared memory, 72 or 80 registers x 320 threads and 64 columns of tensor memory leave
 // room for a second CTA on the SM, and dependents are let go at once.  The next kernel's CTAs set up and bring the first 24 MB of
-// W to L2 as soon as there is room for them, while this kernel's stragglers or its norm are at work.  Now 13.8 us (one row 17.0 ->
-// 12.7, 32 rows 17.9 -> 14.8, 2048 x 6016 12.0 -> 9.5, 8192 x 7168 26.0 -> 23.6, back to back).  0.2 - 0.5 of that came with the
+// W to L2 as soon as there is room for them, while this kernel's stragglers or its norm are at work.  Now 13.5 us (one row 17.0 ->
+// 12.6, 32 rows 17.9 -> 14.5, 2048 x 6016 12.0 -> 9.2, 8192 x 7168 26.0 -> 23.3, back to back; 0.3 of it the norm).  0.2 - 0.5 of that came with the
 // cluster's barrier in two halves: a warp arrives when it has sent its sums and has the others', and its stores pass while the rest
 // of the cluster gets there.  With less of W fetched ahead the memory idles between the launches (16 MB: +0.5), more takes from the
 // stream of the kernel in front (40 MB: +1.6).

@@ -520,19 +520,6 @@ struct RowNormArgs {
   int N;
   float eps;
 };
-// Two fp32 operations in one instruction, each rounded as by itself.
-__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(d)
-      : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)), "l"(*reinterpret_cast<const uint64_t*>(&c)));
-  return *reinterpret_cast<const float2*>(&d);
-}
-__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)));
-  return *reinterpret_cast<const float2*>(&d);
-}
 template <typename T>
 __device__ __forceinline__ void row_norm_squares(float2& ss, uint4 x) {
   const uint32_t xs[4] = {x.x, x.y, x.z, x.w};

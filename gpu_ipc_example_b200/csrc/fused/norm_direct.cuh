@@ -3,7 +3,9 @@
 // once, adds in rank order in fp32, adds each rank's residual, rounds, and normalises; the rows stay in registers between
 // the statistic and the scaling, and the CTAs of a row hand each other their sums of squares through distributed shared
 // memory.  Bound by launch and memory latency at decode sizes (8 ranks, 16 rows of 8192: 9.2 us cold, the flag-in-data
-// kernel 20.4) and by memory above (8 ranks, 512 rows: 53 us for 209 MB).
+// kernel 20.4), above by memory, mostly its writes, and by how many CTAs' loads are in flight beside the arithmetic: on pairs of fp32
+// values (each rounded as by itself) 8 ranks, 512 rows of 8192 48.5 -> 46.7 us for 209 MB (bf16 60.6 -> 60.3: its registers leave room
+// for two CTAs an SM, not three; capped, 52 there and 6 - 18 % more at fewer rows), 300 x 5120 21.9 -> 19.8, 16 x 8192 5.2 -> 4.8.
 #pragma once
 
 #include "../coll/bulk_kernels.cuh"
@@ -42,9 +44,9 @@ __global__ void __launch_bounds__(kDirectNormThreads) direct_norm_kernel(const _
   pdl_launch_dependents();
 
   uint4 keep[N][U];
-  float ss[N];
+  float2 ss2[N];
 #pragma unroll
-  for (int q = 0; q < N; ++q) ss[q] = 0.f;
+  for (int q = 0; q < N; ++q) ss2[q] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const int v = first + tid + u * step;
@@ -55,22 +57,33 @@ __global__ void __launch_bounds__(kDirectNormThreads) direct_norm_kernel(const _
       x[q] = static_cast<const uint4*>(args.x[q])[row0 + v];
       keep[q][u] = static_cast<const uint4*>(args.residual[q])[row0 + v];
     }
-    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float2 a[4];
 #pragma unroll
-    for (int q = 0; q < N; ++q) acc8_add<T>(a, x[q]);
+    for (int e = 0; e < 4; ++e) a[e] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int q = 0; q < N; ++q) {
-      float b[8];
+      const uint32_t xs[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) b[e] = a[e];
-      acc8_add<T>(b, keep[q][u]);
-      keep[q][u] = acc8_pack<T>(b);
-      float r[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      acc8_add<T>(r, keep[q][u]);
+      for (int e = 0; e < 4; ++e) a[e] = add_f32x2(a[e], Cvt<T>::up(xs[e]));
+    }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss[q] += r[e] * r[e];
+    for (int q = 0; q < N; ++q) {
+      const uint4 res = keep[q][u];
+      const uint32_t rs[4] = {res.x, res.y, res.z, res.w};
+      uint32_t ys[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 b = add_f32x2(a[e], Cvt<T>::up(rs[e]));
+        ys[e] = Cvt<T>::down(b.x, b.y);
+        const float2 r = Cvt<T>::up(ys[e]);
+        ss2[q] = fma_f32x2(r, r, ss2[q]);
+      }
+      keep[q][u] = make_uint4(ys[0], ys[1], ys[2], ys[3]);
     }
   }
+  float ss[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) ss[q] = ss2[q].x + ss2[q].y;
   // The row statistic, from the rounded sums; the order depends on nothing but thread and part numbers, so ranks with the
   // same residual get the same bits.
 #pragma unroll
@@ -109,8 +122,8 @@ __global__ void __launch_bounds__(kDirectNormThreads) direct_norm_kernel(const _
       uint32_t ys[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float2 xf = Cvt<T>::up(xs[e]), gf = Cvt<T>::up(gs[e]);
-        ys[e] = Cvt<T>::down(xf.x * inv[q] * gf.x, xf.y * inv[q] * gf.y);
+        const float2 y = mul_f32x2(mul_f32x2(Cvt<T>::up(xs[e]), make_float2(inv[q], inv[q])), Cvt<T>::up(gs[e]));
+        ys[e] = Cvt<T>::down(y.x, y.y);
       }
       static_cast<uint4*>(args.res_out[q])[row0 + v] = keep[q][u];
       static_cast<uint4*>(args.out[q])[row0 + v] = make_uint4(ys[0], ys[1], ys[2], ys[3]);

@@ -20,10 +20,11 @@
 //
 // Few tiles (decode, narrow layers): K is split over the pairs of a cluster of 2, 4 or 8 CTAs; after the last MMA every
 // pair hands its fp32 partial sums for a share of the rows to the pair that owns them through distributed shared
-// memory (st.async, counted on the receiver's barrier), and the owners add them in a fixed order (the result does not depend on timing) and run the epilogue.
+// memory (st.async, counted on the receiver's barrier), and the owners add them in a fixed order (the result does not depend on
+// timing) and run the epilogue.
 // What bounds it, one B200: a large product the tensor pipe (98 % of active cycles at 2 x 4096 x 8192 x 7168, 657 us at the
 // power cap, the kernel with the exchange 950); one row of tiles per SM pair or less, the chain of launch, first loads (2.5 us)
-// and epilogue (0.9 + 0.013 BN us); decode sizes the weight stream (16 x 3584 x 8192: 15.5 us back to back, 58.7 MB).
+// and epilogue (0.9 + 0.013 BN us); up to 64 rows the weight stream, where gemm_stream.cuh is ahead (16 x 3584 x 8192 with norm 17.2 us here, 13.5).
 // The issuing threads had bounded it before: a lane picked by its number made every MMA and TMA copy cost ~90 ns (elect.sync:
 // 393 -> 302 ns per 256 x 256 x 64 block), and integer divisions of the ring position another 160 ns of the loads' loop.
 // Epilogue: 2-byte stores, 64 contiguous bytes of a row per warp, 3.3 us per 256 x 256 tile; transposed through shared memory

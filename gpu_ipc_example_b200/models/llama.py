@@ -132,7 +132,7 @@ class LlamaTP:
             nbytes = C.attention_workspace_bytes(batch, self.hq, self.hkv, self.attn_splits)
             self.attn_ws = [torch.zeros(nbytes, dtype=torch.uint8, device=dev) for _ in range(self.nlocal)]
         # The whole step as one kernel: measured ahead of the chain at every shape tried (1 - 64 sequences, 64 - 4096 positions,
-        # 1 - 4 KV heads per rank; 104 us against 142 for batch 1 at 64 positions, 274 against 294 for batch 64 at 4096).
+        # 1 - 4 KV heads per rank; 102 us against 138 for batch 1 at 64 positions, 266 against 283 for batch 64 at 4096, as graphs).
         self.one_kernel = False
         if self.kernels and fusion == "gemm" and comm is not None and comm._direct and not pack_weights and not self.local_gemm:
             nbytes = C.decode_step_workspace_bytes(comm._h, batch, cfg.layers, H, self.hq, self.hkv, self.ffn_local, cfg.vocab // W, max_ctx)

@@ -522,26 +522,6 @@ struct RowNormArgs {
   float eps;
 };
 template <typename T>
-__device__ __forceinline__ void row_norm_squares(float2& ss, uint4 x) {
-  const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float2 f = Cvt<T>::up(xs[e]);
-    ss = fma_f32x2(f, f, ss);
-  }
-}
-template <typename T>
-__device__ __forceinline__ uint4 row_norm_scale(uint4 x, uint4 g, float inv) {
-  const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, gs[4] = {g.x, g.y, g.z, g.w};
-  uint32_t ys[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float2 y = mul_f32x2(mul_f32x2(Cvt<T>::up(xs[e]), make_float2(inv, inv)), Cvt<T>::up(gs[e]));
-    ys[e] = Cvt<T>::down(y.x, y.y);
-  }
-  return make_uint4(ys[0], ys[1], ys[2], ys[3]);
-}
-template <typename T>
 __global__ void __launch_bounds__(512) row_norm_kernel(const __grid_constant__ RowNormArgs args) {
   constexpr int U = 4;
   __shared__ float s_part[16];

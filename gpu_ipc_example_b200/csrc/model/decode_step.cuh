@@ -926,7 +926,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
                 found[part0] = make_float2(best.v, __int_as_float(best.i));
                 is_last = atom_acq_rel_gpu_add(args.arrivals + at.sequences + b, 1u) == uint32_t(parts - 1);
               }
-              if (__shfl_sync(0xffffffffu, is_last, 0)) {
+              is_last = __shfl_sync(0xffffffffu, is_last, 0);
+              __syncwarp();  // a shuffle orders no memory: lane 0's acquire comes before the other lanes' loads through this
+              if (is_last) {
                 const float2 f = __ldcg(found + lane % parts);
                 best = warp_best(Best{f.x, __float_as_int(f.y)});
                 if (lane == 0) args.ids[b] = best.i;

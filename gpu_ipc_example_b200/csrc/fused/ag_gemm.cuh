@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) ag_gemm_kernel(const __grid_c
       mbar_init(&s.acc_full[i], 1);
       mbar_init(&s.acc_empty[i], 4);
     }
+    mbar_init(&s.mma_done, 1);
     s.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -170,9 +171,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) ag_gemm_kernel(const __grid_c
           tma_load_2d(s.b[st][0], tb, &s.full[st], kb * kGemmBK, nt * BN);
         }
       }
+      const uint64_t t0 = globaltimer_ns();
       for (uint32_t back = 0; back < uint32_t(STAGES) && back < it; ++back) {
         const uint32_t j = it - 1 - back;
-        mbar_wait(&s.full[j % STAGES], (j / STAGES) & 1u, abort_flag, me.timeout_ns);
+        mbar_drain(&s.full[j % STAGES], (j / STAGES) & 1u, t0);
       }
     }
   } else if (warp == 1) {
@@ -201,6 +203,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) ag_gemm_kernel(const __grid_c
         if (!ok) break;
         umma_commit(&s.acc_full[buf]);
       }
+      umma_commit(&s.mma_done);
+      mbar_drain(&s.mma_done, 0, globaltimer_ns());
     }
   } else if (warp < 6) {
     const int lane_group = warp & 3;

@@ -68,9 +68,10 @@ CollInfo fused_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64
                               cudaStream_t stream);
 
 // The same two layers when this process drives every rank (a world of one, an emulated world): one GEMM over the callers'
-// operands, no exchange and no workspace (gemm_local.cuh).  `workspace` and `packed_kblocks` are not looked at.
+// operands, no exchange and no workspace (gemm_local.cuh).  `workspace` and `packed_kblocks` are not looked at.  Of the flags kMuteSends
+// is known: partial sums of a K split stay unsent, so the waits for them run out.
 CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64_t M, int64_t N, int64_t K, float eps,
-                              bool with_norm, cudaStream_t stream);
+                              bool with_norm, cudaStream_t stream, uint32_t flags = 0);
 CollInfo local_allgather_gemm(Comm& comm, DType t, const AgGemmPtrs* ptrs, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 
 }  // namespace b200ipc

@@ -136,6 +136,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   *abort_flag = 1;
   return false;
 }
+// For a thread that is about to leave: what it issued (copies into shared memory, MMAs) has to be over first, also where the CTA has
+// given up.  So this looks at no abort flag, and a copy that a peer never issued ends it by the limit, counted from `since`.  Copies
+// and MMAs in flight take microseconds.
+constexpr uint64_t kMbarDrainNs = 10000000;
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity, uint64_t since) {
+  for (bool late = false; !mbar_try_wait(bar, parity) && !late;) late = globaltimer_ns() - since > kMbarDrainNs;
+}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -263,6 +270,7 @@ struct GemmSmem {
   uint64_t empty[STAGES];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t mma_done;                           // every MMA of the CTA is over
   alignas(16) unsigned char epi[4][32 * 128];  // transpose patch of each epilogue warp
   uint32_t tmem_base;
   int abort_flag;
@@ -517,6 +525,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_ar_kernel(const __grid_c
       mbar_init(&s.acc_full[i], 1);
       mbar_init(&s.acc_empty[i], 4);  // one arrival per epilogue warp
     }
+    mbar_init(&s.mma_done, 1);
     s.abort_flag = 0;
     s.owner_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -581,9 +590,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_ar_kernel(const __grid_c
       }
       gemm_trace(me, lay, 2);
       // copies in flight land in this CTA's shared memory: wait for the ones still pending
+      const uint64_t t0 = globaltimer_ns();
       for (uint32_t back = 0; back < uint32_t(STAGES) && back < it; ++back) {
         const uint32_t j = it - 1 - back;
-        mbar_wait(&s.full[j % STAGES], (j / STAGES) & 1u, abort_flag, timeout_ns);
+        mbar_drain(&s.full[j % STAGES], (j / STAGES) & 1u, t0);
       }
     }
   } else if (warp == 1) {
@@ -617,6 +627,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_ar_kernel(const __grid_c
         if (!ok) break;
         umma_commit(&s.acc_full[buf]);  // accumulator complete
       }
+      umma_commit(&s.mma_done);
+      mbar_drain(&s.mma_done, 0, globaltimer_ns());
       gemm_trace(me, lay, 3);
     }
   } else if (warp < 6) {

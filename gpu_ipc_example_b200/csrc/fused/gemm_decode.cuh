@@ -36,6 +36,7 @@ struct DecodeSmem {
   uint64_t empty[kDecStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t mma_done;
   uint32_t tmem_base;
   int abort_flag;
   int owner_fail;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
       mbar_init(&s.acc_full[i], 1);
       mbar_init(&s.acc_empty[i], 4);
     }
+    mbar_init(&s.mma_done, 1);
     s.abort_flag = 0;
     s.owner_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -150,9 +152,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
         }
       }
       gemm_trace(me, lay, 2);
+      const uint64_t t0 = globaltimer_ns();
       for (uint32_t back = 0; back < uint32_t(kDecStages) && back < it; ++back) {
         const uint32_t j = it - 1 - back;
-        mbar_wait(&s.full[j % kDecStages], (j / kDecStages) & 1u, abort_flag, timeout_ns);
+        mbar_drain(&s.full[j % kDecStages], (j / kDecStages) & 1u, t0);
       }
     }
   } else if (warp == 1) {
@@ -191,6 +194,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
         if (!ok) break;
         umma_commit(&s.acc_full[buf]);
       }
+      umma_commit(&s.mma_done);
+      mbar_drain(&s.mma_done, 0, globaltimer_ns());
       gemm_trace(me, lay, 3);
     }
   } else if (warp < 6) {

@@ -265,7 +265,7 @@ void check_local(Comm& comm, int64_t M, int64_t N, int64_t K) {
 }  // namespace
 
 CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64_t M, int64_t N, int64_t K, float eps,
-                              bool with_norm, cudaStream_t stream) {
+                              bool with_norm, cudaStream_t stream, uint32_t flags) {
   check_local(comm, M, N, K);
   const int W = comm.world();
   const int64_t kb = ceil_div64(K, kGemmBK) * W;
@@ -279,6 +279,7 @@ CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64
     sargs.K = int(K);
     sargs.segs = W;
     sargs.groups = 1;
+    sargs.mute = (flags & kMuteSends) != 0;
   } else {
     std::memset(&args, 0, sizeof(args));
     args.rows = int(M);
@@ -286,6 +287,7 @@ CollInfo local_gemm_allreduce(Comm& comm, DType t, const GemmArPtrs* ptrs, int64
     args.K = int(K);
     args.segs = W;
     args.shards = args.groups = 1;
+    args.mute = (flags & kMuteSends) != 0;
   }
   RowNormArgs norm;
   std::memset(&norm, 0, sizeof(norm));

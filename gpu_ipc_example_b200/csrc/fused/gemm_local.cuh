@@ -66,6 +66,7 @@ struct LocalGemmArgs {
   int n_tiles;
   int band;      // m-tiles visited before the next W tile
   int splits;    // K splits = pairs per cluster
+  int mute;      // the partial sums stay unsent (failure injection)
   int stages;
   int warm_w;    // the first stages' W boxes are brought to L2 before the wait for the previous kernel
 };
@@ -165,7 +166,7 @@ __device__ __forceinline__ LocTile loc_tile(const LocalGemmArgs& a, int t) {
 template <typename T, int KSUB>
 __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid_constant__ LocalGemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full[kLocMaxStages], empty[kLocMaxStages], acc_full[2], acc_empty[2], slab_full;
+  __shared__ uint64_t full[kLocMaxStages], empty[kLocMaxStages], acc_full[2], acc_empty[2], slab_full, mma_done;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -199,6 +200,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
       mbar_init(&acc_empty[i], 16);  // eight epilogue warps of both CTAs
     }
     mbar_init(&slab_full, 1);
+    mbar_init(&mma_done, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -282,10 +284,11 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
         }
       }
       // copies in flight land in the pair's shared memory: the even CTA sees them all arrive
+      const uint64_t t0 = globaltimer_ns();
       if (side == 0)
         for (uint32_t back = 0; back < uint32_t(stages) && back < it; ++back) {
           const uint32_t j = it - 1 - back;
-          mbar_wait(&full[j % uint32_t(stages)], (j / uint32_t(stages)) & 1u, abort_flag, timeout_ns);
+          mbar_drain(&full[j % uint32_t(stages)], (j / uint32_t(stages)) & 1u, t0);
         }
     }
   } else if (warp == 1) {
@@ -322,6 +325,8 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
         if (!ok) break;
         umma_commit_pair(&acc_full[buf], mask);
       }
+      umma_commit_pair(&mma_done, uint16_t(1u << crank));
+      mbar_drain(&mma_done, 0, globaltimer_ns());
     }
   }
 
@@ -449,7 +454,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
     const bool bad = warp < 2 || __any_sync(0xffffffffu, !mbar_wait(&acc_full[0], 0, abort_flag, timeout_ns));
     if (!bad) {
       tc_fence_after_sync();
-      for (int d = 1; d < splits; ++d) {
+      for (int d = 1; d < splits && !args.mute; ++d) {
         const int o = (split + d) % splits;
         const int slot = split < o ? split : split - 1;
         const uint32_t dst = map_to_cta(smem_u32(slab + size_t(slot) * own * 128 + my_n), uint32_t(2 * o + side));
@@ -495,6 +500,11 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   tc_fence_after_sync();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   if (*abort_flag && threadIdx.x == 0) {
+    // What the others had sent before they got here lands first, and copies of an odd CTA that was a stage ahead when the even one,
+    // whose barriers count them, gave up.
+    const uint64_t t0 = globaltimer_ns();
+    if (splits > 1) mbar_drain(&slab_full, 0, t0);
+    while (side == 1 && globaltimer_ns() - t0 < kMbarDrainNs) __nanosleep(1000);
     st_volatile_u32(args.abort_word, 1u);
     if (claim_status(args.abort_word, kTimeout)) {
       StatusBlock* sb = args.status;

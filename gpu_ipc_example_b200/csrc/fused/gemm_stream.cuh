@@ -49,6 +49,7 @@ struct StreamGemmArgs {
   int n_tiles;
   int splits;       // K splits = CTAs per cluster
   int stages;
+  int mute;         // the partial sums stay unsent (failure injection)
   int warm;         // k blocks of W that a CTA brings to L2 before the wait for the previous kernel
 };
 
@@ -67,7 +68,7 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[O]) {
 template <typename T, int BN>
 __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __grid_constant__ StreamGemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full[kStrMaxStages], empty[kStrMaxStages], acc_full, slab_full;
+  __shared__ uint64_t full[kStrMaxStages], empty[kStrMaxStages], acc_full, slab_full, mma_done;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
     }
     mbar_init(&acc_full, 1);
     mbar_init(&slab_full, 1);
+    mbar_init(&mma_done, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -160,8 +162,9 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
         }
       }
       // copies in flight land before the CTA leaves
+      const uint64_t t0 = globaltimer_ns();
       for (int back = 1; back <= min(it, stages); ++back)
-        mbar_wait(&full[(it - back) % stages], uint32_t((it - back) / stages) & 1u, abort_flag, timeout_ns);
+        mbar_drain(&full[(it - back) % stages], uint32_t((it - back) / stages) & 1u, t0);
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -184,6 +187,8 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
         }
       }
       if (ok) umma_commit(&acc_full);
+      umma_commit(&mma_done);
+      mbar_drain(&mma_done, 0, globaltimer_ns());
     }
   } else {
     // ---- epilogue: lane = a row of W (an output column), accumulator columns = rows of X, one half of them per group.  A warp's
@@ -217,6 +222,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
       tc_fence_after_sync();
       if (splits > 1) {  // the others' shares to them, straight from the registers
         constexpr int H = BN / 2;
+        const int sent = args.mute ? 0 : (valid + 3) / 4 * 4;
         uint32_t acc[H];
 #pragma unroll
         for (int c = 0; c < H; c += 8) tmem_ld_8cols(tmem_lane + uint32_t(half * H + c), acc + c);
@@ -231,7 +237,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
             dst = map_to_cta(smem_u32(slab + (size_t(split < o ? split : split - 1) * own + size_t(c - o * own)) * 128 + my_n), uint32_t(o)) - uint32_t(j) * 512u;
             bar = map_to_cta(smem_u32(&slab_full), uint32_t(o));
           }
-          if (o != split && c < (valid + 3) / 4 * 4) st_async(dst + uint32_t(j) * 512u, acc[j], bar);
+          if (o != split && c < sent) st_async(dst + uint32_t(j) * 512u, acc[j], bar);
         }
         ok = !__any_sync(0xffffffffu, !mbar_wait(&slab_full, 0, abort_flag, timeout_ns));
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
@@ -304,6 +310,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
   tc_fence_after_sync();
   if (warp == 1) tmem_dealloc(tmem_base, kStrTmemCols);
   if (*abort_flag && threadIdx.x == 0) {
+    if (splits > 1) mbar_drain(&slab_full, 0, globaltimer_ns());  // what the others had sent before they got here
     st_volatile_u32(args.abort_word, 1u);
     if (claim_status(args.abort_word, kTimeout)) {
       StatusBlock* sb = args.status;

@@ -310,7 +310,7 @@ template <typename T>
 __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __grid_constant__ DecodeStepArgs args) {
   using T2 = typename Num<T>::T2;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full_w[kStepMaxStages], full_x[kStepMaxStages], empty[kStepMaxStages], acc_full[2], acc_empty[2], attn_done;
+  __shared__ uint64_t full_w[kStepMaxStages], full_x[kStepMaxStages], empty[kStepMaxStages], acc_full[2], acc_empty[2], attn_done, mma_done;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort, s_flag;
   __shared__ float s_red[kStepComputeWarps], s_inv;
@@ -357,6 +357,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
       mbar_init(&acc_empty[i], kStepComputeWarps);
     }
     mbar_init(&attn_done, 1);
+    mbar_init(&mma_done, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -407,9 +408,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
             return true;
           });
       // copies in flight land before the CTA leaves
+      const uint64_t t0 = globaltimer_ns();
 #pragma unroll 1
       for (int back = 1; back <= min(it, int(stages)); ++back)
-        mbar_wait(&full_w[uint32_t(it - back) % stages], (uint32_t(it - back) / stages) & 1u, abort_flag, timeout_ns);
+        mbar_drain(&full_w[uint32_t(it - back) % stages], (uint32_t(it - back) / stages) & 1u, t0);
     }
   } else if (warp == 1) {
     // ---- X tiles ----------------------------------------------------------------------------------------------------------
@@ -453,9 +455,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
           advance();
         }
       }
+      const uint64_t t0 = globaltimer_ns();
 #pragma unroll 1
       for (int back = 1; back <= min(it, int(stages)); ++back)
-        mbar_wait(&full_x[uint32_t(it - back) % stages], (uint32_t(it - back) / stages) & 1u, abort_flag, timeout_ns);
+        mbar_drain(&full_x[uint32_t(it - back) % stages], (uint32_t(it - back) / stages) & 1u, t0);
     }
   } else if (warp == 2) {
     // ---- tcgen05.mma ------------------------------------------------------------------------------------------------------
@@ -503,6 +506,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
           st = n % stages;
         }
       }
+      umma_commit(&mma_done);
+      mbar_drain(&mma_done, 0, globaltimer_ns());
     }
   } else if (warp >= 4) {
     // ---- compute ----------------------------------------------------------------------------------------------------------

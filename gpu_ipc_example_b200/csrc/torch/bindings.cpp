@@ -455,7 +455,7 @@ void keep_apart(std::vector<at::Tensor>& ts, const std::vector<at::Tensor>& outs
 // The same two layers with every rank in this process (a world of one or an emulated one): no workspace, outputs anywhere.
 std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::Tensor> ws, std::vector<at::Tensor> residuals,
                                    std::vector<at::Tensor> gammas, std::vector<at::Tensor> outs, std::vector<at::Tensor> res_outs,
-                                   double eps, bool with_norm, int64_t comm_id) {
+                                   double eps, bool with_norm, int64_t comm_id, int64_t flags) {
   Comm& c = get(comm_id);
   check_tensors(c, xs, "x");
   check_tensors(c, ws, "weight");
@@ -487,7 +487,7 @@ std::vector<int64_t> local_gemm_ar(std::vector<at::Tensor> xs, std::vector<at::T
     p[size_t(i)].res_out = res_outs.empty() ? nullptr : res_outs[i].data_ptr();
   }
   return info_vec(local_gemm_allreduce(c, dtype_of(xs[0]), p.data(), M, N, K, float(eps), with_norm,
-                                       at::cuda::getCurrentCUDAStream(c.device())));
+                                       at::cuda::getCurrentCUDAStream(c.device()), uint32_t(flags)));
 }
 
 std::vector<int64_t> local_ag_gemm(std::vector<at::Tensor> xs, std::vector<at::Tensor> ws, std::vector<at::Tensor> outs, int64_t comm_id) {
@@ -866,7 +866,7 @@ PyObject* fast_local_gemm_ar(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!a.ok) Py_RETURN_NONE;
   return report(without_gil([&] {
     return local_gemm_ar(std::move(xs), std::move(ws), std::move(residuals), std::move(gammas), std::move(outs), std::move(res_outs), eps, with_norm,
-                         comm);
+                         comm, 0);
   }));
   END_HANDLE_TH_ERRORS
 }
@@ -905,7 +905,7 @@ TORCH_LIBRARY(b200ipc, m) {
       &fused_gemm_ar);
   m.def(
       "local_gemm_ar(Tensor[] xs, Tensor[] ws, Tensor[] residuals, Tensor[] gammas, Tensor[] outs, Tensor[] res_outs, "
-      "float eps, bool with_norm, int comm) -> int[]",
+      "float eps, bool with_norm, int comm, int flags=0) -> int[]",
       &local_gemm_ar);
   m.def("local_ag_gemm(Tensor[] xs, Tensor[] ws, Tensor[] outs, int comm) -> int[]", &local_ag_gemm);
   m.def("all_reduce_lists(Tensor[] ins, Tensor[] outs, int comm, str algo, int ctas, int warps, int flags) -> int[]", &all_reduce_lists);

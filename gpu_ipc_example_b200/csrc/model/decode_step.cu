@@ -93,7 +93,8 @@ bool decode_step_takes(const Comm& comm, const DecodeStepShape& s, int pos) {
 
 size_t decode_step_workspace_bytes(const Comm& comm, const DecodeStepShape& s) { return step_layout(comm, s).total; }
 
-void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStepPtrs& p, int pos, float eps, float theta, cudaStream_t stream) {
+void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStepPtrs& p, int pos, float eps, float theta, cudaStream_t stream,
+                 uint32_t flags) {
   B200_REQUIRE(decode_step_takes(comm, s, pos) && theta > 0.f, "decode step: shape not supported");
   B200_CUDA_CHECK(cudaSetDevice(comm.device()));
   const int W = comm.world(), G = s.hq / s.hkv, ctas = comm.sm_count();
@@ -126,6 +127,7 @@ void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStep
   a.vocab = s.vocab;
   a.max_ctx = s.max_ctx;
   a.pos = pos;
+  a.mute = (flags & kMuteSends) != 0;
   a.eps = eps;
   a.scale_log2 = 1.4426950408889634f / sqrtf(float(kAttnD));
   a.log2_theta = log2f(theta);

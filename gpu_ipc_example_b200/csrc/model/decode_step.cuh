@@ -20,8 +20,8 @@
 // memory in fp32, in a slot of their own (tile + CTA number), and whoever needs the result adds a tile's slots in order: the
 // result does not depend on timing.
 //
-// CTAs wait on one another: the launch is cooperative.  Every wait is bounded; a CTA whose wait runs out stops arriving, which
-// ends the others' waits the same way.
+// CTAs wait on one another: the launch is cooperative.  Every wait is bounded; a CTA whose wait runs out stops arriving, also at its
+// own barriers (an arrival that stands for a wait that failed could complete a phase early), which ends the others' waits the same way.
 //
 // Measured, four layers and the head of that shape as one step: 423 us as a chain of kernels, 317 here (floor 194: 1.25 GB).
 // Two thirds of a layer are bound by the stream (gate/up and down: 6 - 7 TB/s), the rest by the chain of meetings: about 1.5 us
@@ -101,6 +101,7 @@ struct DecodeStepArgs {
   int world, batch, bn, stages;
   int hidden, hq, hkv, ffn, vocab;  // per rank
   int max_ctx, pos;
+  int mute;  // CTA 0 arrives at no meeting point (failure injection)
   float eps, scale_log2, log2_theta;
 };
 
@@ -540,7 +541,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
     // Everything the compute warps have stored so far is complete: adds one to a meeting point's counter.
     auto arrive = [&](uint32_t* p) {
       bad = compute_sync(bad);
-      if (tid == 0 && !bad) red_release_gpu_add(p, 1u);
+      if (tid == 0 && !bad && !(args.mute && cta == 0)) red_release_gpu_add(p, 1u);
     };
     auto wait = [&](const uint32_t* p, uint32_t target) {
       if (tid == 0 && !bad) bad = !wait_count(p, target);
@@ -598,8 +599,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
         const int t = u / g.kb;
         u = min(g.u1, (t + 1) * g.kb);
         const uint32_t buf = seg_no & 1u;
-        if (!mbar_wait(&acc_full[buf], (seg_no >> 1) & 1u, abort_flag, timeout_ns)) bad = true;
-        __syncwarp();
+        bad = __any_sync(0xffffffffu, !mbar_wait(&acc_full[buf], (seg_no >> 1) & 1u, abort_flag, timeout_ns));
+        if (bad) break;
         tc_fence_after_sync();
         float* slot = args.part + size_t(t + cta) * slot_floats + (warp & 3) * 32 + lane;
 #pragma unroll 1
@@ -732,6 +733,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
               }
             }
             bad = compute_sync(bad);  // nobody is more than a pair ahead, so a stage's parity is never taken for the round before
+            if (bad) break;
             const uint32_t used = 2u * uint32_t(min(2, end - pair));
             uint32_t unused;
             if (uint32_t(tid) < used) mbar_arrive(&empty[stage(uint32_t(tid), &unused)]);
@@ -741,6 +743,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
               ph ^= 1u;
             }
           }
+          if (bad) break;
           lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
           lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
           if (c == 0) {
@@ -846,7 +849,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
           bad = compute_sync(bad);  // the scratch is written again
           u = end;
         }
-        if (tid == 0) mbar_arrive(&attn_done);
+        if (tid == 0 && !bad) mbar_arrive(&attn_done);
         arrive(done);
       } else if (which == kGemmGateUp) {
         // ---- SiLU(gate) * up -----------------------------------------------------------------------------------------------

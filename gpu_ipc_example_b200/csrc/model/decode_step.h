@@ -28,6 +28,8 @@ struct DecodeStepPtrs {
 // per KV head, a hidden size that the row-parallel GEMMs of the chain of kernels take, at least one position in the cache.
 bool decode_step_takes(const Comm& comm, const DecodeStepShape& s, int pos);
 size_t decode_step_workspace_bytes(const Comm& comm, const DecodeStepShape& s);
-void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStepPtrs& p, int pos, float eps, float theta, cudaStream_t stream);
+// Of the flags kMuteSends is known: one CTA stays away from the meeting points, so the waits there run out.
+void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStepPtrs& p, int pos, float eps, float theta, cudaStream_t stream,
+                 uint32_t flags = 0);
 
 }  // namespace b200ipc

@@ -610,7 +610,7 @@ std::vector<at::Tensor> decode_step_op(at::Tensor h, const std::vector<at::Tenso
                                        const std::vector<at::Tensor>& kcache, const std::vector<at::Tensor>& vcache,
                                        const std::vector<at::Tensor>& head, const std::vector<at::Tensor>& gamma_attn,
                                        const std::vector<at::Tensor>& gamma_mlp, at::Tensor gamma_final, at::Tensor workspace, int64_t hq,
-                                       int64_t hkv, int64_t pos, double eps, double theta, int64_t comm_id) {
+                                       int64_t hkv, int64_t pos, double eps, double theta, int64_t comm_id, int64_t flags) {
   Comm& c = get(comm_id);
   const size_t W = size_t(c.world()), L = gamma_mlp.size(), n = L * W;
   if (h.dim() != 2 || L == 0 || gamma_attn.size() != L || head.size() != W || !(theta > 0)) return {};
@@ -657,7 +657,8 @@ std::vector<at::Tensor> decode_step_op(at::Tensor h, const std::vector<at::Tenso
                   size_t(workspace.nbytes()) >= decode_step_workspace_bytes(c, s) && (reinterpret_cast<uintptr_t>(workspace.data_ptr()) & 255) == 0,
               "b200ipc: decode step workspace too small or not 256-byte aligned");
   p.workspace = workspace.data_ptr();
-  decode_step(c, dtype_of(h), s, p, int(pos), float(eps), float(theta), at::cuda::getCurrentCUDAStream(c.device()));
+  decode_step(c, dtype_of(h), s, p, int(pos), float(eps), float(theta), at::cuda::getCurrentCUDAStream(c.device()),
+              uint32_t(flags));
   return out;
 }
 
@@ -928,7 +929,7 @@ TORCH_LIBRARY(b200ipc, m) {
         "int splits, float theta) -> Tensor", &rope_decode_attention_op);
   m.def("decode_step(Tensor(a!) h, Tensor[] wqkv, Tensor[] wo, Tensor[] wgu, Tensor[] wdown, Tensor[] kcache, Tensor[] vcache, Tensor[] head, "
         "Tensor[] gamma_attn, Tensor[] gamma_mlp, Tensor gamma_final, Tensor workspace, int hq, int hkv, int pos, float eps, float theta, "
-        "int comm) -> Tensor[]", &decode_step_op);
+        "int comm, int flags=0) -> Tensor[]", &decode_step_op);
   m.def("rmsnorm(Tensor x, Tensor gamma, float eps) -> Tensor", &rmsnorm_op);
   m.def("row_argmax(Tensor x) -> (Tensor, Tensor)", &row_argmax_op);
   m.def("silu_mul(Tensor gate_up) -> Tensor", &silu_mul_op);

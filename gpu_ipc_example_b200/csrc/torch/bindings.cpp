@@ -689,13 +689,18 @@ at::Tensor silu_mul_op(at::Tensor gate_up) {
 // ---- the list calls of Communicator, past the dispatcher -----------------------------------------------------------------
 // A small collective is bound by its call: through torch.ops the lists of an 8-rank world cost about 7 us before the launch,
 // as CPython calls 2.  A call comes this way only where nothing listens on the way there and its tensors are plain ones: no
-// mode or transform, no profiler, no subclass or wrapper.  Everything else, arguments that do not fit included, gives None,
-// and Communicator makes the call through the operator, which does what it always did.
+// mode or transform, no profiler, no subclass or wrapper, no kernel beside ours registered for the operator (a program's autograd
+// kernel, say).  Everything else, arguments that do not fit included, gives None, and Communicator makes the call through the
+// operator, which does what it always did.
 bool nothing_listens() {
   const auto& tls = c10::impl::tls_local_dispatch_key_set();
   return ((tls.included_ - c10::default_included_set).raw_repr() & ~c10::full_backend_mask) == 0 && !at::impl::torch_function_mode_enabled() &&
          !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::hasCallbacks();
 }
+
+c10::OperatorHandle operator_of(const char* name) { return c10::Dispatcher::singleton().findSchemaOrThrow(name, ""); }
+// Whether somebody has registered a kernel for an operator of this file; ours are composite ones, which stand under no key of their own.
+bool other_kernels(const c10::OperatorHandle& op) { return op.hasKernelForAnyDispatchKey(c10::DispatchKeySet(c10::DispatchKeySet::FULL)); }
 
 bool plain_list(PyObject* o, std::vector<at::Tensor>* ts) {
   static const c10::DispatchKeySet plain =
@@ -719,7 +724,8 @@ struct FastArgs {
   PyObject* const* args;
   Py_ssize_t n, at = 0;
   bool ok;
-  FastArgs(PyObject* const* a, Py_ssize_t count, Py_ssize_t want) : args(a), n(count), ok(count == want && nothing_listens()) {}
+  FastArgs(PyObject* const* a, Py_ssize_t count, Py_ssize_t want, const c10::OperatorHandle& op)
+      : args(a), n(count), ok(count == want && nothing_listens() && !other_kernels(op)) {}
   std::vector<at::Tensor> list() {
     std::vector<at::Tensor> ts;
     if (ok) ok = plain_list(args[at++], &ts);
@@ -783,7 +789,8 @@ auto without_gil(F&& f) {
 
 PyObject* fast_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  FastArgs a(args, n, 7);
+  static const c10::OperatorHandle op = operator_of("b200ipc::all_reduce_lists");
+  FastArgs a(args, n, 7, op);
   const auto ins = a.list(), outs = a.list();
   const int64_t comm = a.integer();
   const std::string algo = a.text();
@@ -795,7 +802,8 @@ PyObject* fast_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 PyObject* fast_all_gather(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  FastArgs a(args, n, 7);
+  static const c10::OperatorHandle op = operator_of("b200ipc::all_gather_lists");
+  FastArgs a(args, n, 7, op);
   const auto ins = a.list(), outs = a.list();
   const int64_t comm = a.integer();
   const std::string algo = a.text();
@@ -807,7 +815,8 @@ PyObject* fast_all_gather(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 PyObject* fast_reduce_scatter(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  FastArgs a(args, n, 6);
+  static const c10::OperatorHandle op = operator_of("b200ipc::reduce_scatter_lists");
+  FastArgs a(args, n, 6, op);
   const auto ins = a.list(), outs = a.list();
   const int64_t comm = a.integer();
   const std::string algo = a.text();
@@ -820,7 +829,8 @@ PyObject* fast_reduce_scatter(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // (outs, residual outs, launch report), or None
 PyObject* fast_ar_rmsnorm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  FastArgs a(args, n, 5);
+  static const c10::OperatorHandle op = operator_of("b200ipc::ar_rmsnorm_lists");
+  FastArgs a(args, n, 5, op);
   const auto xs = a.list(), residuals = a.list(), gammas = a.list();
   const double eps = a.real();
   const int64_t comm = a.integer();
@@ -859,7 +869,8 @@ PyObject* fast_ar_rmsnorm(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 PyObject* fast_local_gemm_ar(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  FastArgs a(args, n, 9);
+  static const c10::OperatorHandle op = operator_of("b200ipc::local_gemm_ar");
+  FastArgs a(args, n, 9, op);
   auto xs = a.list(), ws = a.list(), residuals = a.list(), gammas = a.list(), outs = a.list(), res_outs = a.list();
   const double eps = a.real();
   const bool with_norm = a.boolean();
@@ -874,7 +885,8 @@ PyObject* fast_local_gemm_ar(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 PyObject* fast_local_ag_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  FastArgs a(args, n, 4);
+  static const c10::OperatorHandle op = operator_of("b200ipc::local_ag_gemm");
+  FastArgs a(args, n, 4, op);
   auto xs = a.list(), ws = a.list(), outs = a.list();
   const int64_t comm = a.integer();
   if (!a.ok) Py_RETURN_NONE;

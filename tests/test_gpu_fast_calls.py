@@ -77,3 +77,28 @@ def test_errors_are_the_operators():
             assert errors[0] == errors[1]
         out = comm.all_reduce(a, None)  # the communicator still works
         assert torch.equal(out[0], a[0])
+
+
+@pytest.mark.parametrize("key", ["AutogradCUDA", "CUDA"])
+def test_a_kernel_of_the_program_is_what_runs(key):
+    """A kernel that a program registers for an operator, an autograd one say, is not passed by."""
+    xs = [torch.ones(2, 64, device="cuda").half() for _ in range(2)]
+    seen = []
+
+    def mine(xs, residuals, gammas, eps, comm):
+        seen.append(eps)
+        return [t.clone() for t in xs + residuals], [0] * 9
+
+    with Communicator.virtual(2, 0, staging_bytes=16 << 20) as comm:
+        call = lambda: comm.allreduce_residual_rmsnorm(xs, xs, [x[0] for x in xs], 0.25)
+        plain = call()
+        lib = torch.library.Library("b200ipc", "IMPL")
+        try:
+            lib.impl("ar_rmsnorm_lists", mine, key)
+            out, _ = call()
+            assert seen == [0.25] and torch.equal(out[0], xs[0])
+        finally:
+            lib._destroy()
+        for a, b in zip(sum(call(), []), sum(plain, [])):
+            assert torch.equal(a, b)
+        assert seen == [0.25]

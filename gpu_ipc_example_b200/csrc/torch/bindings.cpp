@@ -939,8 +939,8 @@ TORCH_LIBRARY(b200ipc, m) {
         &decode_attention_op);
   m.def("rope_decode_attention(Tensor qkv, Tensor(a!) kcache, Tensor(b!) vcache, Tensor(c!) workspace, int hq, int hkv, int pos, "
         "int splits, float theta) -> Tensor", &rope_decode_attention_op);
-  m.def("decode_step(Tensor(a!) h, Tensor[] wqkv, Tensor[] wo, Tensor[] wgu, Tensor[] wdown, Tensor[] kcache, Tensor[] vcache, Tensor[] head, "
-        "Tensor[] gamma_attn, Tensor[] gamma_mlp, Tensor gamma_final, Tensor workspace, int hq, int hkv, int pos, float eps, float theta, "
+  m.def("decode_step(Tensor(a!) h, Tensor[] wqkv, Tensor[] wo, Tensor[] wgu, Tensor[] wdown, Tensor(b!)[] kcache, Tensor(c!)[] vcache, Tensor[] head, "
+        "Tensor[] gamma_attn, Tensor[] gamma_mlp, Tensor gamma_final, Tensor(d!) workspace, int hq, int hkv, int pos, float eps, float theta, "
         "int comm, int flags=0) -> Tensor[]", &decode_step_op);
   m.def("rmsnorm(Tensor x, Tensor gamma, float eps) -> Tensor", &rmsnorm_op);
   m.def("row_argmax(Tensor x) -> (Tensor, Tensor)", &row_argmax_op);

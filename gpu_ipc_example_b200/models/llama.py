@@ -19,7 +19,8 @@ over the cache (grouped-query, split over the context) in one, SiLU(gate) * up i
 arg-max over the logits are one kernel each.
 Where one process drives every rank, `fusion="gemm"` with plain weights runs the whole step, head and arg-max included, as one
 persistent kernel (`csrc/model/decode_step.cuh`) for up to 64 sequences and a cache that is not empty; the chain of kernels
-takes the rest, and everything once `one_kernel` is set to False or `stage_events` to a list.
+takes the rest, and everything once `one_kernel` or `kernels` is set to False, `local_gemm` to a projection, `fusion` to something
+else or `stage_events` to a list.
 With `kernels=False` the same steps are plain PyTorch ops (the reference path of the tests).
 
 The reference has no model code; its smoke script all-reduces decode-sized fp16 activations the way a
@@ -214,7 +215,9 @@ class LlamaTP:
         cfg = self.cfg
         B, D = tokens.shape[0], cfg.head_dim
         pos = self.pos
-        if self.one_kernel and self.stage_events is None:
+        # what picks the kernels of the chain picks the chain, also where it is set after construction
+        if (self.one_kernel and self.kernels and self.fusion == "gemm" and self.comm._direct and not self.local_gemm
+                and self.stage_events is None):
             per = lambda ws: [ws[i][l] for l in range(cfg.layers) for i in range(self.nlocal)]
             out = torch.ops.b200ipc.decode_step(self.embed[tokens], per(self.wqkv), per(self.wo_run), per(self.wgu), per(self.wdown_run),
                                                 per(self.kcache), per(self.vcache), self.lm_head, self.norm_attn, self.norm_mlp,

@@ -153,3 +153,28 @@ def test_captured_steps_replay():
             assert torch.equal(got[0], step()) and torch.equal(got[1], m.last_hidden[0])
         torch.cuda.synchronize()
         comm.check()
+
+
+@pytest.mark.parametrize("name,value", [("one_kernel", False), ("kernels", False), ("local_gemm", True), ("fusion", "allreduce"), ("stage_events", [])])
+def test_switches_that_are_set_later_pick_the_chain(name, value):
+    cfg = LlamaConfig(layers=2, hidden=256, n_heads=2, n_kv_heads=1, ffn=128, vocab=64)
+    with Communicator.virtual(1, 0, staging_bytes=64 << 20) as comm:
+        m = LlamaTP(cfg, comm, batch=2, max_ctx=4, fusion="gemm")
+        tokens = torch.tensor([3, 5], device="cuda")
+
+        def step():
+            m.pos, before = 1, comm.launches
+            m.decode(tokens)
+            return comm.launches - before, m.last_hidden[0].float()
+
+        launches, want = step()
+        assert launches == 2
+        setattr(m, name, value)
+        launches, got = step()
+        assert launches != 2
+        # the bound of test_decode_step for each of the two ways; the PyTorch ops of kernels=False round a norm twice
+        assert _rel(got, want) <= 2 * 2.0 ** -11 / 3 ** 0.5 * (11 * cfg.layers + 2) ** 0.5
+        if name == "stage_events":
+            assert {n for n, *_ in m.stage_events} >= {"qkv_gemm", "rope_attention"}
+        torch.cuda.synchronize()
+        comm.check()

@@ -351,9 +351,6 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
   const bool copy_in = (me.aux[1] & kBulkCopyIn) != 0;
   const bool copy_out = (me.aux[1] & kBulkCopyOut) != 0;
 
-  uint32_t bar = me.bar_seq;
-  if (me.seq_dev) bar += ld_volatile_u32(me.seq_dev + 2);
-
   // Shards.  In the caller's buffer shard s holds shard_elems elements starting at
   // s * shard_elems (AllReduce: a vector-aligned cut of the whole buffer;
   // ReduceScatter: nelems / N; AllGather: nelems = one rank's contribution).  In the
@@ -383,6 +380,8 @@ __global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const __grid_constan
     bulk_direct_body<T, N, M>(args, r, shard_elems, valid(r));
     return;
   }
+  uint32_t bar = me.bar_seq;
+  if (me.seq_dev) bar += ld_volatile_u32(me.seq_dev + 2);
   // A slab is blockDim consecutive vectors; slab j belongs to CTA j % gridDim.x on every rank
   // and a CTA keeps kU of its slabs in flight.
   const int64_t ntiles = (shard_vec + nthreads - 1) / nthreads;

@@ -105,28 +105,37 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// The thread may sleep this long in one try.  The default is short: warps that wait for a tile's accumulator try again and again, and
-// a GEMM at the power cap pays for that with its clock (2 x 300 rows x 1792 x 8192 24.6 -> 24.0 us, 2048 x 3584 x 8192 with norm
-// 123.0 -> 121.0, 4096 x 8192 x 7168 on two ranks 776 -> 765).
-constexpr uint32_t kMbarSleepNs = 20000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The thread may sleep for `ns` in one try.
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t ns) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(kMbarSleepNs)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up (and tells the whole CTA through *abort_flag) when the communicator's time
-// limit for one wait has passed.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t timeout_ns) {
+// Bounded wait, one try after the other: gives up (and tells the whole CTA through *abort_flag) when the communicator's time limit for
+// one wait has passed.  Flag and timer are looked at every EVERY tries.
+template <uint32_t EVERY, typename Try>
+__device__ __forceinline__ bool mbar_wait_by(Try attempt, volatile int* abort_flag, uint64_t timeout_ns) {
   uint64_t t0 = 0;
   for (uint32_t n = 0;; ++n) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((n & 15u) == 15u) {
+    if (attempt()) return true;
+    if ((n & (EVERY - 1)) == EVERY - 1) {
       if (*abort_flag) return false;
       const uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;
@@ -135,6 +144,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
   *abort_flag = 1;
   return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t timeout_ns) {
+  return mbar_wait_by<1024>([=]() { return mbar_try_wait(bar, parity); }, abort_flag, timeout_ns);
+}
+// The same with long sleeps, for the kernels of a process that drives every rank.  A try is short by default: warps that wait for a
+// tile's accumulator try again and again, and a GEMM at the power cap pays for that with its clock (2 x 300 rows x 1792 x 8192 24.6 ->
+// 24.0 us, 2048 x 3584 x 8192 with norm 123.0 -> 121.0; 4096 x 8192 x 7168 on two ranks level).  The kernels with the exchange gain
+// nothing (4096 gathered rows 513 us either way) and one of them loses: 16 rows x 3584 x 8192 without the exchange 12.5 us with short
+// tries and 12.8 with long ones, packed with norm 16.2 and 16.4.
+constexpr uint32_t kMbarSleepNs = 20000;
+__device__ __forceinline__ bool mbar_wait_long(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t timeout_ns) {
+  return mbar_wait_by<16>([=]() { return mbar_try_wait(bar, parity, kMbarSleepNs); }, abort_flag, timeout_ns);
 }
 // For a thread that is about to leave: what it issued (copies into shared memory, MMAs) has to be over first, also where the CTA has
 // given up.  So this looks at no abort flag, and a copy that a peer never issued ends it by the limit, counted from `since`.  Copies

@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
 #pragma unroll 1
         for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
           const int nsub = KSUB == 1 ? 1 : min(KSUB, kb1 - kb);
-          if (!mbar_wait(&empty[st], ph, abort_flag, timeout_ns)) break;
+          if (!mbar_wait_long(&empty[st], ph, abort_flag, timeout_ns)) break;
           if (side == 0) mbar_expect_tx(&full[st], tile_bytes * uint32_t(nsub));
 #pragma unroll
           for (int sub = 0; sub < KSUB; ++sub) {
@@ -298,12 +298,12 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
       for (int tt = cluster; tt < total && !*abort_flag; tt += nclusters, ++i) {
         const uint32_t buf = i & 1u;
         const uint32_t idesc = make_idesc<T>(kLocWRows, KSUB > 1 || tt < args.cut_from ? bn : bn / args.cut);
-        if (!mbar_wait(&acc_empty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, timeout_ns)) break;
+        if (!mbar_wait_long(&acc_empty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, timeout_ns)) break;
         tc_fence_after_sync();
         bool ok = true;
 #pragma unroll 1
         for (int kb = kb0; kb < kb1; kb += KSUB) {
-          if (!mbar_wait(&full[st], ph, abort_flag, timeout_ns)) { ok = false; break; }
+          if (!mbar_wait_long(&full[st], ph, abort_flag, timeout_ns)) { ok = false; break; }
           tc_fence_after_sync();
           const int nsub = KSUB == 1 ? 1 : min(KSUB, kb1 - kb);
 #pragma unroll
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
           }
           if (c0 < valid) load_residual(res0, out_off(t, c0), rows_left(t, c0, kLocChunk), rv);
         }
-        if (__any_sync(0xffffffffu, !mbar_wait(&acc_full[buf], (i >> 1) & 1u, abort_flag, timeout_ns))) break;
+        if (__any_sync(0xffffffffu, !mbar_wait_long(&acc_full[buf], (i >> 1) & 1u, abort_flag, timeout_ns))) break;
         tc_fence_after_sync();
         for (int c = c0; c < valid; c += 2 * kLocChunk) {
           uint32_t acc[kLocChunk];
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
       const int c0 = group * kLocChunk;
       if (res0) load_residual(res0, out_off(t, c_own + c0), rows_left(t, c_own + c0, min(own - c0, kLocChunk)), rv);
     }
-    const bool bad = warp < 2 || __any_sync(0xffffffffu, !mbar_wait(&acc_full[0], 0, abort_flag, timeout_ns));
+    const bool bad = warp < 2 || __any_sync(0xffffffffu, !mbar_wait_long(&acc_full[0], 0, abort_flag, timeout_ns));
     if (!bad) {
       tc_fence_after_sync();
       for (int d = 1; d < splits && !args.mute; ++d) {
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
         }
       }
     }
-    if (!bad && !__any_sync(0xffffffffu, !mbar_wait(&slab_full, 0, abort_flag, timeout_ns))) {
+    if (!bad && !__any_sync(0xffffffffu, !mbar_wait_long(&slab_full, 0, abort_flag, timeout_ns))) {
       asm volatile("fence.acq_rel.cluster;" ::: "memory");
       for (int c = group * kLocChunk; c < own && c_own + c < valid; c += 2 * kLocChunk) {
         const int cw = min(own - c, kLocChunk);

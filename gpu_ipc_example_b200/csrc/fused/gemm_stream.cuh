@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
       const uint64_t policy = evict_first_policy();
 #pragma unroll 1
       for (int kb = kb0; kb < kb1; ++kb, ++it, next_k(k)) {
-        if (!mbar_wait(&empty[st], ph, abort_flag, timeout_ns)) break;
+        if (!mbar_wait_long(&empty[st], ph, abort_flag, timeout_ns)) break;
         mbar_expect_tx(&full[st], stage_bytes);
         unsigned char* dst = ring + st * stage_bytes;
         tma_stream_2d(dst, k.w, &full[st], k.col, n0, policy);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
       bool ok = true;
 #pragma unroll 1
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&full[st], ph, abort_flag, timeout_ns)) { ok = false; break; }
+        if (!mbar_wait_long(&full[st], ph, abort_flag, timeout_ns)) { ok = false; break; }
         tc_fence_after_sync();
         const uint64_t da = make_sw128_kmajor_desc(ring_addr + st * stage_bytes);
         const uint64_t db = make_sw128_kmajor_desc(ring_addr + st * stage_bytes + w_bytes);
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
         if (c + j < mine) rv[j] = p[size_t(j) * size_t(N)];
     };
     if (res0) load_residual(res0, 0);
-    bool ok = !__any_sync(0xffffffffu, !mbar_wait(&acc_full, 0, abort_flag, timeout_ns));
+    bool ok = !__any_sync(0xffffffffu, !mbar_wait_long(&acc_full, 0, abort_flag, timeout_ns));
     if (ok) {
       tc_fence_after_sync();
       if (splits > 1) {  // the others' shares to them, straight from the registers
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) gemm_stream_kernel(const __gri
           }
           if (o != split && c < sent) st_async(dst + uint32_t(j) * 512u, acc[j], bar);
         }
-        ok = !__any_sync(0xffffffffu, !mbar_wait(&slab_full, 0, abort_flag, timeout_ns));
+        ok = !__any_sync(0xffffffffu, !mbar_wait_long(&slab_full, 0, abort_flag, timeout_ns));
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
       }
     }

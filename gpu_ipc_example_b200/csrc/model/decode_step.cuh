@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
       int it = 0;
       const uint64_t policy = evict_first_policy();
       auto ready = [&]() {
-        if (!mbar_wait(&empty[st], ph, abort_flag, timeout_ns)) return false;
+        if (!mbar_wait_long(&empty[st], ph, abort_flag, timeout_ns)) return false;
         mbar_expect_tx(&full_w[st], kStepTileBytes);
         return true;
       };
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
         StepWalk w(g);
 #pragma unroll 1
         for (int u = g.u0; ok && u < g.u1; ++u, w.next()) {
-          ok = mbar_wait(&empty[st], ph, abort_flag, timeout_ns);
+          ok = mbar_wait_long(&empty[st], ph, abort_flag, timeout_ns);
           if (!ok) break;
           mbar_expect_tx(&full_x[st], x_bytes);
           tma_load_2d(ring + st * stage_bytes + kStepTileBytes, g.x + w.rank * g.x_step, &full_x[st], w.col(), 0);
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
         if (which != kGemmQkv) continue;
 #pragma unroll 1
         for (int u = 2 * a0; ok && u < 2 * a1; ++u) {  // K and V tiles have no X beside them
-          ok = mbar_wait(&empty[st], ph, abort_flag, timeout_ns);
+          ok = mbar_wait_long(&empty[st], ph, abort_flag, timeout_ns);
           if (!ok) break;
           mbar_arrive(&full_x[st]);
           advance();
@@ -474,13 +474,13 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
         for (int u = g.u0; ok && u < g.u1; ++seg) {
           const int end = min(g.u1, (u / g.kb + 1) * g.kb);
           const uint32_t buf = seg & 1u;
-          ok = mbar_wait(&acc_empty[buf], ((seg >> 1) & 1u) ^ 1u, abort_flag, timeout_ns);
+          ok = mbar_wait_long(&acc_empty[buf], ((seg >> 1) & 1u) ^ 1u, abort_flag, timeout_ns);
           if (!ok) break;
           tc_fence_after_sync();
           uint32_t accumulate = 0;
 #pragma unroll 1
           for (; u < end; ++u) {
-            ok = mbar_wait(&full_w[st], ph, abort_flag, timeout_ns) && mbar_wait(&full_x[st], ph, abort_flag, timeout_ns);
+            ok = mbar_wait_long(&full_w[st], ph, abort_flag, timeout_ns) && mbar_wait_long(&full_x[st], ph, abort_flag, timeout_ns);
             if (!ok) break;
             tc_fence_after_sync();
             const uint64_t da = make_sw128_kmajor_desc(ring_addr + st * stage_bytes);
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
         if (which == kGemmQkv) {
           // The attention's stages go by.  A wait for the parity of a later round would pass before they have: not until
           // the compute warps are through with them.
-          ok = ok && mbar_wait(&attn_done, uint32_t(l) & 1u, abort_flag, timeout_ns);
+          ok = ok && mbar_wait_long(&attn_done, uint32_t(l) & 1u, abort_flag, timeout_ns);
           const uint32_t n = st + 2u * uint32_t(a1 - a0);
           ph ^= (n / stages) & 1u;
           st = n % stages;
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
         const int t = u / g.kb;
         u = min(g.u1, (t + 1) * g.kb);
         const uint32_t buf = seg_no & 1u;
-        bad = __any_sync(0xffffffffu, !mbar_wait(&acc_full[buf], (seg_no >> 1) & 1u, abort_flag, timeout_ns));
+        bad = __any_sync(0xffffffffu, !mbar_wait_long(&acc_full[buf], (seg_no >> 1) & 1u, abort_flag, timeout_ns));
         if (bad) break;
         tc_fence_after_sync();
         float* slot = args.part + size_t(t + cta) * slot_floats + (warp & 3) * 32 + lane;
@@ -685,11 +685,11 @@ __global__ void __launch_bounds__(kStepThreads, 1) decode_step_kernel(const __gr
             if (v < end) {
               uint32_t pk, pv;
               const uint32_t sk = stage(2u * uint32_t(group), &pk), sv = stage(2u * uint32_t(group) + 1u, &pv);
-              if (!mbar_wait(&full_w[sk], pk, abort_flag, timeout_ns)) bad = true;
-              if (!mbar_wait(&full_w[sv], pv, abort_flag, timeout_ns)) bad = true;
+              if (!mbar_wait_long(&full_w[sk], pk, abort_flag, timeout_ns)) bad = true;
+              if (!mbar_wait_long(&full_w[sv], pv, abort_flag, timeout_ns)) bad = true;
               // (the arrival that stands for the missing X tile, so that this round of the barrier is over as well)
-              if (!mbar_wait(&full_x[sk], pk, abort_flag, timeout_ns)) bad = true;
-              if (!mbar_wait(&full_x[sv], pv, abort_flag, timeout_ns)) bad = true;
+              if (!mbar_wait_long(&full_x[sk], pk, abort_flag, timeout_ns)) bad = true;
+              if (!mbar_wait_long(&full_x[sv], pv, abort_flag, timeout_ns)) bad = true;
               __syncwarp();
               const uint32_t kt = ring_addr + sk * stage_bytes, vt = ring_addr + sv * stage_bytes;
               auto chunk_addr = [&](uint32_t tile, int chunk) {  // 16-byte chunk 0..15 of this lane's position, 128-byte swizzle

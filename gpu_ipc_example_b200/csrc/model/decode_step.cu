@@ -91,6 +91,16 @@ bool decode_step_takes(const Comm& comm, const DecodeStepShape& s, int pos) {
   return std::max(z.units, z.attn_units) * comm.sm_count() < (int64_t(1) << 31) && int64_t(W) * s.vocab < (int64_t(1) << 31);
 }
 
+// Eight heads per KV head and an accumulator for 64 sequences leave room for seven stages, three K and V pairs: too few in flight where
+// the attention is most of the step.  One rank, FFN 3584, graphs, this kernel / the chain: 64 sequences, 4 KV heads, hidden 4096, 166
+// tiles per SM 219 / 214 us, 221 263 / 250, 110 175 / 173; hidden 8192, 8 KV heads, 443 tiles 497 / 457; 56 sequences there 454 / 443,
+// 52 432 / 441, 48 412 / 443 (the chain splits the context less evenly below 56).  Four heads per KV head, 886 tiles 719 / 733; two ranks,
+// 443 tiles 450 / 463.
+bool decode_step_pays(const Comm& comm, const DecodeStepShape& s, int pos) {
+  return !(comm.world() == 1 && s.hq == 8 * s.hkv && s.batch >= 56 &&
+           step_sizes(1, s, pos).attn_units >= int64_t(160) * comm.sm_count());
+}
+
 size_t decode_step_workspace_bytes(const Comm& comm, const DecodeStepShape& s) { return step_layout(comm, s).total; }
 
 void decode_step(Comm& comm, DType t, const DecodeStepShape& s, const DecodeStepPtrs& p, int pos, float eps, float theta, cudaStream_t stream,

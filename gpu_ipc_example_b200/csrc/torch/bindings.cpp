@@ -620,7 +620,7 @@ std::vector<at::Tensor> decode_step_op(at::Tensor h, const std::vector<at::Tenso
   const int64_t B = h.size(0), H = h.size(1), F = wgu[0].size(0) / 2, V = head[0].size(0), ctx = kcache[0].size(2), D = 128;
   if (h.scalar_type() != at::kHalf && h.scalar_type() != at::kBFloat16) return {};
   const DecodeStepShape s{int(B), int(L), int(H), int(hq), int(hkv), int(F), int(V), int(ctx)};
-  if (!decode_step_takes(c, s, int(pos))) return {};
+  if (!decode_step_takes(c, s, int(pos)) || !decode_step_pays(c, s, int(pos))) return {};
   auto takes = [&](const at::Tensor& t, at::IntArrayRef sizes) {
     return t.is_cuda() && t.get_device() == c.device() && t.scalar_type() == h.scalar_type() && t.sizes() == sizes && fits_kernels(t);
   };

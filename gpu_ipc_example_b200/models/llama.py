@@ -132,8 +132,10 @@ class LlamaTP:
             self.attn_splits = C.attention_splits(batch, self.hkv, max_ctx, dev_index)
             nbytes = C.attention_workspace_bytes(batch, self.hq, self.hkv, self.attn_splits)
             self.attn_ws = [torch.zeros(nbytes, dtype=torch.uint8, device=dev) for _ in range(self.nlocal)]
-        # The whole step as one kernel: measured ahead of the chain at every shape tried (1 - 64 sequences, 64 - 4096 positions,
-        # 1 - 4 KV heads per rank; 102 us against 138 for batch 1 at 64 positions, 266 against 283 for batch 64 at 4096, as graphs).
+        # The whole step as one kernel.  Four layers of the 70B shape, one KV head: 284 us against 361 for batch 1 at 64 positions, 319
+        # against 395 for batch 32 at 2048, 419 against 463 for batch 64 at 4096, as graphs.  Ahead nearly everywhere from hidden 1024 up,
+        # 1 - 64 sequences, 64 - 100000 positions, 1 - 16 KV heads (where it is not, the operator answers nothing).  Tiny models: launch by
+        # launch 80 us against 188 (64 sequences, hidden 512), as graphs 79 against 76, 16 sequences 70 against 62.
         self.one_kernel = False
         if self.kernels and fusion == "gemm" and comm is not None and comm._direct and not pack_weights and not self.local_gemm:
             nbytes = C.decode_step_workspace_bytes(comm._h, batch, cfg.layers, H, self.hq, self.hkv, self.ffn_local, cfg.vocab // W, max_ctx)

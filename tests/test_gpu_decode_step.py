@@ -178,3 +178,18 @@ def test_switches_that_are_set_later_pick_the_chain(name, value):
             assert {n for n, *_ in m.stage_events} >= {"qkv_gemm", "rope_attention"}
         torch.cuda.synchronize()
         comm.check()
+
+
+@pytest.mark.parametrize("batch,G,tiles,one", [(56, 8, 0, False), (55, 8, 0, True), (56, 8, -1, True), (56, 4, 0, True)])
+def test_attention_heavy_steps_run_as_the_chain(batch, G, tiles, one):
+    """Both sides of the rule: from 160 tiles of 64 positions per SM on (here exactly, or one tile per sequence less)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    pos = 64 * (-(-160 * sms // (56 * 4)) + tiles)
+    cfg = LlamaConfig(layers=1, hidden=256, n_heads=4 * G, n_kv_heads=4, ffn=128, vocab=64)
+    with Communicator.virtual(1, 0, staging_bytes=64 << 20) as comm:
+        m = LlamaTP(cfg, comm, batch=batch, max_ctx=pos + 1, fusion="gemm")
+        m.pos, before = pos, comm.launches
+        m.decode(torch.zeros(batch, dtype=torch.int64, device="cuda"))
+        assert (comm.launches - before == 2) == one
+        torch.cuda.synchronize()
+        comm.check()

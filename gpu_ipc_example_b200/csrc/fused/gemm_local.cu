@@ -168,7 +168,7 @@ void launch_local(Comm& comm, LocalGemmArgs& args, DType t, const LocalPlan& p, 
   info->ctas = int(cfg.gridDim.x);
   info->warps = kLocThreads / 32;
   info->nwires = info->ctas * info->warps;
-  info->steps = ceil_div64(total, clusters);
+  info->steps = args.cut_from + (total - args.cut_from) * p.cut;  // tiles and parts of tiles that the pairs take
   info->launches = 1;
 }
 

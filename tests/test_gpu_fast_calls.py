@@ -102,3 +102,25 @@ def test_a_kernel_of_the_program_is_what_runs(key):
         for a, b in zip(sum(call(), []), sum(plain, [])):
             assert torch.equal(a, b)
         assert seen == [0.25]
+
+
+def test_the_direct_route_is_taken():
+    """The fast calls answer for plain lists, and for nothing that somebody would see."""
+    W = 2
+    with Communicator.virtual(W, 0, staging_bytes=32 << 20) as comm:
+        h, ones = comm._h, lambda *s: [torch.ones(*s, device="cuda").half() for _ in range(W)]
+        xs, ws, res, gam = ones(16, 512), ones(512, 512), ones(16, 512), ones(512)
+        calls = [lambda x: comm._fast_all_reduce(x, ones(16, 512), h, "auto", 0, 0, 0), lambda x: comm._fast_all_gather(x, ones(32, 512), h, "auto", 0, 0, 0),
+                 lambda x: comm._fast_reduce_scatter(x, ones(8, 512), h, "auto", 0, 0), lambda x: comm._fast_ar_rmsnorm(x, res, gam, 1e-5, h),
+                 lambda x: comm._fast_local_gemm_ar(x, ws, res, gam, ones(16, 512), ones(16, 512), 1e-5, True, h),
+                 lambda x: comm._fast_local_ag_gemm(x, ws, ones(32, 512), h)]
+        for call in calls:
+            assert call(xs) is not None
+            assert call([t.as_subclass(Sub) for t in xs]) is None
+            with Seen():
+                assert call(xs) is None
+            with torch.profiler.profile():
+                assert call(xs) is None
+            assert call([xs[0], None]) is None and call(tuple(xs)) is None and call([t.cpu() for t in xs]) is None
+        torch.cuda.synchronize()
+        comm.check()

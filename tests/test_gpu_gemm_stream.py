@@ -18,6 +18,14 @@ def _close(got, want, dtype):
     torch.testing.assert_close(got.double(), want, atol=1e-4, rtol=1.01 * HALF_ULP[dtype])
 
 
+def _check_kernel(comm, tiles, splits):
+    """One tile per CTA (cluster) is this kernel; the other one reports all of its tiles as steps."""
+    if splits:
+        assert comm.last_info.steps == 1 and comm.last_info.ctas == tiles * splits
+    else:
+        assert comm.last_info.steps > 1
+
+
 # rows: one, the accumulator's steps, one less and one more; no split, two, four, eight; a last tile of 64 rows of W; K that fills
 # no block; ranks that meet inside a share of K; splits 0: the other kernel's side of the rule
 @pytest.mark.parametrize("world,M,K,N,splits", [
@@ -35,7 +43,7 @@ def test_linear(world, M, K, N, splits, dtype):
     y = sum(x.double() @ w.double().t() for x, w in zip(xs, ws))
     with Communicator.virtual(world, 0, staging_bytes=96 << 20) as comm:
         outs = comm.linear_allreduce(xs, ws)
-        assert not splits or comm.last_info.ctas == -(-N // 128) * splits
+        _check_kernel(comm, -(-N // 128), splits)
         for o in outs:
             _close(o, y, dtype)
         for o, s, r in zip(*comm.linear_allreduce(xs, ws, res), res):
@@ -67,7 +75,7 @@ def test_gather_linear(world, rows, K, N, splits, dtype):
     full = torch.cat(xs).double()
     with Communicator.virtual(world, 0, staging_bytes=32 << 20) as comm:
         outs = comm.allgather_linear(xs, ws)
-        assert not splits or comm.last_info.ctas == -(-N // 128) * world * splits
+        _check_kernel(comm, -(-N // 128) * world, splits)
         for o, w in zip(outs, ws):
             _close(o, full @ w.double().t(), dtype)
         torch.cuda.synchronize()

@@ -87,8 +87,11 @@ def main():
             stream.synchronize()
             graph = torch.cuda.CUDAGraph()
             model.pos = args.ctx - 1
+            before = comm.launches if comm is not None else 0
             with torch.cuda.graph(graph, stream=stream):
                 out = model.decode(tokens)
+            # per launch of the one kernel eight layers (of one rank), and the first norm; the chain makes four launches a layer
+            one_kernel = model.one_kernel and comm.launches - before < 2 * cfg.layers + 1
             graph.replay()
             stream.synchronize()
             if multi:
@@ -108,11 +111,12 @@ def main():
         step = float(t.item())
         stages = None
         if args.breakdown:
-            model.pos = args.ctx - 1
-            model.stage_events = []
             with torch.cuda.stream(stream):
-                model.decode(tokens)
-                stream.synchronize()
+                for _ in range(2):  # the first one warms the chain up
+                    model.pos = args.ctx - 1
+                    model.stage_events = []
+                    model.decode(tokens)
+                    stream.synchronize()
             acc = {}
             for name, a, b in model.stage_events:
                 acc[name] = acc.get(name, 0.0) + a.elapsed_time(b)
@@ -125,8 +129,9 @@ def main():
                 "arm": arm, "world": world, "layers": cfg.layers, "batch": args.batch, "ctx": args.ctx,
                 "ms_per_step": round(step * 1e3, 4), "tokens_per_s": round(args.batch / step, 1),
                 "weight_and_kv_stream_floor_ms": round(floor * 1e3, 4), "fraction_of_floor": round(floor / step, 3),
-                "kernels": bool(model.kernels), "packed_weights": bool(args.pack and arm == "gemm"),
-                "stage_ms_eager": stages, "peaks": peaks, "next_token_sample": int(out[0]),
+                "kernels": bool(model.kernels), "one_kernel": one_kernel, "packed_weights": bool(args.pack and arm == "gemm"),
+                # the stages are those of the chain of kernels, also where the step that was timed is the one kernel
+                "stage_ms_eager": stages, "stages_of": "chain of kernels" if stages else None, "peaks": peaks, "next_token_sample": int(out[0]),
             }), flush=True)
         del model, graph
         if comm is not None:

@@ -325,8 +325,6 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
         if (!ok) break;
         umma_commit_pair(&acc_full[buf], mask);
       }
-      umma_commit_pair(&mma_done, uint16_t(1u << crank));
-      mbar_drain(&mma_done, 0, globaltimer_ns());
     }
   }
 
@@ -495,6 +493,12 @@ __global__ void __launch_bounds__(kLocThreads, 1) gemm_local_kernel(const __grid
   // ---- the pair leaves together; tensor memory goes back ------------------------------------------------------
   tc_fence_before_sync();
   __syncthreads();
+  if (warp == 1 && side == 0 && *abort_flag) {  // elsewhere the epilogue has seen every accumulator complete
+    if (elect_one()) {  // (the lane that issued the MMAs: the same one is elected every time)
+      umma_commit_pair(&mma_done, uint16_t(1u << crank));
+      mbar_drain(&mma_done, 0, globaltimer_ns());
+    }
+  }
   __syncwarp();
   cluster_sync_all();
   tc_fence_after_sync();

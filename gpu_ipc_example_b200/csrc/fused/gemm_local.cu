@@ -188,8 +188,8 @@ struct StreamPlan {
 // are places for CTAs (two on an SM), with at least eight blocks of K and four rows to finish for each; a narrow layer pads its rows
 // to 32 for an eighth split (8 rows x 8192 x 1280: four splits 13.1 us, eight 9.6, the other kernel 11.4).  That one keeps what
 // it measured ahead or level in (with norm, this kernel / that one): more than 16 rows for a CTA to finish (24 rows x 448 x 4864
-// 8.2 us / 7.8), more than 32 rows where that leaves places empty (48 x 3584 x 8192, 256 CTAs 17.0 / 18.7; 48 x 3000 x 5120, 160
-// CTAs 15.2 / 14.0), weights of which the part fetched ahead is next to nothing (470 MB: 81 / 80).
+// 8.2 us / 7.8), more than 32 rows where that leaves places empty (fewer than 200 of the 296 that 148 SMs have: 48 x 3584 x 8192, 256
+// CTAs 17.0 / 18.7; 48 x 3000 x 5120, 160 CTAs 15.2 / 14.0), weights of which the part fetched ahead is next to nothing (470 MB: 81 / 80).
 StreamPlan plan_stream(const Comm& comm, int64_t columns, bool exact, int64_t tiles, int64_t kb_total) {
   StreamPlan p;
   if (columns > kStrMaxRows || (exact && columns != 16 && columns != 32 && columns != 64)) return p;
